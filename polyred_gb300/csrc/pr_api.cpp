@@ -230,6 +230,10 @@ struct Ctx {
     cudaEvent_t ev_resolved = nullptr, ev_ao0 = nullptr, ev_ao = nullptr;
     bool ao_marched = false;  // the last frame ran the AO march (ev_ao0, ev_ao hold it)
     DevBuf<float> ao_T;
+    DevBuf<float> linemax;  // [4][H][W], AO's line maxima
+    DevBuf<uint8_t> ao_tab;  // AO's tap tables for frames of width ao_tab_w and rounding ao_tab_ulp
+    int ao_tab_w = 0;
+    float ao_tab_ulp = 0.0f;
     int n_sms = 1;
 };
 
@@ -826,10 +830,10 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         // lists no pixel, and both launches are left out.
         const bool with_ao = out && out->rgba && c->sb.has_ao;
         c->ao_marched = with_ao;
-        if (with_ao && (rc = c->ao_T.ensure(npx))) return rc;
+        if (with_ao && ((rc = c->ao_T.ensure(npx)) || (rc = c->linemax.ensure(4 * npx)))) return rc;
         KTRY(prk::launch_resolve_listing(W, H, c->keys.p, c->nanseq.p, c->beaten.p, dcnt, c->win.p, c->depth_ao.p,
                                          c->first_rec.p, c->attr_state.p, c->vis_list.p, c->sb.tri_flags.p,
-                                         with_ao ? c->ao_list.p : nullptr, st));
+                                         with_ao ? c->ao_list.p : nullptr, c->linemax.p, st));
         prk::AoParams ap{};
         if (with_ao) {
             CUDA_TRY(cudaEventRecord(c->ev_resolved, st));
@@ -845,6 +849,16 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             ap.list = c->ao_list.p;
             ap.cnt = dcnt;
             ap.T = c->ao_T.p;
+            ap.linemax = c->linemax.p;
+            ap.exact_T = dh ? 1 : 0;
+            if (c->ao_tab_w != W || c->ao_tab_ulp != ap.ao_half_ulp) {
+                c->ao_tab_w = 0;
+                if ((rc = c->ao_tab.ensure(prk::ao_tables_bytes()))) return rc;
+                KTRY(prk::launch_ao_tables(ap, c->ao_tab.p, sc));
+                c->ao_tab_w = W;
+                c->ao_tab_ulp = ap.ao_half_ulp;
+            }
+            ap.tables = c->ao_tab.p;
             KTRY(prk::launch_ao_T(ap, sc));
             CUDA_TRY(cudaEventRecord(c->ev_ao, sc));
             launches += 1;
@@ -1088,7 +1102,7 @@ int pr_destroy(void* ctx) {
     if (c->ev_resolved) cudaEventDestroy(c->ev_resolved);
     if (c->ev_ao0) cudaEventDestroy(c->ev_ao0);
     if (c->ev_ao) cudaEventDestroy(c->ev_ao);
-    c->ao_T.release();
+    c->ao_T.release(); c->linemax.release(); c->ao_tab.release();
     if (c->stream_c) {
         cudaStreamSynchronize(c->stream_c);
         cudaStreamDestroy(c->stream_c);
@@ -1556,7 +1570,7 @@ struct Batch {
     DevBuf<prk::Counters> cnt;
     DevBuf<unsigned long long> keys;
     DevBuf<uint32_t> nanseq, beaten, win, ao_list, chunk, smaps;
-    DevBuf<float> depth_ao;
+    DevBuf<float> depth_ao, linemax;
     // job tables
     DevBuf<prk::SetupParams> d_sj, d_mj;
     DevBuf<prk::RasterParams> d_rj, d_fj;
@@ -1646,11 +1660,13 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
     p.n_first = nfirst;
     p.n_smap = nsm;
     int rc;
+    bool any_ao = false;
+    for (uint32_t v = 0; v < nv; v++) any_ao |= b->scenes[views[v].scene]->sb.has_ao;
     if ((rc = b->rrec.ensure(std::max<size_t>(rec, 1))) || (rc = b->arec.ensure(std::max<size_t>(p.n_rec_main, 1))) ||
         (rc = b->tasks.ensure(std::max<size_t>(task, 1))) || (rc = b->first_rec.ensure(nfirst)) ||
         (rc = b->clip_list.ensure(nfirst)) || (rc = b->cnt.ensure(nv + p.S)) || (rc = b->keys.ensure(npx)) ||
         (rc = b->nanseq.ensure(npx)) || (rc = b->beaten.ensure(npx)) || (rc = b->win.ensure(npx)) ||
-        (rc = b->ao_list.ensure(npx)) || (rc = b->depth_ao.ensure(npx)) || (rc = b->chunk.ensure(nv)) ||
+        (rc = b->ao_list.ensure(npx)) || (rc = b->depth_ao.ensure(npx)) || (rc = b->linemax.ensure(any_ao ? 4 * npx : 1)) || (rc = b->chunk.ensure(nv)) ||
         (rc = b->smaps.ensure(std::max<size_t>(nsm, 1))))
         return rc;
     if (b->h_cnt_n < nv + p.S) {
@@ -1797,6 +1813,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
                                           ap.dir_tiny);
         ap.depth = R.depth_ao;
         ap.list = sp.ao_list;
+        ap.linemax = b->linemax.p + (any_ao ? 4 * o : 0);
         ap.cnt = mp.cnt;
         ap.rgba = sp.rgba;
         std::memcpy(ap.gamma, sp.gamma, 256);
@@ -1870,8 +1887,9 @@ int batch_launch(Batch* b, const BatchPlan& p, uint32_t* launches) {
     KTRY(prk::launch_raster_batch(b->d_fj.p, b->d_fitems.p, (int)V, b->d_queue.p + 1, b->n_sms * b->raster_bps, st));
     KTRY(prk::launch_resolve_batch(b->d_res.p, blk_r, (int)V, p.nb_r, st));
     KTRY(prk::launch_shade_batch(b->d_sh.p, blk_sh, (int)V, p.nb_sh, st));
+    KTRY(prk::launch_ao_linemax_batch(b->d_ao.p, blk_sh, (int)V, p.nb_sh, st));
     KTRY(prk::launch_ao_batch(b->d_ao.p, (int)V, b->chunk.p, b->n_sms * 4, st));
-    n += 10;
+    n += 11;
     CUDA_TRY(cudaMemcpyAsync(b->h_cnt, b->cnt.p, sizeof(prk::Counters) * (V + S), cudaMemcpyDeviceToHost, st));
     *launches = n;
     return PR_OK;
@@ -1974,7 +1992,8 @@ int batch_run(Batch* b, uint32_t nv, const pr_batch_view* views) {
         }
         size_t bytes = dev_bytes(b->rrec) + dev_bytes(b->arec) + dev_bytes(b->tasks) + dev_bytes(b->first_rec) +
                        dev_bytes(b->clip_list) + dev_bytes(b->keys) + dev_bytes(b->nanseq) + dev_bytes(b->beaten) +
-                       dev_bytes(b->win) + dev_bytes(b->ao_list) + dev_bytes(b->depth_ao) + dev_bytes(b->smaps);
+                       dev_bytes(b->win) + dev_bytes(b->ao_list) + dev_bytes(b->depth_ao) + dev_bytes(b->linemax) +
+                       dev_bytes(b->smaps);
         b->stats.device_bytes = bytes;
         if (grow) {
             b->stats.n_retries++;
@@ -2039,7 +2058,7 @@ int pr_batch_destroy(void* batch) {
     for (Ctx* c : b->scenes) pr_destroy(c);
     b->rrec.release(); b->arec.release(); b->tasks.release(); b->first_rec.release(); b->clip_list.release();
     b->cnt.release(); b->keys.release(); b->nanseq.release(); b->beaten.release(); b->win.release();
-    b->ao_list.release(); b->chunk.release(); b->smaps.release(); b->depth_ao.release();
+    b->ao_list.release(); b->chunk.release(); b->smaps.release(); b->depth_ao.release(); b->linemax.release();
     b->d_sj.release(); b->d_mj.release(); b->d_rj.release(); b->d_fj.release(); b->d_res.release();
     b->d_sh.release(); b->d_ao.release(); b->d_blk.release(); b->d_items.release(); b->d_fitems.release();
     b->d_queue.release();

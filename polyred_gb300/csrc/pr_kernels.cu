@@ -1128,18 +1128,53 @@ PR_DEV void resolve_one(int W, int H, const unsigned long long* keys, const uint
     depth_ao[i] = d;
 }
 
+// The line maxima of a frame's depths, which AO's march skips taps by: plane
+// 0 along x, 1 along the rows, 2 along the diagonal, 3 along the antidiagonal,
+// each entry the maximum of the kLineReach + 1 cells that start at its pixel
+// in memory order. One 32 x 8 tile per 256-thread block; depth(x, row) of any
+// pixel of the frame. Bound by its 16 B of stores a pixel.
+constexpr int kLineReach = 3;
+template <class F>
+PR_DEV void ao_linemax_tile(int W, int H, int x0, int r0, float* linemax, F depth) {
+    constexpr int TW = 32 + 2 * kLineReach, TH = 8 + kLineReach;
+    __shared__ float s_d[TH][TW];
+    const int tid = threadIdx.x + threadIdx.y * blockDim.x, tx = tid & 31, ty = tid >> 5;
+    for (int e = tid; e < TH * TW; e += 256) {
+        const int q = e / TW, c = e - q * TW, x = x0 + c - kLineReach, r = r0 + q;
+        s_d[q][c] = (x >= 0 && x < W && r < H) ? depth(x, r) : -3.40282347e38f;
+    }
+    __syncthreads();
+    const int x = x0 + tx, r = r0 + ty;
+    if (x >= W || r >= H) return;
+    const int c = tx + kLineReach;
+    float m[4];
+    m[0] = m[1] = m[2] = m[3] = s_d[ty][c];
+#pragma unroll
+    for (int j = 1; j <= kLineReach; j++) {
+        m[0] = fmaxf(m[0], s_d[ty][c + j]);
+        m[1] = fmaxf(m[1], s_d[ty + j][c]);
+        m[2] = fmaxf(m[2], s_d[ty + j][c + j]);
+        m[3] = fmaxf(m[3], s_d[ty + j][c - j]);
+    }
+    const size_t i = (size_t)r * W + x, plane = (size_t)W * H;
+#pragma unroll
+    for (int q = 0; q < 4; q++) linemax[q * plane + i] = m[q];
+}
+
 // Resolve (resolve_one) that also lists the winners' deferred attribute
 // records (the first pixel to find its record pending, 1 -> 2, appends it)
 // and, with ao_list, the frame's AO pixels: every covered pixel whose winning
 // triangle's material has AO (tri_flags kTriAO; AmbientOcclusionShade's own
 // condition, material/ao.go:22), appended tile by tile (32 x 8 blocks, warps
-// in order) for the march's locality. One atomic per block and list.
+// in order) for the march's locality, and writes the line maxima of the
+// frame's depths (a halo of kLineReach keys more per tile). One atomic per
+// block and list.
 __global__ void __launch_bounds__(256) resolve_listing_kernel(int W, int H, const unsigned long long* keys,
                                                               uint32_t* nanseq, uint32_t* beaten,
                                                               Counters* cnt, uint32_t* win, float* depth_ao,
                                                               const uint32_t* first_rec, uint32_t* attr_state,
                                                               uint32_t* vis, const uint8_t* tri_flags,
-                                                              uint32_t* ao_list) {
+                                                              uint32_t* ao_list, float* linemax) {
     const int x = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
     const int lane = threadIdx.x, warp = threadIdx.y;
     bool want = false, ao = false;
@@ -1185,6 +1220,11 @@ __global__ void __launch_bounds__(256) resolve_listing_kernel(int W, int H, cons
         for (int q = 0; q < warp; q++) o += s_cnt[1][q];
         ao_list[o] = (uint32_t)i;
     }
+    if (ao_list && !cnt->nan_flag)  // uniform; a frame with NaN depths marches without them
+        ao_linemax_tile(W, H, blockIdx.x * 32, blockIdx.y * 8, linemax, [&](int cx, int cr) {
+            const unsigned long long key = keys[(size_t)cr * W + cx];
+            return key != 0ull ? fkey_decode((uint32_t)(key >> 32)) : -1.0f;
+        });
 }
 
 // The deferred attribute records of the listed records: everything comes
@@ -1648,9 +1688,40 @@ __global__ void __launch_bounds__(256, 4) shade_kernel(const __grid_constant__ S
 __constant__ float c_ao_dir[2][8];
 
 constexpr int kAoTaps = 100;     // t = 0 .. 99 (material/ao.go:44)
-constexpr int kAoTable = 100;    // tap offsets for t = 2 .. 101 (t >= 100: padding, offset 0)
+constexpr int kAoTable = 100;    // tap offsets for t = 2 .. 101 (t >= 100: padding)
 constexpr float kAoSkip = 1.0f - 0x1p-20f;
 constexpr int kAoThreads = 256;
+constexpr int kAoGroups = kAoTable / 4;  // groups of four taps: 2 .. 5, 6 .. 9, ...
+constexpr int kNearGroups = 2;           // groups always looked at tap by tap
+constexpr int kAoWin = 24;               // line windows, one per later group (the last entry is neutral)
+static_assert(kAoGroups - kNearGroups <= kAoWin && kAoWin % 4 == 0, "one window per group, four at a time");
+
+// A block's tap tables in shared memory: per (direction, tap) the byte
+// offset and bounds on 1/dist, and the same per (direction, line window).
+struct __align__(16) AoTables {
+    int off[8][kAoTable];
+    float rlo[8][kAoTable], rhi[8][kAoTable];
+    int woff[8][kAoWin];
+    float wlo[8][kAoWin], whi[8][kAoWin];
+};
+
+// Bounds on 1/dist of a tap at p + (ax, ay). Along an axis (ax or ay an
+// integer t, the other below 2^-16) dist is t itself: p + t is exact, and the
+// other's square, at most 2^-30, is lost in t^2. Else
+// |dist - |(ax, ay)|| <= sqrt(2) (h + 2^-18) + 2.5e-7 |(ax, ay)|: h bounds the rounding of
+// cur = RN(p + a), 2^-18 that of p - cur, the rest the float32 steps of both distances
+PR_DEV void ao_inv_dist(const AoParams& P, float ax, float ay, float* rlo, float* rhi) {
+    const float t = fmaxf(fabsf(ax), fabsf(ay));
+    if (fminf(fabsf(ax), fabsf(ay)) < 0x1p-16f && t == floorf(t)) {
+        *rlo = __frcp_rd(t);
+        *rhi = __frcp_ru(t);
+        return;
+    }
+    const float d0 = __fsqrt_rn(__fmaf_rn(ax, ax, __fmul_rn(ay, ay)));
+    const float dl = __fadd_ru(__fmul_ru(1.5f, __fadd_ru(P.ao_half_ulp, 4e-6f)), __fmul_ru(d0, 4e-7f));
+    *rlo = __frcp_rd(__fadd_ru(d0, dl));
+    *rhi = __frcp_ru(__fsub_rd(d0, dl));
+}
 
 // distance of material/ao.go:52, p.Sub(cur).Len() with z = w = 0
 PR_DEV float ao_distance(float pxf, float pyf, float cx, float cy) {
@@ -1686,12 +1757,16 @@ PR_DEV bool ao_tap_exact(int t, float pxf, float pyf, float dX, float dY, int W,
     return true;
 }
 
+// p[0] moved by a signed number of bytes; base at an unsigned one (32-bit sums: one add per load)
+PR_DEV float ld_at(const float* p, int bytes) { return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + bytes)); }
+PR_DEV float ld_at_u(const float* base, uint32_t bytes) { return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(base) + bytes)); }
+
 // The elevation of fast-path tap t again (settling a pending tap reloads it
 // instead of carrying it).
 PR_DEV float ao_tap_elev(const int (*s_off)[kAoTable], int k, int t, const float* p0, const float* pA, int tstar, float z,
                          bool tiny) {
     const float* q = (tiny && t < tstar) ? pA : p0;
-    return __fsub_rn(__ldg(q + s_off[k][t - 2]), z);
+    return __fsub_rn(ld_at(q, s_off[k][t - 2]), z);
 }
 
 // maxElevationAngle's march for taps 2 .. 101 in groups of four, from shared
@@ -1720,10 +1795,11 @@ PR_DEV bool ao_fast_groups(int n_groups, const int (*s_off)[kAoTable], const flo
         const float* q2 = (TINY && t0 + 2 < tstar) ? pA : p0;
         const float* q3 = (TINY && t0 + 3 < tstar) ? pA : p0;
         float el[4], hi[4];
-        el[0] = __fsub_rn(__ldg(q0 + o.x), z);
-        el[1] = __fsub_rn(__ldg(q1 + o.y), z);
-        el[2] = __fsub_rn(__ldg(q2 + o.z), z);
-        el[3] = __fsub_rn(__ldg(q3 + o.w), z);
+        el[0] = __fsub_rn(ld_at(q0, o.x), z);
+        el[1] = __fsub_rn(ld_at(q1, o.y), z);
+        el[2] = __fsub_rn(ld_at(q2, o.z), z);
+        el[3] = __fsub_rn(ld_at(q3, o.w), z);
+        if (g == kAoGroups - 1) el[2] = el[3] = 0.0f;  // padding taps
         hi[0] = __fmul_ru(el[0], rh.x);
         hi[1] = __fmul_ru(el[1], rh.y);
         hi[2] = __fmul_ru(el[2], rh.z);
@@ -1787,78 +1863,118 @@ __device__ __noinline__ float ao_settle_group(const int (*s_off)[kAoTable], cons
     return r;
 }
 
-// The march of ao_fast_groups for frames without NaN depths, bookkept per
-// unit of two groups of four taps (eight taps; a last odd group alone): a
-// unit is a candidate when the largest upper bound of its taps exceeds lb;
-// it then raises lb by the largest lower bound of its taps and becomes the
-// pending unit (bounded above by that largest upper bound phi). A pending
-// unit is settled (its taps above lb evaluated exactly, group by group) only
-// when a later candidate's lower bound does not clear phi, and at the end.
-// Every tap above the final lb is thus evaluated exactly, and best is the
-// exact maximum, whatever the unit's size; eight taps per unit halve the
-// candidate steps a warp issues (some lane of a warp is a candidate in most
-// units). UNROLL: the unit loop unrolled by two (the single-view kernel, at
-// 64 registers; the batched kernel keeps one unit at a time).
-template <bool TINY, bool UNROLL>
-PR_DEV void ao_fast_groups_nf(int n_groups, const int (*s_off)[kAoTable], const float (*s_rlo)[kAoTable],
-                              const float (*s_rhi)[kAoTable], int k, const float* p0, const float* pA, int tstar,
-                              float z, float pxf, float pyf, float dX, float dY, float& best) {
-    float lb = best;
-    int pg = -1, pn = 0;  // pending unit: first group, group count
-    float phi = 0.0f;
-    // the elevations of group g's taps and the largest upper bound of their ratios
-    auto group_hi = [&](int g, float& gh, float e[4]) {
+// A direction's term of the total, RN(HalfPi - float32(Atan(x))), for its
+// largest ratio x >= 0. Up to 2.4e-4, x^3/3 is below a quarter of the gap to
+// the float32 below x, and atan_f32 is x itself.
+PR_DEV float ao_term(float x) {
+    return __fsub_rn(1.57079632679489661923f, x <= 2.4e-4f ? x : atan_f32(x));
+}
+// The largest ratio known to give the same term r = ao_term(lb) as lb: for
+// lb <= x <= cut, Atan(lb) <= Atan(x) <= x, and HalfPi - x lies less than half
+// an ulp of r (2^-24, r in (1, 2)) below r.
+PR_DEV float ao_cut(float lb, float r) {
+    return r > 1.0f ? fmaxf(lb, __fadd_rd(__fsub_rn(1.57079632679489661923f, r), 5.96e-8f)) : lb;
+}
+
+// The march of ao_fast_groups for frames without NaN depths: the term of one
+// direction, whose taps outside the groups have the exact maximum best. All
+// 32 lanes call, each with a pixel of its own.
+// A term has 2^-23 steps and most ratios are below 1e-3, so bounds on the
+// largest ratio usually fix it: lb <= ratio <= ub, and every tap that cannot
+// exceed cut (ao_cut(lb)) is left out. The nearest two groups are looked at
+// tap by tap; each group after them first as a whole, by its line maximum
+// (ao_linemax_tile): the largest elevation among the window's four cells
+// times the bounds on 1/dist of its nearest and its farthest tap bounds the
+// window's largest ratio from both sides. A group that some lane's ratio may
+// exceed the cut in is then looked at tap by tap, by all lanes at once (their
+// pixels are neighbours, a group costs a third of a divergent lane's). Where
+// the terms of lb and ub differ, the lane's open groups are evaluated exactly.
+// GEN: lanes may have fewer groups than all, or a tiny component that crosses
+// among their taps (b0 from tap tstar on, bA before); else every lane has
+// all groups at b0.
+// b0, bA: byte offsets of the pixel in depth and lm (frames hold at most 2^28
+// pixels), moved by a column or row for a tiny component; either may wrap
+// below 0, and offset sums wrap back. pix: the pixel's own.
+template <bool GEN>
+PR_DEV float ao_march(int n_groups, const AoTables& S, int k, const float* depth, uint32_t pix, uint32_t b0, uint32_t bA,
+                      int tstar, float z, const float* lm, float pxf, float pyf, float dX, float dY, float best) {
+    float lb = best, ub = best, cut = ao_cut(lb, ao_term(lb));
+    unsigned open = 0;  // groups with a tap that may exceed the cut
+    auto look = [&](int g) {
         const int t0 = 4 * g + 2;
-        const int4 o = *reinterpret_cast<const int4*>(&s_off[k][4 * g]);
-        const float4 rh = *reinterpret_cast<const float4*>(&s_rhi[k][4 * g]);
-        const float* q0 = (TINY && t0 < tstar) ? pA : p0;
-        const float* q1 = (TINY && t0 + 1 < tstar) ? pA : p0;
-        const float* q2 = (TINY && t0 + 2 < tstar) ? pA : p0;
-        const float* q3 = (TINY && t0 + 3 < tstar) ? pA : p0;
-        e[0] = __fsub_rn(__ldg(q0 + o.x), z);
-        e[1] = __fsub_rn(__ldg(q1 + o.y), z);
-        e[2] = __fsub_rn(__ldg(q2 + o.z), z);
-        e[3] = __fsub_rn(__ldg(q3 + o.w), z);
-        gh = fmaxf(fmaxf(__fmul_ru(e[0], rh.x), __fmul_ru(e[1], rh.y)), fmaxf(__fmul_ru(e[2], rh.z), __fmul_ru(e[3], rh.w)));
+        const int4 o = *reinterpret_cast<const int4*>(&S.off[k][4 * g]);
+        const float4 rh = *reinterpret_cast<const float4*>(&S.rhi[k][4 * g]);
+        uint32_t q[4] = {b0 + (uint32_t)o.x, b0 + (uint32_t)o.y, b0 + (uint32_t)o.z, b0 + (uint32_t)o.w};
+        if (GEN) {
+            const uint32_t d = bA - b0;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (t0 + u < tstar) q[u] += d;
+                if (g >= n_groups) q[u] = pix;  // elevation 0
+            }
+        }
+        float e[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) e[u] = __fsub_rn(ld_at_u(depth, q[u]), z);
+        const float gh = fmaxf(fmaxf(__fmul_ru(e[0], rh.x), __fmul_ru(e[1], rh.y)),
+                               fmaxf(__fmul_ru(e[2], rh.z), __fmul_ru(e[3], rh.w)));
+        if (gh > cut) {
+            const float4 rl = *reinterpret_cast<const float4*>(&S.rlo[k][4 * g]);
+            const float gl = fmaxf(fmaxf(__fmul_rd(e[0], rl.x), __fmul_rd(e[1], rl.y)),
+                                   fmaxf(__fmul_rd(e[2], rl.z), __fmul_rd(e[3], rl.w)));
+            lb = fmaxf(lb, gl);
+            ub = fmaxf(ub, gh);
+            cut = fmaxf(cut, lb);
+            open |= 1u << g;
+        }
     };
-    auto group_lo = [&](int g, const float e[4]) {
-        const float4 rl = *reinterpret_cast<const float4*>(&s_rlo[k][4 * g]);
-        return fmaxf(fmaxf(__fmul_rd(e[0], rl.x), __fmul_rd(e[1], rl.y)), fmaxf(__fmul_rd(e[2], rl.z), __fmul_rd(e[3], rl.w)));
-    };
-    auto settle = [&]() {
-        for (int q = 0; q < pn; q++)
-            best = fmaxf(best, ao_settle_group<TINY>(s_off, s_rhi, k, pg + q, p0, pA, tstar, z, pxf, pyf, dX, dY, lb));
+#pragma unroll
+    for (int g = 0; g < kNearGroups; g++) look(g);
+    unsigned todo = 0;  // groups (less kNearGroups) to be looked at tap by tap
+#pragma unroll 2
+    for (int w4 = 0; w4 < kAoWin; w4 += 4) {
+        const int4 o = *reinterpret_cast<const int4*>(&S.woff[k][w4]);
+        const float4 rh = *reinterpret_cast<const float4*>(&S.whi[k][w4]);
+        const float4 rl = *reinterpret_cast<const float4*>(&S.wlo[k][w4]);
+        const int oo[4] = {o.x, o.y, o.z, o.w};
+        const float hh[4] = {rh.x, rh.y, rh.z, rh.w}, ll[4] = {rl.x, rl.y, rl.z, rl.w};
+        float e[4];
+        bool split[4], out[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int t1 = 4 * (w4 + u + kNearGroups) + 5;  // the group's last tap; a window reaches back to t1 - 5
+            uint32_t q = b0 + (uint32_t)oo[u];
+            split[u] = out[u] = false;
+            if (GEN) {
+                out[u] = w4 + u + kNearGroups >= n_groups;
+                split[u] = tstar <= t1 && tstar > t1 - 6;  // the crossing tap lies inside the window
+                if (t1 < tstar) q += bA - b0;
+                if (out[u] || split[u]) q = pix;
+            }
+            e[u] = __fsub_rn(ld_at_u(lm, q), z);
+        }
+        float l = lb;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (!out[u] && (split[u] || __fmul_ru(e[u], hh[u]) > cut)) todo |= 1u << (w4 + u);
+            if (!out[u] && !split[u]) l = fmaxf(l, __fmul_rd(e[u], ll[u]));
+        }
+        lb = l;
+        cut = fmaxf(cut, l);
+    }
+    todo = __reduce_or_sync(0xffffffffu, todo & ((1u << (kAoGroups - kNearGroups)) - 1u));
+    cut = fmaxf(cut, ao_cut(lb, ao_term(lb)));
+    for (; todo; todo &= todo - 1u) look(__ffs(todo) - 1 + kNearGroups);
+    const float r = ao_term(lb);
+    if (ub <= ao_cut(lb, r) || ao_term(ub) == r) return r;
+    while (open) {
+        const int g = __ffs(open) - 1;
+        open &= open - 1u;
+        best = fmaxf(best, ao_settle_group<GEN>(S.off, S.rhi, k, g, depth + ((int)b0 >> 2), depth + ((int)bA >> 2), tstar, z,
+                                                pxf, pyf, dX, dY, lb));
         lb = fmaxf(lb, best);
-    };
-    int g = 0;
-#pragma unroll(UNROLL ? 2 : 1)
-    for (; g + 1 < n_groups; g += 2) {
-        float ea[4], eb[4], ha, hb;
-        group_hi(g, ha, ea);
-        group_hi(g + 1, hb, eb);
-        const float gh = fmaxf(ha, hb);
-        if (gh > lb) {
-            const float gl = fmaxf(group_lo(g, ea), group_lo(g + 1, eb));
-            lb = fmaxf(lb, gl);
-            if (pg >= 0 && gl < phi) settle();
-            pg = g;
-            pn = 2;
-            phi = gh;
-        }
     }
-    if (g < n_groups) {  // the last group alone
-        float e[4], gh;
-        group_hi(g, gh, e);
-        if (gh > lb) {
-            const float gl = group_lo(g, e);
-            lb = fmaxf(lb, gl);
-            if (pg >= 0 && gl < phi) settle();
-            pg = g;
-            pn = 1;
-            phi = gh;
-        }
-    }
-    if (pg >= 0) settle();
+    return ao_term(lb);  // a tap left out lies between an earlier lb and its cut, where the term is the same
 }
 
 // AmbientOcclusionShade (material/ao.go:20-73) for the pixels the shade
@@ -1886,126 +2002,196 @@ PR_DEV void ao_fast_groups_nf(int n_groups, const int (*s_off)[kAoTable], const 
 // tiny component. Taps with cur < 0 (int truncates toward zero there) and
 // the last taps that do not fill a group of four take the float path.
 // Tap 1 always takes it: its distance may fall below 1 (diagonals).
+
 // The tap tables of a W x H frame (every thread of the block calls).
-PR_DEV void ao_tables(const AoParams& P, int (*s_off)[kAoTable], float (*s_rlo)[kAoTable], float (*s_rhi)[kAoTable]) {
+PR_DEV void ao_tables(const AoParams& P, AoTables& S) {
     const int W = P.W;
     for (int e = threadIdx.x; e < 8 * kAoTable; e += blockDim.x) {
         const int k = e / kAoTable, q = e - k * kAoTable, t = q + 2;
         int o = 0;
         float rlo = 0.0f, rhi = 0.0f;
-        if (t < kAoTaps && k < P.n_dirs) {
-            const float tf = small_u2f((uint32_t)t);
+        if (k < P.n_dirs) {
+            // the padding taps 100, 101 read the last tap's cell, with bounds 0
+            const float tf = small_u2f((uint32_t)min(t, kAoTaps - 1));
             const float ax = __fmul_rn(c_ao_dir[0][k], tf), ay = __fmul_rn(c_ao_dir[1][k], tf);
             o = (int)floorf(ax) - (int)floorf(ay) * W;
-            // |dist - |(ax, ay)|| <= sqrt(2) (h + 2^-18) + 2.5e-7 |(ax, ay)|: h bounds the rounding of
-            // cur = RN(p + a), 2^-18 that of p - cur, the rest the float32 steps of both distances
-            const float d0 = __fsqrt_rn(__fmaf_rn(ax, ax, __fmul_rn(ay, ay)));
-            const float dl = __fadd_ru(__fmul_ru(1.5f, __fadd_ru(P.ao_half_ulp, 4e-6f)), __fmul_ru(d0, 4e-7f));
-            rlo = __frcp_rd(__fadd_ru(d0, dl));
-            rhi = __frcp_ru(__fsub_rd(d0, dl));
+            if (t < kAoTaps) ao_inv_dist(P, ax, ay, &rlo, &rhi);
         }
-        s_off[k][q] = o;
-        s_rlo[k][q] = rlo;
-        s_rhi[k][q] = rhi;
+        S.off[k][q] = 4 * o;
+        S.rlo[k][q] = rlo;
+        S.rhi[k][q] = rhi;
+    }
+    // the line window of each group after the nearest: the four cells that end at the cell of its last tap t1
+    for (int e = threadIdx.x; e < 8 * kAoWin; e += blockDim.x) {
+        // the neutral last entry reads the window before it, with bounds 0
+        const int k = e / kAoWin, w = e - k * kAoWin, g = min(w + kNearGroups, kAoGroups - 1);
+        int o = 0;
+        float lo = 0.0f, hi = 0.0f;
+        if (k < P.n_dirs) {
+            const float cx = c_ao_dir[0][k], cy = c_ao_dir[1][k];
+            const int t1 = min(4 * g + 5, kAoTaps - 1);
+            auto cell_x = [&](int t) { return (int)floorf(__fmul_rn(cx, small_u2f((uint32_t)t))); };
+            auto cell_y = [&](int t) { return (int)floorf(__fmul_rn(cy, small_u2f((uint32_t)t))); };
+            auto reach = [&](int t) { return max(abs(cell_x(t1) - cell_x(t)), abs(cell_y(t1) - cell_y(t))); };
+            int t0 = t1;  // the window's nearest tap
+            while (t0 > 2 && reach(t0 - 1) <= kLineReach) t0--;
+            const int near = cell_x(t0) - cell_y(t0) * W, far = cell_x(t1) - cell_y(t1) * W;
+            o = min(near, far);
+            float a, b;
+            ao_inv_dist(P, __fmul_rn(cx, small_u2f((uint32_t)t0)), __fmul_rn(cy, small_u2f((uint32_t)t0)), &a, &hi);
+            ao_inv_dist(P, __fmul_rn(cx, small_u2f((uint32_t)t1)), __fmul_rn(cy, small_u2f((uint32_t)t1)), &lo, &b);
+            if (w + kNearGroups >= kAoGroups) lo = hi = 0.0f;
+        }
+        S.woff[k][w] = 4 * o;
+        S.wlo[k][w] = lo;
+        S.whi[k][w] = hi;
     }
 }
 
 PR_DEV void ao_finish(const AoParams& P, uint32_t i, float T);
 
-// One pixel of the AO list: its total T, then (kApply) the colour scaling,
-// or (!kApply) T stored for ao_apply_kernel.
-template <bool kApply>
-PR_DEV void ao_one(const AoParams& P, uint32_t j, const int (*s_off)[kAoTable], const float (*s_rlo)[kAoTable],
-                   const float (*s_rhi)[kAoTable]) {
-    const int W = P.W, H = P.H;
-    const float fW = (float)W, fH = (float)H;
-    const uint32_t i = P.list[j];
-    const int r = (int)(i / (uint32_t)W);
-    const int x = (int)i - r * W;
-    const int y = H - 1 - r;
+// A pixel's march along direction k: the first tap outside the frame and the
+// first with cur < 0 (kAoTaps: none), by binary search.
+PR_DEV void ao_reach(const AoParams& P, float pxf, float pyf, float dX, float dY, int* t_end, int* t_fast) {
+    const float fW = (float)P.W, fH = (float)P.H;
+    const float cx = __fadd_rn(pxf, __fmul_rn(dX, 99.0f)), cy = __fadd_rn(pyf, __fmul_rn(dY, 99.0f));
+    *t_end = *t_fast = kAoTaps;
+    if (cx >= 0.0f && cx < fW && cy >= 0.0f && cy < fH) return;
+    int lo = 1, hi = kAoTaps;  // first tap outside (-1, W) x (-1, H), then first tap with cur < 0
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        const float tf = small_u2f((uint32_t)mid);
+        const float mx = __fadd_rn(pxf, __fmul_rn(dX, tf)), my = __fadd_rn(pyf, __fmul_rn(dY, tf));
+        if (mx > -1.0f && mx < fW && my > -1.0f && my < fH)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    *t_end = lo;
+    hi = lo;
+    lo = 1;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        const float tf = small_u2f((uint32_t)mid);
+        const float mx = __fadd_rn(pxf, __fmul_rn(dX, tf)), my = __fadd_rn(pyf, __fmul_rn(dY, tf));
+        if (mx >= 0.0f && my >= 0.0f)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    *t_fast = lo;
+}
+
+// The tap t* of a tiny component c at coordinate p: the first with |c t| above half the gap below p.
+PR_DEV int ao_tiny_cross(float c, float p) {
+    const float cf = fabsf(c);
+    const uint32_t vb = __float_as_uint(p);
+    const float h = __uint_as_float(((vb >> 23) - ((vb & 0x7fffffu) ? 24u : 25u)) << 23);
+    if (!(__fmul_rn(cf, 99.0f) > h)) return kAoTaps;
+    int lo = 1, hi = kAoTaps - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (__fmul_rn(cf, small_u2f((uint32_t)mid)) > h)
+            hi = mid;
+        else
+            lo = mid + 1;
+    }
+    return lo;
+}
+
+// Pixel i's total T in a frame with NaN depths (NaN: a direction met one).
+__device__ __noinline__ float ao_total_nan(const AoParams& P, uint32_t i, const AoTables& S) {
+    const int W = P.W, H = P.H, r = (int)(i / (uint32_t)W), x = (int)i - r * W, y = H - 1 - r;
     const float* p0 = P.depth + i;
     const float z = *p0;
     const float pxf = small_u2f((uint32_t)x), pyf = small_u2f((uint32_t)y);
-    // no NaN-depth fragment reached this frame's depth buffer (the raster flags every one)
-    const bool nan_free = P.cnt->nan_flag == 0u;
     float total = 0.0f;
-    bool nanpix = false;
     for (int k = 0; k < P.n_dirs; k++) {
         const float dX = c_ao_dir[0][k], dY = c_ao_dir[1][k];
-        int t_end = kAoTaps, t_fast = kAoTaps;
-        {
-            const float cx = __fadd_rn(pxf, __fmul_rn(dX, 99.0f)), cy = __fadd_rn(pyf, __fmul_rn(dY, 99.0f));
-            if (!(cx >= 0.0f && cx < fW && cy >= 0.0f && cy < fH)) {
-                // first tap outside (-1, W) x (-1, H), then first tap with cur < 0
-                int lo = 1, hi = kAoTaps;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    const float tf = small_u2f((uint32_t)mid);
-                    const float mx = __fadd_rn(pxf, __fmul_rn(dX, tf)), my = __fadd_rn(pyf, __fmul_rn(dY, tf));
-                    if (mx > -1.0f && mx < fW && my > -1.0f && my < fH)
-                        lo = mid + 1;
-                    else
-                        hi = mid;
-                }
-                t_end = lo;
-                lo = 1;
-                hi = t_end;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    const float tf = small_u2f((uint32_t)mid);
-                    const float mx = __fadd_rn(pxf, __fmul_rn(dX, tf)), my = __fadd_rn(pyf, __fmul_rn(dY, tf));
-                    if (mx >= 0.0f && my >= 0.0f)
-                        lo = mid + 1;
-                    else
-                        hi = mid;
-                }
-                t_fast = lo;
-            }
-        }
-        // the padding taps 100, 101 read the pixel itself: elev 0 needs a finite depth
+        int t_end, t_fast;
+        ao_reach(P, pxf, pyf, dX, dY, &t_end, &t_fast);
+        // the tables' bounds (0 for the padding taps 100, 101) need finite elevations of a finite depth
         if (!P.dir_fast[k] || !isfinite(z)) t_fast = 1;
         float best = 0.0f;
         bool ok = true;
         if (t_end > 1) ok = ao_tap_exact(1, pxf, pyf, dX, dY, W, H, P.depth, z, 0.0f, best);
         int t = 2;
         if (ok && t_fast > 2) {
-            const int n_groups = t_fast == kAoTaps ? kAoTable / 4 : (t_fast - 2) >> 2;
+            const int n_groups = t_fast == kAoTaps ? kAoGroups : (t_fast - 2) >> 2;
             const int tiny = P.dir_tiny[k];
-            if (tiny) {
-                // t*: first tap with |a| above half the gap below the coordinate
-                const float cf = fabsf(tiny == 1 ? dX : dY);
-                const uint32_t vb = __float_as_uint(tiny == 1 ? pxf : pyf);
-                const float h = __uint_as_float(((vb >> 23) - ((vb & 0x7fffffu) ? 24u : 25u)) << 23);
-                int lo = 1, hi = kAoTaps;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (__fmul_rn(cf, small_u2f((uint32_t)mid)) > h)
-                        hi = mid;
-                    else
-                        lo = mid + 1;
-                }
-                const float* pA = p0 + (tiny == 1 ? 1 : -W);
-                if (nan_free)
-                    ao_fast_groups_nf<true, !kApply>(n_groups, s_off, s_rlo, s_rhi, k, p0, pA, lo, z, pxf, pyf, dX, dY,
-                                                     best);
-                else
-                    ok = ao_fast_groups<true>(n_groups, s_off, s_rlo, s_rhi, k, p0, pA, lo, z, pxf, pyf, dX, dY, best);
-            } else if (nan_free) {
-                ao_fast_groups_nf<false, !kApply>(n_groups, s_off, s_rlo, s_rhi, k, p0, p0, 0, z, pxf, pyf, dX, dY, best);
-            } else {
-                ok = ao_fast_groups<false>(n_groups, s_off, s_rlo, s_rhi, k, p0, p0, 0, z, pxf, pyf, dX, dY, best);
-            }
+            if (tiny)
+                ok = ao_fast_groups<true>(n_groups, S.off, S.rlo, S.rhi, k, p0, p0 + (tiny == 1 ? 1 : -W),
+                                          ao_tiny_cross(tiny == 1 ? dX : dY, tiny == 1 ? pxf : pyf), z, pxf, pyf, dX, dY, best);
+            else
+                ok = ao_fast_groups<false>(n_groups, S.off, S.rlo, S.rhi, k, p0, p0, 0, z, pxf, pyf, dX, dY, best);
             t = 2 + 4 * n_groups;
         }
         for (; ok && t < t_end; t++) ok = ao_tap_exact(t, pxf, pyf, dX, dY, W, H, P.depth, z, best, best);
-        if (!ok) {
-            nanpix = true;
-            break;
-        }
-        const float ma = best > 0.0f ? atan_f32(best) : 0.0f;
-        total = __fadd_rn(total, __fsub_rn(1.57079632679489661923f, ma));  // HalfPi - angle
+        if (!ok) return __uint_as_float(0x7fc00000u);
+        total = __fadd_rn(total, ao_term(best));
     }
-    const float T = nanpix ? __uint_as_float(0x7fc00000u) : __fdiv_rn(total, 12.5663706143591729539f);
+    return __fdiv_rn(total, 12.5663706143591729539f);
+}
+
+// Pixel j of the AO list's n (every lane of a warp calls, those past the end
+// with the last pixel and nothing to write): its total T, then (kApply) the
+// colour scaling, or (!kApply) T stored for ao_apply_kernel.
+template <bool kApply>
+PR_DEV void ao_one(const AoParams& P, uint32_t j, uint32_t n, const AoTables& S) {
+    const bool mine = j < n;
+    const uint32_t i = P.list[min(j, n - 1u)];
+    float T;
+    if (P.cnt->nan_flag != 0u) {  // some NaN-depth fragment reached this frame (the raster flags every one)
+        T = ao_total_nan(P, i, S);
+    } else {
+        const int W = P.W, H = P.H, r = (int)(i / (uint32_t)W), x = (int)i - r * W, y = H - 1 - r;
+        const float z = P.depth[i];
+        const float pxf = small_u2f((uint32_t)x), pyf = small_u2f((uint32_t)y);
+        const bool inner = x >= 100 && x < W - 100 && y >= 100 && y < H - 100 && isfinite(z);  // every tap inside the frame
+        const bool all_inner = __all_sync(0xffffffffu, inner);
+        float total = 0.0f, shut = 0.0f;  // shut: the sum of the angles
+        for (int k = 0; k < P.n_dirs; k++) {
+            const float dX = c_ao_dir[0][k], dY = c_ao_dir[1][k];
+            int t_end = kAoTaps, t_fast = kAoTaps;
+            if (!all_inner) ao_reach(P, pxf, pyf, dX, dY, &t_end, &t_fast);
+            if (!P.dir_fast[k] || !isfinite(z)) t_fast = 1;
+            const int n_groups = t_fast == kAoTaps ? kAoGroups : max(t_fast - 2, 0) >> 2;
+            float best = 0.0f;
+            bool ok = true;  // false: a NaN elevation (z infinite)
+            if (all_inner && fminf(fabsf(dX), fabsf(dY)) < 0x1p-16f)  // along an axis the first tap's dist is 1 (ao_inv_dist)
+                best = fmaxf(0.0f, __fsub_rn(P.depth[i + (fabsf(dX) > 0.5f ? (dX > 0.0f ? 1 : -1) : (dY > 0.0f ? -W : W))], z));
+            else if (t_end > 1)
+                ok = ao_tap_exact(1, pxf, pyf, dX, dY, W, H, P.depth, z, 0.0f, best);
+            // the taps past the last whole group, exactly
+            for (int t = n_groups == kAoGroups ? kAoTaps : 2 + 4 * n_groups; ok && t < t_end; t++)
+                ok = ao_tap_exact(t, pxf, pyf, dX, dY, W, H, P.depth, z, best, best);
+            const int tiny = P.dir_tiny[k];
+            int tstar = 0;
+            const uint32_t pix = 4u * i;
+            uint32_t b0 = pix, bA = pix;
+            if (tiny) {
+                tstar = ao_tiny_cross(tiny == 1 ? dX : dY, tiny == 1 ? pxf : pyf);
+                bA = pix + (uint32_t)(tiny == 1 ? 4 : -4 * W);
+                if (tstar >= kAoTaps) b0 = bA;  // the whole march stays in the pixel's column (or row)
+                if (tstar <= 2 || tstar >= kAoTaps) tstar = 0;
+            }
+            // the line the direction runs along: x, rows, diagonal (x and row grow together), antidiagonal
+            const int line = fabsf(dY) < 0.5f ? 0 : (fabsf(dX) < 0.5f ? 1 : ((dX > 0.0f) != (dY > 0.0f) ? 2 : 3));
+            const float* lm = P.linemax + (size_t)line * ((size_t)W * H);
+            const float term =
+                __all_sync(0xffffffffu, n_groups == kAoGroups && tstar == 0)
+                    ? ao_march<false>(kAoGroups, S, k, P.depth, pix, b0, b0, 0, z, lm, pxf, pyf, dX, dY, best)
+                    : ao_march<true>(n_groups, S, k, P.depth, pix, b0, bA, tstar, z, lm, pxf, pyf, dX, dY, best);
+            total = ok ? __fadd_rn(total, term) : __uint_as_float(0x7fc00000u);
+            // Each term left is at most HalfPi: with the angles so far above 7.6e-3, T <= 1 - 6e-4 whatever they are
+            // (the float32 sum and quotient err by less than 1e-5 of the 5.9e-5 to spare), and ao_scale gives 0,
+            // as it does for NaN.
+            shut = __fadd_rn(shut, __fsub_rn(1.57079632679489661923f, term));
+            if (!P.exact_T && __all_sync(0xffffffffu, shut > 7.6e-3f || !ok)) break;
+        }
+        T = !P.exact_T && shut > 7.6e-3f ? 0.0f : __fdiv_rn(total, 12.5663706143591729539f);
+    }
+    if (!mine) return;
     if (kApply)
         ao_finish(P, i, T);
     else
@@ -2031,19 +2217,29 @@ PR_DEV void ao_finish(const AoParams& P, uint32_t i, float T) {
     P.rgba[i] = make_uchar4(o.x, o.y, o.z, c.w);
 }
 
-// 4 blocks per SM (up to 64 registers): the march's eight-tap units, two
-// at a time, keep sixteen depth loads in flight per thread without spills.
-template <bool kApply>
+// 4 blocks per SM (64 registers). The tap tables come from the context
+// (ao_tables_kernel): building them cost each block of 256 pixels 7% of its
+// instructions. Bound by issue (71% active): 713k pixels at 1920x1080 take
+// 218 us and 171 M warp instructions; every tap compared by itself, eight to
+// a unit, took 286 us and 227 M.
 __global__ void __launch_bounds__(kAoThreads, 4) ao_kernel(const __grid_constant__ AoParams P) {
-    __shared__ __align__(16) int s_off[8][kAoTable];
-    __shared__ __align__(16) float s_rlo[8][kAoTable];
-    __shared__ __align__(16) float s_rhi[8][kAoTable];
+    __shared__ AoTables S;
     const uint32_t n = P.cnt->n_ao;
     if (blockIdx.x * blockDim.x >= n) return;  // whole block: no pixel of the list
-    ao_tables(P, s_off, s_rlo, s_rhi);
+    static_assert(sizeof(AoTables) % 16 == 0, "copied in 16-byte words");
+    for (uint32_t e = threadIdx.x; e < sizeof(AoTables) / 16; e += blockDim.x)
+        reinterpret_cast<uint4*>(&S)[e] = reinterpret_cast<const uint4*>(P.tables)[e];
     __syncthreads();
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-        ao_one<kApply>(P, j, s_off, s_rlo, s_rhi);
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x)
+        ao_one<false>(P, base + threadIdx.x, n, S);
+}
+// The tap tables of a frame size, once per context and size.
+__global__ void __launch_bounds__(kAoThreads) ao_tables_kernel(const __grid_constant__ AoParams P, void* out) {
+    __shared__ AoTables S;
+    ao_tables(P, S);
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < sizeof(AoTables) / 16; e += blockDim.x)
+        reinterpret_cast<uint4*>(out)[e] = reinterpret_cast<const uint4*>(&S)[e];
 }
 
 // The colour scaling of every listed pixel from its stored total.
@@ -2181,13 +2377,22 @@ __global__ void __launch_bounds__(256) shade_batch_kernel(const ShadeParams* vie
     if (P.ao_list) ao_append_tile(P, pending, (uint32_t)r * (uint32_t)P.W + (uint32_t)x);
 }
 
+// The line maxima of every view with AO pixels, on shade_batch_kernel's tiles.
+__global__ void __launch_bounds__(256) ao_linemax_batch_kernel(const AoParams* views, const uint32_t* blk, int n_views) {
+    const int v = job_of(blk, n_views, blockIdx.x);
+    const AoParams& P = views[v];
+    if (P.cnt->nan_flag || P.cnt->n_ao == 0) return;
+    const uint32_t b = blockIdx.x - blk[v], tiles_x = (uint32_t)(P.W + 31) / 32u;
+    const uint32_t ty = b / tiles_x;
+    ao_linemax_tile(P.W, P.H, (int)((b - ty * tiles_x) * 32u), (int)(ty * 8u), P.linemax,
+                    [&](int x, int r) { return P.depth[(size_t)r * P.W + x]; });
+}
+
 // Persistent AO over every view's list, in chunks of one block taken from
 // per-view counters; tap tables rebuilt when the frame size changes.
 __global__ void __launch_bounds__(kAoThreads) ao_batch_kernel(const AoParams* views, int n_views,
                                                                 uint32_t* chunk_ctr) {
-    __shared__ __align__(16) int s_off[8][kAoTable];
-    __shared__ __align__(16) float s_rlo[8][kAoTable];
-    __shared__ __align__(16) float s_rhi[8][kAoTable];
+    __shared__ AoTables S;
     __shared__ uint32_t s_chunk;
     int tab_w = -1, tab_dirs = -1;
     float tab_h = -1.0f;
@@ -2197,7 +2402,7 @@ __global__ void __launch_bounds__(kAoThreads) ao_batch_kernel(const AoParams* vi
         if (n == 0) continue;
         if (P.W != tab_w || P.ao_half_ulp != tab_h || P.n_dirs != tab_dirs) {
             __syncthreads();
-            ao_tables(P, s_off, s_rlo, s_rhi);
+            ao_tables(P, S);
             __syncthreads();
             tab_w = P.W;
             tab_h = P.ao_half_ulp;
@@ -2209,8 +2414,7 @@ __global__ void __launch_bounds__(kAoThreads) ao_batch_kernel(const AoParams* vi
             const uint32_t c = s_chunk;
             __syncthreads();
             if (c * blockDim.x >= n) break;
-            const uint32_t j = c * blockDim.x + threadIdx.x;
-            if (j < n) ao_one<true>(P, j, s_off, s_rlo, s_rhi);
+            ao_one<true>(P, c * blockDim.x + threadIdx.x, n, S);
         }
     }
 }
@@ -2255,11 +2459,11 @@ int launch_setup_main_only(const SetupParams& p, uint32_t* clip_list, void* stre
 int launch_resolve_listing(int W, int H, const unsigned long long* keys, uint32_t* nanseq, uint32_t* beaten,
                            Counters* cnt, uint32_t* win, float* depth_ao, const uint32_t* first_rec,
                            uint32_t* attr_state, uint32_t* vis, const uint8_t* tri_flags, uint32_t* ao_list,
-                           void* stream) {
+                           float* linemax, void* stream) {
     if (W <= 0 || H <= 0) return 0;
     const dim3 blk(32, 8), grd((unsigned)((W + 31) / 32), (unsigned)((H + 7) / 8));
     resolve_listing_kernel<<<grd, blk, 0, (cudaStream_t)stream>>>(W, H, keys, nanseq, beaten, cnt, win, depth_ao,
-                                                                 first_rec, attr_state, vis, tri_flags, ao_list);
+                                                                 first_rec, attr_state, vis, tri_flags, ao_list, linemax);
     return check(cudaGetLastError());
 }
 int launch_attr(const SetupParams& p, const uint32_t* vis, void* stream) {
@@ -2429,13 +2633,23 @@ int launch_msaa_resize(const uchar4* in, int in_w, int in_h, uchar4* out, int w,
     return check(cudaGetLastError());
 }
 
+size_t ao_tables_bytes() { return sizeof(AoTables); }
+int launch_ao_tables(const AoParams& p, void* out, void* stream) {
+    ao_tables_kernel<<<1, kAoThreads, 0, (cudaStream_t)stream>>>(p, out);
+    return check(cudaGetLastError());
+}
+int launch_ao_linemax_batch(const AoParams* views, const uint32_t* blk, int n_views, uint32_t n_blocks, void* stream) {
+    if (n_blocks == 0) return 0;
+    ao_linemax_batch_kernel<<<n_blocks, 256, 0, (cudaStream_t)stream>>>(views, blk, n_views);
+    return check(cudaGetLastError());
+}
 int launch_ao_T(const AoParams& p, void* stream) {
     // One pixel per thread for the largest possible list (every pixel): the
     // block scheduler balances the uneven per-pixel work; blocks past the
     // list's length exit at once.
     const size_t n = (size_t)p.W * p.H;
     if (n == 0) return 0;
-    ao_kernel<false><<<(unsigned)((n + kAoThreads - 1) / kAoThreads), kAoThreads, 0, (cudaStream_t)stream>>>(p);
+    ao_kernel<<<(unsigned)((n + kAoThreads - 1) / kAoThreads), kAoThreads, 0, (cudaStream_t)stream>>>(p);
     return check(cudaGetLastError());
 }
 int launch_ao_apply(const AoParams& p, int n_blocks, void* stream) {

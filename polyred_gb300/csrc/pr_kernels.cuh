@@ -197,6 +197,9 @@ struct AoParams {
     float ao_half_ulp;   // half an ulp of float32 at max(W, H) + 100
     float4* dgb;         // differentiation only: multiply the G-buffer's factor by the AO factor
     float* T;            // [list] the AO total of each listed pixel (ao_T_kernel -> ao_apply_kernel)
+    int exact_T;         // 1: T itself is wanted (differentiation); 0: only the colours it gives
+    const void* tables;  // the frame size's tap tables (launch_ao_tables); batches build their own
+    float* linemax;      // [4][H][W] maxima of four depths along x, rows, diagonal, antidiagonal
 };
 
 
@@ -246,11 +249,12 @@ int launch_obj_trans(const PassMats& pm, int n_pass, const float* obj_model, uin
 // NaN bookkeeping (nanseq, beaten) back to kNone / 0 after a frame that used
 // it, and, with
 // ao_list, the pixels whose winner's material has AO (tri_flags kTriAO) in
-// ao_list (count in cnt->n_ao), tile by tile (32 x 8).
+// ao_list (count in cnt->n_ao), tile by tile (32 x 8), with the depths' line maxima
+// ([4][H][W], AoParams::linemax) in linemax.
 int launch_resolve_listing(int W, int H, const unsigned long long* keys, uint32_t* nanseq, uint32_t* beaten,
                            Counters* cnt, uint32_t* win, float* depth_ao, const uint32_t* first_rec,
                            uint32_t* attr_state, uint32_t* vis, const uint8_t* tri_flags, uint32_t* ao_list,
-                           void* stream);
+                           float* linemax, void* stream);
 // The attribute records of the records resolve listed (P: the main view's setup parameters).
 int launch_attr(const SetupParams& p, const uint32_t* vis, void* stream);
 int launch_setup_shadow(const SetupParams& p, void* stream);
@@ -265,6 +269,8 @@ int launch_shade(const ShadeParams& p, void* stream);
 // the march writing p.T (after resolve), and the colour scaling and gamma
 // of the listed pixels (after both the march and shading).
 int launch_ao_T(const AoParams& p, void* stream);
+size_t ao_tables_bytes();
+int launch_ao_tables(const AoParams& p, void* out, void* stream);  // the tap tables of p's frame size (a multiple of 16 bytes)
 int launch_ao_apply(const AoParams& p, int n_blocks, void* stream);
 // passAntialiasing's imageutil.Resize of the n*W x n*H image `in` to W x H
 // (rows top-down, both buffers on the device).
@@ -293,6 +299,7 @@ int launch_raster_batch(const RasterParams* jobs, const uint32_t* items, int n_j
                         void* stream);
 int launch_resolve_batch(const ResolveParams* jobs, const uint32_t* blk, int n_jobs, uint32_t n_blocks, void* stream);
 int launch_shade_batch(const ShadeParams* views, const uint32_t* blk, int n_views, uint32_t n_blocks, void* stream);
+int launch_ao_linemax_batch(const AoParams* views, const uint32_t* blk, int n_views, uint32_t n_blocks, void* stream);
 // Persistent; chunk counters [n_views] zeroed by the caller.
 int launch_ao_batch(const AoParams* views, int n_views, uint32_t* chunk_ctr, int n_blocks, void* stream);
 int launch_col_to_float(const uchar4* col, float4* out, size_t n, void* stream);
