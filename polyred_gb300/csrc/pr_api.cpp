@@ -452,6 +452,16 @@ int viewport_std(const float* m) {
     return (m[10] == 1.0f && m[15] == 1.0f) ? 1 : 0;
 }
 
+// The zeros world_of relies on: ViewportMatrix's inverse, and the inverse of
+// a perspective matrix (entries 0, 5, 11, 14 and 15 alone).
+int inverses_std(const float* vp_inv, const float* proj_inv) {
+    for (int e : {1, 2, 4, 6, 8, 9, 11, 12, 13, 14})
+        if (vp_inv[e] != 0.0f) return 0;
+    for (int e : {1, 2, 3, 4, 6, 7, 8, 9, 10, 12, 13})
+        if (proj_inv[e] != 0.0f) return 0;
+    return 1;
+}
+
 void fill_scene_ptrs(Ctx* c, prk::SetupParams& p) {
     p.pos = c->sb.pos.p;
     p.nor = c->sb.nor.p;
@@ -768,6 +778,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         std::memcpy(mp.viewport_inv, vp_inv.m, 64);
         std::memcpy(mp.proj_inv, proj_inv.m, 64);
         std::memcpy(mp.view_inv, view_inv.m, 64);
+        mp.inv_std = inverses_std(mp.viewport_inv, mp.proj_inv);
         mp.rrec = c->rrec.p;
         mp.arec = c->arec.p;
         mp.cap_rec = c->cap_rec;
@@ -1748,6 +1759,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
         std::memcpy(mp.viewport_inv, m.vp_inv.m, 64);
         std::memcpy(mp.proj_inv, m.proj_inv.m, 64);
         std::memcpy(mp.view_inv, m.view_inv.m, 64);
+        mp.inv_std = inverses_std(mp.viewport_inv, mp.proj_inv);
         mp.rrec = b->rrec.p + rec_m[v];
         mp.arec = b->arec.p + rec_m[v];
         mp.cap_rec = b->cap_main_rec[v];

@@ -317,10 +317,41 @@ PR_DEV int sutherland_hodgman_group(V4* v, int n, float w, float h, uint32_t sub
 // instruction cache (no_instruction stalls dominated), one shared copy
 // does not.
 __device__ __noinline__ V4 apply4_outline(V4 v, const float* m) { return apply4(v, m); }
+// Vec4.Apply's x, y and z (w = 0).
+PR_DEV V4 apply3_try(V4 v, const float* m, bool& bad) {
+    return {fma64f_try(m[0], v.x, fma64f_try(m[1], v.y, fma64f_try(m[2], v.z, __fmul_rn(m[3], v.w), bad), bad), bad),
+            fma64f_try(m[4], v.x, fma64f_try(m[5], v.y, fma64f_try(m[6], v.z, __fmul_rn(m[7], v.w), bad), bad), bad),
+            fma64f_try(m[8], v.x, fma64f_try(m[9], v.y, fma64f_try(m[10], v.z, __fmul_rn(m[11], v.w), bad), bad), bad), 0.0f};
+}
+__device__ __noinline__ V4 apply3_outline(V4 v, const float* m) {
+    bool bad = false;
+    const V4 r = apply3_try(v, m, bad);
+    return __builtin_expect(bad, 0) ? apply4_exact(v, m) : r;
+}
 
-// A screen-space vertex back in world space (render/raster.go:467-469).
+// A screen-space vertex back in world space (render/raster.go:467-469), x, y
+// and z: pos through ViewportInv, ProjInv and ViewInv. With P.inv_std the
+// first two have the zero pattern of ViewportMatrix's and of a perspective
+// matrix's inverse; a zero first factor or a +-0 addend rounds alike in
+// float64 and float32 (fma64f_try), so 12 of the chain's 48 FMAs need the
+// float64 emulation. The matrices' own zeros stay in every term.
+__device__ __noinline__ V4 world_of_exact(const SetupParams& P, V4 pos) {
+    return apply4(apply4(apply4(pos, P.viewport_inv), P.proj_inv), P.view_inv);
+}
 PR_DEV V4 world_of(const SetupParams& P, V4 pos) {
-    return apply4_outline(apply4_outline(apply4_outline(pos, P.viewport_inv), P.proj_inv), P.view_inv);
+    if (!P.inv_std) return world_of_exact(P, pos);  // uniform
+    bool bad = false;
+    const float *a = P.viewport_inv, *b = P.proj_inv, *c = P.view_inv;
+    const V4 v = {fma64f_try(a[0], pos.x, __fmaf_rn(a[1], pos.y, __fmaf_rn(a[2], pos.z, __fmul_rn(a[3], pos.w))), bad),
+                  __fmaf_rn(a[4], pos.x, fma64f_try(a[5], pos.y, __fmaf_rn(a[6], pos.z, __fmul_rn(a[7], pos.w)), bad)),
+                  __fmaf_rn(a[8], pos.x, __fmaf_rn(a[9], pos.y, __fmaf_rn(a[10], pos.z, __fmul_rn(a[11], pos.w)))),
+                  __fmaf_rn(a[12], pos.x, __fmaf_rn(a[13], pos.y, __fmaf_rn(a[14], pos.z, __fmul_rn(a[15], pos.w))))};
+    const V4 q = {__fmaf_rn(b[0], v.x, __fmaf_rn(b[1], v.y, __fmaf_rn(b[2], v.z, __fmul_rn(b[3], v.w)))),
+                  __fmaf_rn(b[4], v.x, __fmaf_rn(b[5], v.y, __fmaf_rn(b[6], v.z, __fmul_rn(b[7], v.w)))),
+                  __fmaf_rn(b[8], v.x, __fmaf_rn(b[9], v.y, __fmaf_rn(b[10], v.z, __fmul_rn(b[11], v.w)))),
+                  __fmaf_rn(b[12], v.x, __fmaf_rn(b[13], v.y, fma64f_try(b[14], v.z, __fmul_rn(b[15], v.w), bad)))};
+    const V4 m = apply3_try(q, c, bad);
+    return __builtin_expect(bad, 0) ? world_of_exact(P, pos) : m;
 }
 
 // The attribute record of record ridx (drawClipped's per-vertex inputs).
@@ -564,7 +595,7 @@ PR_DEV void vertex_attrs(const SetupParams& P, uint32_t t, uint32_t o, SubVtx* v
     const float* nm = P.obj_normal + o * 16;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        v[k].nor = apply4_outline(ld4(P.nor[t * 3 + k]), nm);
+        v[k].nor = apply3_outline(ld4(P.nor[t * 3 + k]), nm);
         const float2 uv = P.uv[t * 3 + k];
         v[k].u = uv.x;
         v[k].v = uv.y;
@@ -707,7 +738,7 @@ PR_DEV void clip_one_group(const SetupParams& P, const uint32_t* clip_list, uint
         const V4 cp = mulv(trans, ld4(P.pos[t * 3 + k]));
         const float rw = P.perspective ? __fdiv_rn(-1.0f, cp.w) : 1.0f;
         const V4 sp = pos4(viewport_apply(P, cp));
-        const V4 nn = apply4_outline(ld4(P.nor[t * 3 + k]), P.obj_normal + o * 16);
+        const V4 nn = apply3_outline(ld4(P.nor[t * 3 + k]), P.obj_normal + o * 16);
         if (sub < 3u) {
             G.pos[k] = sp;
             G.nor[k] = nn;
@@ -1250,9 +1281,9 @@ __global__ void __launch_bounds__(128) attr_kernel(const __grid_constant__ Setup
             o = P.blk_obj[t >> 7];
             while (o + 1 < P.n_objects && P.obj_first[o + 1] <= t) o++;
             const V4 pos = {R[3 * k], R[3 * k + 1], R[3 * k + 2], 1.0f};
-            const V4 nor = apply4_outline(ld4(P.nor[t * 3 + k]), P.obj_normal + o * 16);
+            const V4 nor = apply3_outline(ld4(P.nor[t * 3 + k]), P.obj_normal + o * 16);
             const float2 uv = P.uv[t * 3 + k];
-            m = apply4_outline(apply4_outline(apply4_outline(pos, P.viewport_inv), P.proj_inv), P.view_inv);  // render/raster.go:467-469
+            m = world_of(P, pos);  // render/raster.go:467-469
             float* A = s_rec[warp][r];
             A[k] = R[13 + k];  // recipw
             A[3 + 3 * k] = nor.x;

@@ -98,6 +98,7 @@ struct SetupParams {
     float viewport[16];
     int vp_std;                  // 1: viewport has ViewportMatrix's zero/one pattern (apply_viewport)
     float viewport_inv[16], proj_inv[16], view_inv[16];
+    int inv_std;                 // 1: viewport_inv and proj_inv have the zero pattern world_of relies on
     RasterRec* rrec;
     AttrRec* arec;
     uint32_t cap_rec;
