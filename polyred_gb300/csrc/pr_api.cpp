@@ -186,7 +186,7 @@ struct Ctx {
     DevBuf<prk::AttrRec> arec;
     DevBuf<uint2> tasks;
     DevBuf<uint32_t> first_rec, clip_list;
-    DevBuf<uint32_t> attr_state, vis_list;  // deferred attribute records: per-record state, visible list
+    DevBuf<uint8_t> attr_state;  // deferred attribute records: per-record state
     uint32_t cap_rec = 0, cap_tasks = 0;
     // framebuffer
     int W = 0, H = 0;
@@ -429,7 +429,6 @@ int ensure_work(Ctx* c, uint32_t need_rec, uint32_t need_tasks) {
         if ((rc = c->rrec.ensure(cap))) return rc;
         if ((rc = c->arec.ensure(cap))) return rc;
         if ((rc = c->attr_state.ensure(cap))) return rc;
-        if ((rc = c->vis_list.ensure(cap))) return rc;
         if ((rc = c->rrec_s.ensure(cap))) return rc;
         c->cap_rec = cap;
     }
@@ -842,9 +841,8 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         const bool with_ao = out && out->rgba && c->sb.has_ao;
         c->ao_marched = with_ao;
         if (with_ao && ((rc = c->ao_T.ensure(npx)) || (rc = c->linemax.ensure(4 * npx)))) return rc;
-        KTRY(prk::launch_resolve_listing(W, H, c->keys.p, c->nanseq.p, c->beaten.p, dcnt, c->win.p, c->depth_ao.p,
-                                         c->first_rec.p, c->attr_state.p, c->vis_list.p, c->sb.tri_flags.p,
-                                         with_ao ? c->ao_list.p : nullptr, c->linemax.p, st));
+        KTRY(prk::launch_resolve(W, H, c->keys.p, c->nanseq.p, c->beaten.p, dcnt, c->win.p, c->depth_ao.p, c->first_rec.p,
+                                 c->attr_state.p, c->sb.tri_flags.p, with_ao ? c->ao_list.p : nullptr, c->linemax.p, st));
         prk::AoParams ap{};
         if (with_ao) {
             CUDA_TRY(cudaEventRecord(c->ev_resolved, st));
@@ -874,7 +872,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             CUDA_TRY(cudaEventRecord(c->ev_ao, sc));
             launches += 1;
         }
-        KTRY(prk::launch_attr(mp, c->vis_list.p, st));
+        KTRY(prk::launch_attr(mp, st));
         CUDA_TRY(cudaEventRecord(c->ev[3], st));
         launches += 7;
 
@@ -885,7 +883,6 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         fill_shade_frame(c, f, s2w, SW, SH, sp);
         sp.win = c->win.p;
         sp.depth_ao = c->depth_ao.p;
-        sp.first_rec = c->first_rec.p;
         sp.rrec = c->rrec.p;
         sp.arec = c->arec.p;
         sp.smaps = shadows ? c->smap.p : nullptr;
@@ -1098,7 +1095,7 @@ int pr_destroy(void* ctx) {
     if (c->ev_d2h) cudaEventDestroy(c->ev_d2h);
     if (c->stream_u) cudaStreamDestroy(c->stream_u);
     if (c->stream_d) cudaStreamDestroy(c->stream_d);
-    c->rrec.release(); c->arec.release(); c->tasks.release(); c->first_rec.release(); c->attr_state.release(); c->vis_list.release();
+    c->rrec.release(); c->arec.release(); c->tasks.release(); c->first_rec.release(); c->attr_state.release();
     c->clip_list.release();
     c->keys.release(); c->nanseq.release(); c->beaten.release(); c->win.release(); c->depth_ao.release();
     c->ao_list.release();
@@ -1792,6 +1789,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
         R.nanseq = rp.nanseq;
         R.beaten = rp.beaten;
         R.cnt = mp.cnt;
+        R.first_rec = mp.first_rec;
         R.win = b->win.p + o;
         R.depth_ao = b->depth_ao.p + o;
         prk::ShadeParams& sp = p.sh[v];
@@ -1800,7 +1798,6 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
         fill_shade_frame(c, f, m.s2w, SW, SH, sp);
         sp.win = R.win;
         sp.depth_ao = R.depth_ao;
-        sp.first_rec = mp.first_rec;
         sp.rrec = mp.rrec;
         sp.arec = mp.arec;
         sp.smaps = (f->flags & PR_FRAME_SHADOWMAP) ? b->smaps.p + sm[v] : nullptr;

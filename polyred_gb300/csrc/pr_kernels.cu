@@ -357,13 +357,11 @@ PR_DEV V4 world_of(const SetupParams& P, V4 pos) {
 // The attribute record of record ridx (drawClipped's per-vertex inputs).
 // mw: the vertices' world positions when the caller has them (the chain
 // below of each vertex's screen position), else null.
-PR_DEV void write_attr(const SetupParams& P, uint32_t ridx, const SubVtx* v, const float* recipw, int matid,
-                       const V4* mw) {
+PR_DEV void write_attr(const SetupParams& P, uint32_t ridx, const SubVtx* v, int matid, const V4* mw) {
     AttrRec A;
     V4 m[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        A.recipw[k] = recipw[k];
         A.nor[k * 3 + 0] = v[k].nor.x;
         A.nor[k * 3 + 1] = v[k].nor.y;
         A.nor[k * 3 + 2] = v[k].nor.z;
@@ -382,7 +380,7 @@ PR_DEV void write_attr(const SetupParams& P, uint32_t ridx, const SubVtx* v, con
     const float4* as = reinterpret_cast<const float4*>(&A);
     float4* ad = reinterpret_cast<float4*>(P.arec + ridx);
 #pragma unroll
-    for (int k = 0; k < 9; k++) ad[k] = as[k];
+    for (int k = 0; k < 8; k++) ad[k] = as[k];
 }
 
 // Build and store the records of one sub-triangle; returns its pixel area
@@ -405,13 +403,16 @@ PR_DEV uint32_t write_sub(const SetupParams& P, uint32_t ridx, uint32_t seq, con
     uint32_t area = 0;
     // no pixel to test: no task will name the record, no pixel can pick it
     // as its winner, so nothing reads it
-    if (!pixel_box(v[0].pos, v[1].pos, v[2].pos, R.sabc, P.W, P.H, &R.bx, &R.by, &area)) return 0;
+    if (!pixel_box(v[0].pos, v[1].pos, v[2].pos, R.sabc, P.W, P.H, &R.bx, &R.by, &area)) {
+        if (P.attr_state) P.attr_state[ridx] = kAttrDone;
+        return 0;
+    }
     const float4* rs = reinterpret_cast<const float4*>(&R);
     float4* rd = reinterpret_cast<float4*>(P.rrec + ridx);
 #pragma unroll
     for (int k = 0; k < 4; k++) rd[k] = rs[k];
-    if (P.attr_state) P.attr_state[ridx] = P.defer_attr ? 1u : 0u;
-    if (P.arec && !P.defer_attr) write_attr(P, ridx, v, recipw, matid, mw);
+    if (P.attr_state) P.attr_state[ridx] = P.defer_attr ? kAttrDeferred : kAttrDone;
+    if (P.arec && !P.defer_attr) write_attr(P, ridx, v, matid, mw);
     return area;
 }
 
@@ -1142,11 +1143,12 @@ __global__ void __launch_bounds__(kRasterWarps * 32, 6) raster_kernel(const __gr
         raster_warp(P, P.tasks, base, n_tasks, s_w[warp], n_tasks >= nw * 32u);
 }
 
-PR_DEV void resolve_one(int W, int H, const unsigned long long* keys, const uint32_t* nanseq, const uint32_t* beaten,
-                        const Counters* cnt, uint32_t* win, float* depth_ao, size_t i) {
-    if (i >= (size_t)W * H) return;
+// The winner of pixel i: its depth, its record (kNone: none) and its seq.
+PR_DEV uint32_t resolve_one(const unsigned long long* keys, const uint32_t* nanseq, const uint32_t* beaten,
+                            const Counters* cnt, const uint32_t* first_rec, uint32_t* win, float* depth_ao, size_t i,
+                            uint32_t* ridx) {
     unsigned long long key = keys[i];
-    uint32_t w = kNone;
+    uint32_t w = kNone, rec = kNone;
     float d = -1.0f;
     if (cnt->nan_flag && nanseq[i] != kNone && beaten[i] == 0u) {
         w = nanseq[i];
@@ -1155,8 +1157,11 @@ PR_DEV void resolve_one(int W, int H, const unsigned long long* keys, const uint
         w = 0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFull);
         d = fkey_decode((uint32_t)(key >> 32));
     }
-    win[i] = w;
+    if (w != kNone) rec = first_rec[w >> 3] + (w & 7u);
+    win[i] = rec;
     depth_ao[i] = d;
+    *ridx = rec;
+    return w;
 }
 
 // The line maxima of a frame's depths, which AO's march skips taps by: plane
@@ -1192,135 +1197,145 @@ PR_DEV void ao_linemax_tile(int W, int H, int x0, int r0, float* linemax, F dept
     for (int q = 0; q < 4; q++) linemax[q * plane + i] = m[q];
 }
 
-// Resolve (resolve_one) that also lists the winners' deferred attribute
-// records (the first pixel to find its record pending, 1 -> 2, appends it)
-// and, with ao_list, the frame's AO pixels: every covered pixel whose winning
+// Resolve (resolve_one) that also marks the winners' deferred attribute
+// records for attr_kernel (every pixel of a record stores the same byte) and,
+// with ao_list, lists the frame's AO pixels: every covered pixel whose winning
 // triangle's material has AO (tri_flags kTriAO; AmbientOcclusionShade's own
 // condition, material/ao.go:22), appended tile by tile (32 x 8 blocks, warps
 // in order) for the march's locality, and writes the line maxima of the
 // frame's depths (a halo of kLineReach keys more per tile). One atomic per
-// block and list.
-__global__ void __launch_bounds__(256) resolve_listing_kernel(int W, int H, const unsigned long long* keys,
-                                                              uint32_t* nanseq, uint32_t* beaten,
-                                                              Counters* cnt, uint32_t* win, float* depth_ao,
-                                                              const uint32_t* first_rec, uint32_t* attr_state,
-                                                              uint32_t* vis, const uint8_t* tri_flags,
-                                                              uint32_t* ao_list, float* linemax) {
+// block. Bound by the latency of its chain of gathers (key, first_rec, state).
+__global__ void __launch_bounds__(256) resolve_kernel(int W, int H, const unsigned long long* keys, uint32_t* nanseq,
+                                                      uint32_t* beaten, Counters* cnt, uint32_t* win, float* depth_ao,
+                                                      const uint32_t* first_rec, uint8_t* attr_state,
+                                                      const uint8_t* tri_flags, uint32_t* ao_list, float* linemax) {
     const int x = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
     const int lane = threadIdx.x, warp = threadIdx.y;
-    bool want = false, ao = false;
-    uint32_t ridx = 0;
+    bool ao = false;
     const size_t i = (size_t)r * W + x;
     if (x < W && r < H) {
-        resolve_one(W, H, keys, nanseq, beaten, cnt, win, depth_ao, i);
+        uint32_t ridx;
+        const uint32_t w = resolve_one(keys, nanseq, beaten, cnt, first_rec, win, depth_ao, i, &ridx);
         // the NaN bookkeeping back to its rest state (resolve reads it last)
         if (cnt->nan_flag && nanseq[i] != kNone) {
             nanseq[i] = kNone;
             beaten[i] = 0u;
         }
-        const uint32_t w = win[i];
         if (w != kNone) {
-            ridx = first_rec[w >> 3] + (w & 7u);
-            // most pixels find their record listed already: a plain read first
-            want = attr_state[ridx] == 1u && atomicCAS(&attr_state[ridx], 1u, 2u) == 1u;
+            // most pixels find their record marked already: a plain read first
+            if (attr_state[ridx] == kAttrDeferred) attr_state[ridx] = kAttrWanted;
             ao = ao_list && (tri_flags[w >> 3] & kTriAO) != 0;
         }
     }
-    __shared__ uint32_t s_cnt[2][8];
-    __shared__ uint32_t s_base[2];
-    const unsigned m = __ballot_sync(0xffffffffu, want), ma = __ballot_sync(0xffffffffu, ao);
-    if (lane == 0) {
-        s_cnt[0][warp] = (uint32_t)__popc(m);
-        s_cnt[1][warp] = (uint32_t)__popc(ma);
-    }
+    if (!ao_list) return;  // uniform
+    __shared__ uint32_t s_cnt[8];
+    __shared__ uint32_t s_base;
+    const unsigned ma = __ballot_sync(0xffffffffu, ao);
+    if (lane == 0) s_cnt[warp] = (uint32_t)__popc(ma);
     __syncthreads();
-    if (warp == 0 && lane < 2) {
+    if (warp == 0 && lane == 0) {
         uint32_t tot = 0;
-        for (int q = 0; q < 8; q++) tot += s_cnt[lane][q];
-        s_base[lane] = tot ? atomicAdd(lane ? &cnt->n_ao : &cnt->n_vis, tot) : 0u;
+        for (int q = 0; q < 8; q++) tot += s_cnt[q];
+        s_base = tot ? atomicAdd(&cnt->n_ao, tot) : 0u;
     }
     __syncthreads();
-    const uint32_t below = (1u << lane) - 1u;
-    if (want) {
-        uint32_t o = s_base[0] + (uint32_t)__popc(m & below);
-        for (int q = 0; q < warp; q++) o += s_cnt[0][q];
-        vis[o] = ridx;
-    }
     if (ao) {
-        uint32_t o = s_base[1] + (uint32_t)__popc(ma & below);
-        for (int q = 0; q < warp; q++) o += s_cnt[1][q];
+        uint32_t o = s_base + (uint32_t)__popc(ma & ((1u << lane) - 1u));
+        for (int q = 0; q < warp; q++) o += s_cnt[q];
         ao_list[o] = (uint32_t)i;
     }
-    if (ao_list && !cnt->nan_flag)  // uniform; a frame with NaN depths marches without them
+    if (!cnt->nan_flag)  // uniform; a frame with NaN depths marches without them
         ao_linemax_tile(W, H, blockIdx.x * 32, blockIdx.y * 8, linemax, [&](int cx, int cr) {
             const unsigned long long key = keys[(size_t)cr * W + cx];
             return key != 0ull ? fkey_decode((uint32_t)(key >> 32)) : -1.0f;
         });
 }
 
-// The deferred attribute records of the listed records: everything comes
-// back from the raster record (screen positions, -1/W, the triangle in seq)
+// The deferred attribute records of the records resolve marked: everything
+// comes back from the raster record (screen positions, the triangle in seq)
 // and the scene, by the same functions the setup uses, so the bits are
-// those an eager setup writes. Three lanes per record, one per vertex (ten
-// records per warp), and the face normal from the three world positions
-// gathered by shuffles.
-__global__ void __launch_bounds__(128) attr_kernel(const __grid_constant__ SetupParams P, const uint32_t* vis) {
-    __shared__ __align__(16) float s_rec[4][10][36];  // each warp's ten records, stored whole
-    const uint32_t n = P.cnt->n_vis;
+// those an eager setup writes. A warp takes a run of consecutive records,
+// packs the marked ones and writes them ten at a time, three lanes per record
+// (one per vertex), the face normal from the three world positions gathered
+// by shuffles. Record order follows triangle order, so the reads of the scene
+// share sectors; taken in the order pixels found them (a list), the
+// 10M-triangle soup's 3.6M records read 2.2 GB in 579 us, so 1.0 GB.
+// Long lists go in runs of 128 records, shorter ones (under two such runs a
+// warp) in 32, each taken from a queue (a static stride left the 1M-triangle
+// field's clusters to a few warps: 44 us), and those under 32 records a warp
+// in tens, one batch each, by warp index.
+constexpr int kAttrRun = 128;
+__global__ void __launch_bounds__(128) attr_kernel(const __grid_constant__ SetupParams P) {
+    __shared__ __align__(16) float s_rec[4][10][36];  // each warp's ten records (36: their words in different banks)
+    __shared__ uint32_t s_idx[4][kAttrRun];
+    const uint32_t n = min(P.cnt->n_rec, P.cap_rec);  // setup and clip wrote the state of each
     const int lane = threadIdx.x & 31, r = lane / 3, k = lane - 3 * r, warp = threadIdx.x >> 5;
     const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t base = wid * 10u; base < n; base += nw * 10u) {
-        const uint32_t j = base + (uint32_t)r;
-        const bool act = lane < 30 && j < n;
-        V4 m = {0.0f, 0.0f, 0.0f, 0.0f};
-        uint32_t ridx = 0, t = 0, o = 0;
-        if (act) {
-            ridx = vis[j];
-            const float* R = reinterpret_cast<const float*>(P.rrec + ridx);
-            t = __float_as_uint(R[12]) >> 3;
-            o = P.blk_obj[t >> 7];
-            while (o + 1 < P.n_objects && P.obj_first[o + 1] <= t) o++;
-            const V4 pos = {R[3 * k], R[3 * k + 1], R[3 * k + 2], 1.0f};
-            const V4 nor = apply3_outline(ld4(P.nor[t * 3 + k]), P.obj_normal + o * 16);
-            const float2 uv = P.uv[t * 3 + k];
-            m = world_of(P, pos);  // render/raster.go:467-469
-            float* A = s_rec[warp][r];
-            A[k] = R[13 + k];  // recipw
-            A[3 + 3 * k] = nor.x;
-            A[4 + 3 * k] = nor.y;
-            A[5 + 3 * k] = nor.z;
-            A[12 + 2 * k] = uv.x;
-            A[13 + 2 * k] = uv.y;
-            A[18 + k] = __uint_as_float(pack_col(P.col[t * 3 + k]));
-            A[21 + 3 * k] = m.x;
-            A[22 + 3 * k] = m.y;
-            A[23 + 3 * k] = m.z;
+    const uint32_t run = n >= nw * 2u * kAttrRun ? kAttrRun : n >= nw * 32u ? 32u : 10u;
+    for (uint32_t first = wid * run;; first += nw * run) {
+        if (run != 10u) {  // marked records come in clusters: runs from a queue
+            if (lane == 0) first = atomicAdd(&P.cnt->take_attr, run);
+            first = __shfl_sync(0xffffffffu, first, 0);
         }
-        const float m1x = __shfl_down_sync(0xffffffffu, m.x, 1), m1y = __shfl_down_sync(0xffffffffu, m.y, 1),
-                    m1z = __shfl_down_sync(0xffffffffu, m.z, 1);
-        const float m2x = __shfl_down_sync(0xffffffffu, m.x, 2), m2y = __shfl_down_sync(0xffffffffu, m.y, 2),
-                    m2z = __shfl_down_sync(0xffffffffu, m.z, 2);
-        if (act && k == 0) {
-            const V4 m1 = {m1x, m1y, m1z, 0.0f}, m2 = {m2x, m2y, m2z, 0.0f};
-            const V4 fn = unit4(cross4(sub4(m1, m), sub4(m2, m)));  // render/raster.go:479
-            float* A = s_rec[warp][r];
-            A[30] = fn.x;
-            A[31] = fn.y;
-            A[32] = fn.z;
-            A[33] = fn.w;
-            int matid = P.mat[t];
-            if (matid >= 0) matid += P.obj_matbase[o];
-            A[34] = __int_as_float(matid);
-            A[35] = 0.0f;
+        if (first >= n) break;
+        uint32_t m_n = 0;  // marked records of the run
+        for (uint32_t c = 0; c < run; c += 32u) {
+            const uint32_t q = first + c + (uint32_t)lane;
+            const bool want = c + (uint32_t)lane < run && q < n && P.attr_state[q] == kAttrWanted;
+            const unsigned b = __ballot_sync(0xffffffffu, want);
+            if (want) s_idx[warp][m_n + __popc(b & ((1u << lane) - 1u))] = q;
+            m_n += __popc(b);
         }
         __syncwarp();
-        // the warp's records out as whole 16-byte words: 9 per record
-        const uint32_t nr = min(10u, n - base);
-        for (uint32_t e = (uint32_t)lane; e < nr * 9u; e += 32u) {
-            const uint32_t rr = e / 9u, w4 = e - rr * 9u;
-            reinterpret_cast<float4*>(P.arec + vis[base + rr])[w4] = reinterpret_cast<const float4*>(s_rec[warp][rr])[w4];
+        for (uint32_t at = 0; at < m_n; at += 10u) {
+            const uint32_t j = at + (uint32_t)r;
+            const bool act = lane < 30 && j < m_n;
+            V4 m = {0.0f, 0.0f, 0.0f, 0.0f};
+            uint32_t t = 0, o = 0;
+            if (act) {
+                const float* R = reinterpret_cast<const float*>(P.rrec + s_idx[warp][j]);
+                t = __float_as_uint(R[12]) >> 3;
+                o = P.blk_obj[t >> 7];
+                while (o + 1 < P.n_objects && P.obj_first[o + 1] <= t) o++;
+                const V4 pos = {R[3 * k], R[3 * k + 1], R[3 * k + 2], 1.0f};
+                const V4 nor = apply3_outline(ld4(P.nor[t * 3 + k]), P.obj_normal + o * 16);
+                const float2 uv = P.uv[t * 3 + k];
+                m = world_of(P, pos);  // render/raster.go:467-469
+                float* A = s_rec[warp][r];
+                A[3 * k] = nor.x;
+                A[1 + 3 * k] = nor.y;
+                A[2 + 3 * k] = nor.z;
+                A[9 + 2 * k] = uv.x;
+                A[10 + 2 * k] = uv.y;
+                A[15 + k] = __uint_as_float(pack_col(P.col[t * 3 + k]));
+                A[18 + 3 * k] = m.x;
+                A[19 + 3 * k] = m.y;
+                A[20 + 3 * k] = m.z;
+            }
+            const float m1x = __shfl_down_sync(0xffffffffu, m.x, 1), m1y = __shfl_down_sync(0xffffffffu, m.y, 1),
+                        m1z = __shfl_down_sync(0xffffffffu, m.z, 1);
+            const float m2x = __shfl_down_sync(0xffffffffu, m.x, 2), m2y = __shfl_down_sync(0xffffffffu, m.y, 2),
+                        m2z = __shfl_down_sync(0xffffffffu, m.z, 2);
+            if (act && k == 0) {
+                const V4 m1 = {m1x, m1y, m1z, 0.0f}, m2 = {m2x, m2y, m2z, 0.0f};
+                const V4 fn = unit4(cross4(sub4(m1, m), sub4(m2, m)));  // render/raster.go:479
+                float* A = s_rec[warp][r];
+                A[27] = fn.x;
+                A[28] = fn.y;
+                A[29] = fn.z;
+                A[30] = fn.w;
+                int matid = P.mat[t];
+                if (matid >= 0) matid += P.obj_matbase[o];
+                A[31] = __int_as_float(matid);
+            }
+            __syncwarp();
+            // the warp's records out as whole 16-byte words: 8 per record
+            const uint32_t nr = min(10u, m_n - at);
+            for (uint32_t e = (uint32_t)lane; e < nr * 8u; e += 32u)
+                reinterpret_cast<float4*>(P.arec + s_idx[warp][at + (e >> 3)])[e & 7u] =
+                    reinterpret_cast<const float4*>(s_rec[warp][e >> 3])[e & 7u];
+            __syncwarp();
         }
-        __syncwarp();
     }
 }
 
@@ -1491,10 +1506,10 @@ PR_DEV bool shade_one(const ShadeParams& P, int x, int r) {
     const int W = P.W, H = P.H;
     const int y = H - 1 - r;
     const size_t i = (size_t)r * W + x;
-    const uint32_t seq = P.win[i];
+    const uint32_t ridx = P.win[i];
     uint32_t c0, c1, c2, c3;
     bool ao_pending = false;
-    if (seq == kNone) {
+    if (ridx == kNone) {
         c0 = P.background[0]; c1 = P.background[1]; c2 = P.background[2]; c3 = P.background[3];
         if (P.tri_id) P.tri_id[i] = kNone;
         if (P.depth) P.depth[i] = 0.0f;
@@ -1512,9 +1527,9 @@ PR_DEV bool shade_one(const ShadeParams& P, int x, int r) {
             D[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     } else {
-        const uint32_t ridx = P.first_rec[seq >> 3] + (seq & 7u);
         const float4* rp = reinterpret_cast<const float4*>(P.rrec + ridx);
-        float4 q0 = rp[0], q1 = rp[1], q2 = rp[2];
+        const float4 q0 = rp[0], q1 = rp[1], q2 = rp[2], q3 = rp[3];
+        const uint32_t seq = __float_as_uint(q3.x);
         const float X0 = q0.x, Y0 = q0.y, Z0 = q0.z, X1 = q0.w, Y1 = q1.x, Z1 = q1.y, X2 = q1.z, Y2 = q1.w, Z2 = q2.x;
         const float sabc = q2.y;
         const AttrRec& A = P.arec[ridx];
@@ -1522,7 +1537,7 @@ PR_DEV bool shade_one(const ShadeParams& P, int x, int r) {
         float bc[3];
         barycoord_s(fx, fy, X0, Y0, X1, Y1, X2, Y2, sabc, bc);
         const float z = __fadd_rn(__fadd_rn(__fmul_rn(bc[0], Z0), __fmul_rn(bc[1], Z1)), __fmul_rn(bc[2], Z2));
-        const float rw0 = A.recipw[0], rw1 = A.recipw[1], rw2 = A.recipw[2];
+        const float rw0 = q3.y, rw1 = q3.z, rw2 = q3.w;
         const float wc1 = __fmul_rn(rw0, bc[0]), wc2 = __fmul_rn(rw1, bc[1]), wc3 = __fmul_rn(rw2, bc[2]);
         const bool persp = (P.flags & PR_FRAME_PERSPECTIVE) != 0;
         const float norm = persp ? __fdiv_rn(1.0f, __fadd_rn(__fadd_rn(wc1, wc2), wc3)) : 1.0f;
@@ -2393,8 +2408,10 @@ __global__ void __launch_bounds__(kRasterWarps * 32, 6) raster_batch_kernel(cons
 __global__ void resolve_batch_kernel(const ResolveParams* jobs, const uint32_t* blk, int n_jobs) {
     const int j = job_of(blk, n_jobs, blockIdx.x);
     const ResolveParams& R = jobs[j];
-    resolve_one(R.W, R.H, R.keys, R.nanseq, R.beaten, R.cnt, R.win, R.depth_ao,
-                (size_t)(blockIdx.x - blk[j]) * blockDim.x + threadIdx.x);
+    const size_t i = (size_t)(blockIdx.x - blk[j]) * blockDim.x + threadIdx.x;
+    uint32_t ridx;
+    if (i < (size_t)R.W * R.H)
+        resolve_one(R.keys, R.nanseq, R.beaten, R.cnt, R.first_rec, R.win, R.depth_ao, i, &ridx);
 }
 
 // 256-thread blocks as 32 x 8 pixel tiles, row-major over each view's tiles.
@@ -2487,18 +2504,17 @@ int launch_setup_main_only(const SetupParams& p, uint32_t* clip_list, void* stre
     setup_main_kernel<<<(p.n_tris + 127) / 128, 128, 0, (cudaStream_t)stream>>>(p, clip_list);
     return check(cudaGetLastError());
 }
-int launch_resolve_listing(int W, int H, const unsigned long long* keys, uint32_t* nanseq, uint32_t* beaten,
-                           Counters* cnt, uint32_t* win, float* depth_ao, const uint32_t* first_rec,
-                           uint32_t* attr_state, uint32_t* vis, const uint8_t* tri_flags, uint32_t* ao_list,
-                           float* linemax, void* stream) {
+int launch_resolve(int W, int H, const unsigned long long* keys, uint32_t* nanseq, uint32_t* beaten, Counters* cnt,
+                   uint32_t* win, float* depth_ao, const uint32_t* first_rec, uint8_t* attr_state,
+                   const uint8_t* tri_flags, uint32_t* ao_list, float* linemax, void* stream) {
     if (W <= 0 || H <= 0) return 0;
     const dim3 blk(32, 8), grd((unsigned)((W + 31) / 32), (unsigned)((H + 7) / 8));
-    resolve_listing_kernel<<<grd, blk, 0, (cudaStream_t)stream>>>(W, H, keys, nanseq, beaten, cnt, win, depth_ao,
-                                                                 first_rec, attr_state, vis, tri_flags, ao_list, linemax);
+    resolve_kernel<<<grd, blk, 0, (cudaStream_t)stream>>>(W, H, keys, nanseq, beaten, cnt, win, depth_ao, first_rec,
+                                                         attr_state, tri_flags, ao_list, linemax);
     return check(cudaGetLastError());
 }
-int launch_attr(const SetupParams& p, const uint32_t* vis, void* stream) {
-    attr_kernel<<<(unsigned)sm_count() * 8u, 128, 0, (cudaStream_t)stream>>>(p, vis);
+int launch_attr(const SetupParams& p, void* stream) {
+    attr_kernel<<<(unsigned)sm_count() * 8u, 128, 0, (cudaStream_t)stream>>>(p);
     return check(cudaGetLastError());
 }
 int launch_obj_trans(const PassMats& pm, int n_pass, const float* obj_model, uint32_t n_objects, float* out,

@@ -38,10 +38,10 @@ struct alignas(16) RasterRec {
 };
 static_assert(sizeof(RasterRec) == 64, "RasterRec is four float4");
 
-// Attribute record: the rest of drawClipped's inputs for one sub-triangle.
-// 36 words = 144 bytes.
-struct alignas(16) AttrRec {
-    float recipw[3];  // parent triangle's -1/W (render/raster.go:403-406, 440-443)
+// Attribute record: the rest of drawClipped's inputs for one sub-triangle
+// (the parent's -1/W is in its raster record). 32 words = 128 bytes, aligned
+// so that a record is four whole 32-byte sectors.
+struct alignas(128) AttrRec {
     float nor[9];     // vertex normals after Apply(Normal) (xyz per vertex)
     float uv[6];
     uint32_t col[3];  // RGBA8 per vertex
@@ -49,7 +49,9 @@ struct alignas(16) AttrRec {
     float fn[4];      // face normal fN (render/raster.go:479)
     int32_t matid;    // flat material id (<0 = vertex colour)
 };
-static_assert(sizeof(AttrRec) == 144, "AttrRec is nine float4");
+static_assert(sizeof(AttrRec) == 128, "AttrRec is eight float4");
+// State of a record's attributes (SetupParams::attr_state)
+constexpr uint8_t kAttrDone = 0, kAttrDeferred = 1, kAttrWanted = 2;  // written (or none); left out; to be written
 
 struct Counters {
     uint32_t n_rec;       // records emitted (main view)
@@ -62,7 +64,7 @@ struct Counters {
     uint32_t need_tasks;  // tasks needed when overflow
     uint32_t n_ao;        // pixels listed for ambient occlusion
     uint32_t take[2];     // raster work-queue heads: the pass, its NaN fix-up pass
-    uint32_t n_vis;       // records listed for their attributes (resolve)
+    uint32_t take_attr;   // work-queue head of the attribute records
     uint32_t pad[4];
 };
 
@@ -85,7 +87,7 @@ struct SetupParams {
     const uint32_t* obj_first;   // [n_objects + 1]
     const float* obj_model;      // [n_objects][16]
     const float* obj_trans;      // [n_objects][16] this pass's Proj·View·Model, or null: per-block cache
-    uint32_t* attr_state;        // per record: 1 = attributes deferred, 0 = written here; null: no bookkeeping
+    uint8_t* attr_state;         // per record: kAttr*; null: no bookkeeping
     int defer_attr;              // 1: leave the attribute record to attr_kernel (visible records only)
     const uint32_t* blk_obj;     // [n_tris / 128] object of each 128-triangle block's first triangle
     const float* obj_normal;     // [n_objects][16] Model.Inv().T()
@@ -143,9 +145,8 @@ struct RasterParams {
 struct ShadeParams {
     int W, H;
     uint32_t flags;             // PR_FRAME_*
-    const uint32_t* win;        // winning seq per pixel
+    const uint32_t* win;        // winning record per pixel (kNone: not covered)
     const float* depth_ao;      // depth where covered, -1 elsewhere (material/ao.go:57-62)
-    const uint32_t* first_rec;
     const RasterRec* rrec;
     const AttrRec* arec;
     const pr_material* mats;
@@ -245,19 +246,17 @@ struct PassMats {
 };
 int launch_obj_trans(const PassMats& pm, int n_pass, const float* obj_model, uint32_t n_objects, float* out,
                      void* stream);
-// Resolve that also lists, once each, the winning records whose attributes
-// were deferred (attr_state 1 -> 2) in vis (count in cnt->n_vis), puts the
-// NaN bookkeeping (nanseq, beaten) back to kNone / 0 after a frame that used
-// it, and, with
-// ao_list, the pixels whose winner's material has AO (tri_flags kTriAO) in
-// ao_list (count in cnt->n_ao), tile by tile (32 x 8), with the depths' line maxima
-// ([4][H][W], AoParams::linemax) in linemax.
-int launch_resolve_listing(int W, int H, const unsigned long long* keys, uint32_t* nanseq, uint32_t* beaten,
-                           Counters* cnt, uint32_t* win, float* depth_ao, const uint32_t* first_rec,
-                           uint32_t* attr_state, uint32_t* vis, const uint8_t* tri_flags, uint32_t* ao_list,
-                           float* linemax, void* stream);
-// The attribute records of the records resolve listed (P: the main view's setup parameters).
-int launch_attr(const SetupParams& p, const uint32_t* vis, void* stream);
+// Resolve that also marks the winning records whose attributes were deferred
+// (attr_state kAttrDeferred -> kAttrWanted), puts the NaN bookkeeping
+// (nanseq, beaten) back to kNone / 0 after a frame that used it, and, with
+// ao_list, lists the pixels whose winner's material has AO (tri_flags kTriAO)
+// in ao_list (count in cnt->n_ao), tile by tile (32 x 8), with the depths'
+// line maxima ([4][H][W], AoParams::linemax) in linemax.
+int launch_resolve(int W, int H, const unsigned long long* keys, uint32_t* nanseq, uint32_t* beaten, Counters* cnt,
+                   uint32_t* win, float* depth_ao, const uint32_t* first_rec, uint8_t* attr_state,
+                   const uint8_t* tri_flags, uint32_t* ao_list, float* linemax, void* stream);
+// The attribute records of the records resolve marked (P: the main view's setup parameters).
+int launch_attr(const SetupParams& p, void* stream);
 int launch_setup_shadow(const SetupParams& p, void* stream);
 int launch_raster(const RasterParams& p, int n_blocks, void* stream);
 int launch_shadow_fixup_reset(int W, int H, const uint32_t* lastnan, uint32_t* smap, const Counters* cnt,
@@ -285,6 +284,7 @@ struct ResolveParams {
     const uint32_t* nanseq;
     const uint32_t* beaten;
     const Counters* cnt;
+    const uint32_t* first_rec;
     uint32_t* win;
     float* depth_ao;
 };
