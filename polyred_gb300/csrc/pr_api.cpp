@@ -1606,6 +1606,7 @@ struct BatchPlan {
     std::vector<prk::AoParams> ao;
     std::vector<uint32_t> blk;             // blk_s[S+1] blk_m[V+1] blk_r[V+1] blk_sh[V+1]
     uint32_t nb_s = 0, nb_m = 0, nb_r = 0, nb_sh = 0;
+    bool fast = true;                      // every view's shading is shade_is_fast
     std::vector<int> shadow_view;          // view of each shadow pass
     size_t n_rec = 0, n_rec_main = 0, n_tasks = 0, n_px = 0, n_smap = 0, n_first = 0;
     std::string key;
@@ -1813,6 +1814,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
         sp.guvd = (float4*)out->uvd;
         sp.gvcol = (uchar4*)out->vcol;
         sp.gmat = out->mat_id;
+        p.fast &= prk::shade_is_fast(sp);
         prk::AoParams& ap = p.ao[v];
         ap.W = f->width;
         ap.H = f->height;
@@ -1845,8 +1847,8 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
     (void)osh;
     // the graph's shape: everything a captured launch depends on
     char kb[128];
-    snprintf(kb, sizeof(kb), "%u/%u/%u/%u/%u/%u/%d/%zu/%zu|", nv, p.S, p.nb_s, p.nb_m, p.nb_r, p.nb_sh, b->raster_bps,
-             p.n_px, p.n_smap);
+    snprintf(kb, sizeof(kb), "%u/%u/%u/%u/%u/%u/%d/%zu/%zu/%d|", nv, p.S, p.nb_s, p.nb_m, p.nb_r, p.nb_sh, b->raster_bps,
+             p.n_px, p.n_smap, (int)p.fast);
     p.key = kb;
     // every pointer the captured launches take as an argument
     const void* args[] = {b->cnt.p, b->keys.p, b->nanseq.p, b->beaten.p, b->chunk.p, b->smaps.p, b->h_cnt,
@@ -1895,7 +1897,7 @@ int batch_launch(Batch* b, const BatchPlan& p, uint32_t* launches) {
     KTRY(prk::launch_batch_scan(b->d_fj.p, (int)V, b->d_fitems.p, b->d_queue.p + 1, 1, st));
     KTRY(prk::launch_raster_batch(b->d_fj.p, b->d_fitems.p, (int)V, b->d_queue.p + 1, b->n_sms * b->raster_bps, st));
     KTRY(prk::launch_resolve_batch(b->d_res.p, blk_r, (int)V, p.nb_r, st));
-    KTRY(prk::launch_shade_batch(b->d_sh.p, blk_sh, (int)V, p.nb_sh, st));
+    KTRY(prk::launch_shade_batch(b->d_sh.p, blk_sh, (int)V, p.nb_sh, p.fast, st));
     KTRY(prk::launch_ao_linemax_batch(b->d_ao.p, blk_sh, (int)V, p.nb_sh, st));
     KTRY(prk::launch_ao_batch(b->d_ao.p, (int)V, b->chunk.p, b->n_sms * 4, st));
     n += 11;

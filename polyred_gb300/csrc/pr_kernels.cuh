@@ -265,6 +265,7 @@ int launch_shadow_fixup_reset(int W, int H, const uint32_t* lastnan, uint32_t* s
 int launch_nan_cleanup(size_t n, uint32_t* a, uint32_t va, uint32_t* b, uint32_t vb, const Counters* cnt,
                        void* stream);
 int launch_shade(const ShadeParams& p, void* stream);
+bool shade_is_fast(const ShadeParams& p);  // colours and depths alone: certified lighting
 // AO split so that its march overlaps shading: the list (made by resolve),
 // the march writing p.T (after resolve), and the colour scaling and gamma
 // of the listed pixels (after both the march and shading).
@@ -299,7 +300,8 @@ int launch_batch_scan(const RasterParams* jobs, int n_jobs, uint32_t* items, uin
 int launch_raster_batch(const RasterParams* jobs, const uint32_t* items, int n_jobs, uint32_t* queue, int n_blocks,
                         void* stream);
 int launch_resolve_batch(const ResolveParams* jobs, const uint32_t* blk, int n_jobs, uint32_t n_blocks, void* stream);
-int launch_shade_batch(const ShadeParams* views, const uint32_t* blk, int n_views, uint32_t n_blocks, void* stream);
+// fast: every view is shade_is_fast
+int launch_shade_batch(const ShadeParams* views, const uint32_t* blk, int n_views, uint32_t n_blocks, bool fast, void* stream);
 int launch_ao_linemax_batch(const AoParams* views, const uint32_t* blk, int n_views, uint32_t n_blocks, void* stream);
 // Persistent; chunk counters [n_views] zeroed by the caller.
 int launch_ao_batch(const AoParams* views, int n_views, uint32_t* chunk_ctr, int n_blocks, void* stream);
