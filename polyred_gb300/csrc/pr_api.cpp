@@ -435,9 +435,10 @@ int ensure_work(Ctx* c, uint32_t need_rec, uint32_t need_tasks) {
     if (need_tasks > c->cap_tasks) {
         uint32_t cap = std::max(need_tasks, c->cap_tasks * 2);
         c->cap_tasks = 0;
-        if ((rc = c->tasks.ensure(cap))) return rc;
-        if ((rc = c->tasks_s.ensure(cap))) return rc;
-        if ((rc = c->tasks_c.ensure(cap))) return rc;
+        const size_t room = (size_t)cap + prk::big_room(cap);
+        if ((rc = c->tasks.ensure(room))) return rc;
+        if ((rc = c->tasks_s.ensure(room))) return rc;
+        if ((rc = c->tasks_c.ensure(room))) return rc;
         c->cap_tasks = cap;
     }
     return PR_OK;
@@ -510,7 +511,7 @@ void collect_stats(Ctx* c) {
     c->stats.n_clipped_tris = c->h_cnt[0].n_clipped;
     c->stats.n_nan_fragments = c->h_cnt[0].n_nan;
     uint32_t n_tasks = 0;
-    for (int k = 0; k < prk::kNumCounters; k++) n_tasks += c->h_cnt[k].n_tasks;
+    for (int k = 0; k < prk::kNumCounters; k++) n_tasks += c->h_cnt[k].n_tasks + c->h_cnt[k].n_big_px;
     c->stats.n_raster_tasks = n_tasks;
     // 0 for an interval whose events a failed frame did not record; the
     // error that reports it must not be left for the next launch check
@@ -733,6 +734,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
                 sp.cap_rec = c->cap_rec;
                 sp.tasks = c->tasks_s.p;
                 sp.cap_tasks = c->cap_tasks;
+                sp.cap_big = prk::big_room(c->cap_tasks);
                 sp.first_rec = nullptr;
                 sp.cnt = dcnt + 1 + l;
                 sp.obj_trans = c->obj_trans.p + (size_t)(1 + l) * n_obj * 16;
@@ -742,6 +744,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
                 prk::RasterParams rp{};
                 rp.rrec = c->rrec_s.p;
                 rp.tasks = c->tasks_s.p;
+                rp.big = rp.tasks + c->cap_tasks;
                 rp.cnt = dcnt + 1 + l;
                 rp.cnt_w = dcnt + 1 + l;
                 rp.W = SW;
@@ -783,6 +786,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         mp.cap_rec = c->cap_rec;
         mp.tasks = c->tasks.p;
         mp.cap_tasks = c->cap_tasks;
+        mp.cap_big = prk::big_room(c->cap_tasks);
         mp.first_rec = c->first_rec.p;
         mp.cnt = dcnt;
         if (dh) {
@@ -807,6 +811,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         prk::RasterParams rp{};
         rp.rrec = c->rrec.p;
         rp.tasks = c->tasks.p;
+        rp.big = rp.tasks + c->cap_tasks;
         rp.cnt = dcnt;
         rp.cnt_w = dcnt;
         rp.W = W;
@@ -818,6 +823,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         rp.take = &dcnt[0].take[0];
         prk::RasterParams rc_ = rp;
         rc_.tasks = c->tasks_c.p;
+        rc_.big = rc_.tasks + c->cap_tasks;
         rc_.cnt = dclip;
         rc_.take = &dclip->take[0];
         rc_.grab = 32;  // a short list (the frame's clipped triangles): spread it over warps
@@ -830,6 +836,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         rp.mode = prk::kMainFixup;
         rp.take = &dcnt[0].take[1];
         rp.tasks2 = c->tasks_c.p;
+        rp.big2 = rc_.big;
         rp.cnt2 = dclip;
         rp.take2 = &dclip->take[1];
         KTRY(prk::launch_raster(rp, c->n_sms * 8, st));
@@ -1634,7 +1641,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
         rec_m[v] = rec;
         rec += cr;
         task_m[v] = task;
-        task += ct;
+        task += (size_t)ct + prk::big_room(ct);
         b->cap_main_rec[v] = cr;
         b->cap_main_tasks[v] = ct;
         px[v] = npx;
@@ -1659,7 +1666,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
             if (!f->lights[l].cast_shadow) continue;
             sps.push_back({v, l, rec, task});
             rec += std::max<uint32_t>(n, 1);
-            task += ct;
+            task += (size_t)ct + prk::big_room(ct);
         }
     }
     p.S = (uint32_t)sps.size();
@@ -1715,6 +1722,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
         sp.cap_rec = std::max<uint32_t>(c->sb.n_tris, 1);
         sp.tasks = b->tasks.p + q.task;
         sp.cap_tasks = b->cap_shadow_tasks[q.v];
+        sp.cap_big = prk::big_room(sp.cap_tasks);
         sp.first_rec = nullptr;
         sp.cnt = dcnt + nv + s;
         sp.task_shift = b->task_shift;
@@ -1722,6 +1730,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
         prk::RasterParams& rp = p.rj[nv + s];
         rp.rrec = sp.rrec;
         rp.tasks = sp.tasks;
+        rp.big = sp.tasks + sp.cap_tasks;
         rp.cnt = sp.cnt;
         rp.cnt_w = sp.cnt;
         rp.W = SW;
@@ -1763,6 +1772,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
         mp.cap_rec = b->cap_main_rec[v];
         mp.tasks = b->tasks.p + task_m[v];
         mp.cap_tasks = b->cap_main_tasks[v];
+        mp.cap_big = prk::big_room(mp.cap_tasks);
         mp.first_rec = b->first_rec.p + first[v];
         mp.clip_list = b->clip_list.p + first[v];
         mp.cnt = dcnt + v;
@@ -1772,6 +1782,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
         prk::RasterParams& rp = p.rj[v];
         rp.rrec = mp.rrec;
         rp.tasks = mp.tasks;
+        rp.big = mp.tasks + mp.cap_tasks;
         rp.cnt = mp.cnt;
         rp.cnt_w = mp.cnt;
         rp.W = f->width;
@@ -2152,7 +2163,7 @@ int pr_batch_tune(void* batch, uint32_t n_views, const pr_batch_view* views, cha
         const prk::Counters& k = b->h_cnt[v];
         const uint32_t n = b->scenes[views[v].scene]->sb.n_tris;
         b->cap_main_rec[v] = std::max(k.n_rec + k.n_rec / 16 + 64, std::min(b->cap_main_rec[v], n + n / 8 + 1024));
-        b->cap_main_tasks[v] = k.n_tasks + k.n_tasks / 16 + 64;
+        b->cap_main_tasks[v] = std::max(k.n_tasks + k.n_tasks / 16, 4u * (k.n_big + k.n_big / 16)) + 64;
         rec += b->cap_main_rec[v];
         tasks += b->cap_main_tasks[v];
     }

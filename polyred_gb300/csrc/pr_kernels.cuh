@@ -53,6 +53,9 @@ static_assert(sizeof(AttrRec) == 128, "AttrRec is eight float4");
 // State of a record's attributes (SetupParams::attr_state)
 constexpr uint8_t kAttrDone = 0, kAttrDeferred = 1, kAttrWanted = 2;  // written (or none); left out; to be written
 
+// Block tasks per task capacity: a task buffer of cap tasks holds cap + big_room(cap) entries.
+inline uint32_t big_room(uint32_t cap) { return cap / 4 + 64; }
+
 struct Counters {
     uint32_t n_rec;       // records emitted (main view)
     uint32_t n_tasks;     // raster tasks emitted
@@ -65,7 +68,9 @@ struct Counters {
     uint32_t n_ao;        // pixels listed for ambient occlusion
     uint32_t take[2];     // raster work-queue heads: the pass, its NaN fix-up pass
     uint32_t take_attr;   // work-queue head of the attribute records
-    uint32_t pad[4];
+    uint32_t n_big;       // block tasks of large records (raster_block)
+    uint32_t n_big_px;    // ... counted as tasks of 2^task_shift pixels
+    uint32_t pad[2];
 };
 
 struct LightK {
@@ -104,8 +109,9 @@ struct SetupParams {
     RasterRec* rrec;
     AttrRec* arec;
     uint32_t cap_rec;
-    uint2* tasks;
+    uint2* tasks;                // (record, chunk); block tasks of large records follow at tasks + cap_tasks
     uint32_t cap_tasks;
+    uint32_t cap_big;            // room for block tasks (big_room of the task capacity), 0: none are made
     uint32_t* first_rec;
     Counters* cnt;
     float* tri_scr;              // differentiation only: [n_tris][12] screen x, y, recipw per vertex
@@ -130,13 +136,14 @@ struct RasterParams {
     uint32_t* smap;            // shadow: orderable depth keys, index x + y*W
     uint32_t* lastnan;         // shadow: 1 + max seq of NaN-depth fragments, 0 if none
     uint32_t task_shift = kTaskShift;  // as the setup that wrote the tasks
-    uint32_t* take = nullptr;          // zeroed work-queue head (warps take grab tasks at a time), or
-                                       // null: a static stride over the tasks
+    uint32_t* take = nullptr;          // zeroed work-queue head (warps take grab tasks at a time; unused by batches)
     uint32_t grab = 0;                 // tasks per queue grab, a multiple of 32; 0: from the task count
                                        // (64 below 256 tasks per warp of the grid, else 128)
     // a second task list drained after the first (its own counters and
     // queue head, the same records): the NaN fix-up of the main and the
     // clipped lists in one launch
+    const uint2* big = nullptr;        // block tasks (cnt->n_big of them), or null
+    const uint2* big2 = nullptr;       // the second list's
     const uint2* tasks2 = nullptr;
     const Counters* cnt2 = nullptr;
     uint32_t* take2 = nullptr;
