@@ -1506,6 +1506,8 @@ int pr_diff_backward(void* ctx, const pr_frame_desc* frame, const pr_diff_params
     K.grad = (const float4*)grad_radiance;
     K.g_vcol = (float4*)grads->vertex_color;
     K.g_vnor = (float4*)grads->vertex_normal;
+    K.vec_vcol = ((uintptr_t)grads->vertex_color & 15u) == 0;
+    K.vec_vnor = ((uintptr_t)grads->vertex_normal & 15u) == 0;
     K.g_acc = c->d_acc.p;
     KTRY(prk::launch_diff(K, true, st));
     std::vector<double> acc(std::max<size_t>(n_acc, 1));

@@ -236,6 +236,7 @@ struct DiffParamsK {
     const float4* grad;          // backward input
     float4* g_vcol;              // backward outputs (may be null)
     float4* g_vnor;
+    int vec_vcol, vec_vnor;      // 1: g_vcol / g_vnor is 16-byte aligned
     double* g_acc;               // [n_mats*7 + n_lights*4 + n_ambient]: kd3 ks3 shin | pos3 I | ambient
 };
 
