@@ -3039,24 +3039,57 @@ constexpr size_t kNaRecords = kNaObjModel + kNoAllocMaxObjects * 64; // RasterRe
 constexpr size_t kNaTasks = kNaRecords + (size_t)kNoAllocMaxTris * sizeof(RasterRec);
 constexpr size_t kNaKeys = kNaTasks + (size_t)kNoAllocMaxTasks * sizeof(uint2);
 constexpr size_t kNaLastNan = kNaKeys + (size_t)kNoAllocMaxTexels * 4;
-constexpr size_t kNaBytes = kNaLastNan + (size_t)kNoAllocMaxTexels * 4;
+constexpr size_t kNaObjTrans = kNaLastNan + (size_t)kNoAllocMaxTexels * 4;  // f32 [kNaParamObjects][16]
+constexpr uint32_t kNaParamObjects = 32;                                   // objects passed as kernel parameters
+constexpr size_t kNaBlkObj = kNaObjTrans + kNaParamObjects * 64;           // u32 [max_tris / 128]
+constexpr size_t kNaBytes = kNaBlkObj + kNoAllocMaxTris / 128 * 4;
 static_assert(kNaBytes <= (16u << 20), "scratch layout exceeds 16 MiB");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[16u << 20];
 
-__global__ void encode_map_kernel(const float* depth, uint32_t* keys, size_t n) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float d = depth[i];
-    keys[i] = isnan(d) ? 0u : fkey(d);  // key 0 stands for NaN (below every value)
+// The objects of a call with few of them, and Proj·View, by value.
+struct NaObjects {
+    uint32_t n;  // 0: the tables come by copies
+    uint32_t first[kNaParamObjects + 1];
+    float model[kNaParamObjects][16];
+    float pv[16];
+};
+
+// Everything a call needs before its setup, in one launch: the keys of the
+// caller's map, the NaN bookkeeping and counters at rest, and (O.n) the object
+// tables: first triangles, Proj·View·Model (as obj_trans_kernel) and the object
+// of each 128-triangle block.
+__global__ void __launch_bounds__(256) noalloc_init_kernel(const float* depth, uint32_t* keys, uint32_t* lastnan, size_t n,
+                                                           Counters* cnt, uint32_t* obj_first, float* obj_trans,
+                                                           uint32_t* blk_obj, uint32_t n_tris,
+                                                           const __grid_constant__ NaObjects O) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        const float d = depth[i];
+        keys[i] = isnan(d) ? 0u : fkey(d);  // key 0 stands for NaN (below every value)
+        lastnan[i] = 0u;
+    }
+    if (blockIdx.x != 0) return;
+    for (uint32_t e = threadIdx.x; e < sizeof(Counters) / 4; e += blockDim.x) reinterpret_cast<uint32_t*>(cnt)[e] = 0u;
+    if (O.n == 0) return;
+    for (uint32_t e = threadIdx.x; e <= O.n; e += blockDim.x) obj_first[e] = O.first[e];
+    for (uint32_t e = threadIdx.x; e < O.n * 16u; e += blockDim.x) {
+        const uint32_t r = (e >> 2) & 3u, c = e & 3u;
+        const float* m = O.pv + r * 4;
+        const float* q = O.model[e >> 4];
+        obj_trans[e] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[0], q[c]), __fmul_rn(m[1], q[4 + c])), __fmul_rn(m[2], q[8 + c])),
+                                 __fmul_rn(m[3], q[12 + c]));
+    }
+    for (uint32_t e = threadIdx.x; e * 128u < n_tris; e += blockDim.x) blk_obj[e] = find_object(O.first, O.n, e * 128u);
 }
 
 // Back into the caller's map: a texel whose key the raster changed takes the
 // decoded key; the others keep their bits, so a -0 or a NaN payload that no
 // fragment replaced stays as it was, as in the reference's map.
-__global__ void decode_changed_kernel(const uint32_t* keys, float* depth, size_t n) {
+// After a task overflow the map stays as it was.
+__global__ void decode_changed_kernel(const uint32_t* keys, float* depth, size_t n, const Counters* cnt) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n || cnt->overflow) return;
     const float d = depth[i];
     const uint32_t k0 = isnan(d) ? 0u : fkey(d), k = keys[i];
     if (k != k0) depth[i] = fkey_decode(k);
@@ -3119,23 +3152,40 @@ extern "C" int pr_depth_map_noalloc(const pr_depth_map_desc* d) {
     uint32_t* lastnan = (uint32_t*)(base + kNaLastNan);
     const size_t n = (size_t)d->width * d->height;
 
-    // object tables (host -> the scratch array)
+    prh::M4 pv = prh::mulm(prh::M4{{d->proj[0], d->proj[1], d->proj[2], d->proj[3], d->proj[4], d->proj[5], d->proj[6],
+                                     d->proj[7], d->proj[8], d->proj[9], d->proj[10], d->proj[11], d->proj[12],
+                                     d->proj[13], d->proj[14], d->proj[15]}},
+                           prh::M4{{d->view[0], d->view[1], d->view[2], d->view[3], d->view[4], d->view[5], d->view[6],
+                                     d->view[7], d->view[8], d->view[9], d->view[10], d->view[11], d->view[12],
+                                     d->view[13], d->view[14], d->view[15]}});
+    // object tables: a few as kernel parameters, more by copies (host -> the scratch array)
+    const bool by_param = d->n_objects > 0 && d->n_objects <= kNaParamObjects;
+    NaObjects O;
+    O.n = by_param ? d->n_objects : 0u;
+    cudaError_t e = cudaSuccess;
     uint32_t first[kNoAllocMaxObjects + 1];
     float model[kNoAllocMaxObjects * 16];
-    for (uint32_t o = 0; o < d->n_objects; o++) {
-        first[o] = d->objects[o].first_tri;
-        std::memcpy(model + o * 16, d->objects[o].model, 64);
-    }
-    first[d->n_objects] = d->n_tris;
-    cudaError_t e = cudaSuccess;
-    if (d->n_objects > 0) {
+    if (by_param) {
+        for (uint32_t o = 0; o < d->n_objects; o++) {
+            O.first[o] = d->objects[o].first_tri;
+            std::memcpy(O.model[o], d->objects[o].model, 64);
+        }
+        O.first[d->n_objects] = d->n_tris;
+        std::memcpy(O.pv, pv.m, 64);
+    } else if (d->n_objects > 0) {
+        for (uint32_t o = 0; o < d->n_objects; o++) {
+            first[o] = d->objects[o].first_tri;
+            std::memcpy(model + o * 16, d->objects[o].model, 64);
+        }
+        first[d->n_objects] = d->n_tris;
         e = cudaMemcpyAsync(obj_first, first, (d->n_objects + 1) * 4, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(obj_model, model, d->n_objects * 64, cudaMemcpyHostToDevice, st);
     }
-    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(Counters), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(lastnan, 0, n * 4, st);
     if (e != cudaSuccess) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: scratch initialisation failed");
-    encode_map_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d->depth, keys, n);
+    float* obj_trans = (float*)(base + kNaObjTrans);
+    uint32_t* blk_obj = (uint32_t*)(base + kNaBlkObj);
+    noalloc_init_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d->depth, keys, lastnan, n, cnt, obj_first, obj_trans,
+                                                                  blk_obj, d->n_tris, O);
 
     SetupParams sp{};
     sp.pos = (const float4*)d->pos;
@@ -3146,15 +3196,14 @@ extern "C" int pr_depth_map_noalloc(const pr_depth_map_desc* d) {
     sp.W = d->width;
     sp.H = d->height;
     sp.perspective = 0;
-    prh::M4 pv = prh::mulm(prh::M4{{d->proj[0], d->proj[1], d->proj[2], d->proj[3], d->proj[4], d->proj[5], d->proj[6],
-                                     d->proj[7], d->proj[8], d->proj[9], d->proj[10], d->proj[11], d->proj[12],
-                                     d->proj[13], d->proj[14], d->proj[15]}},
-                           prh::M4{{d->view[0], d->view[1], d->view[2], d->view[3], d->view[4], d->view[5], d->view[6],
-                                     d->view[7], d->view[8], d->view[9], d->view[10], d->view[11], d->view[12],
-                                     d->view[13], d->view[14], d->view[15]}});
+    if (by_param) {
+        sp.obj_trans = obj_trans;
+        sp.blk_obj = blk_obj;
+    }
     prh::M4 vp = prh::viewport((float)d->width, (float)d->height);
     std::memcpy(sp.pv, pv.m, 64);
     std::memcpy(sp.viewport, vp.m, 64);
+    sp.vp_std = 1;  // prh::viewport's pattern
     sp.rrec = rrec;
     sp.cap_rec = kNoAllocMaxTris;
     sp.tasks = tasks;
@@ -3180,6 +3229,9 @@ extern "C" int pr_depth_map_noalloc(const pr_depth_map_desc* d) {
     rp.take = &cnt->take[1];
     if (!rc) rc = launch_raster(rp, sm_count() * 8, st);
     if (rc) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: kernel launch failed");
+    decode_changed_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(keys, d->depth, n, cnt);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: kernel launch failed");
     Counters h{};
     e = cudaMemcpyAsync(&h, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -3187,9 +3239,5 @@ extern "C" int pr_depth_map_noalloc(const pr_depth_map_desc* d) {
     if (h.overflow)
         return err(PR_ERR_OVERFLOW, "pr_depth_map_noalloc: more raster tasks than PR_NOALLOC_MAX_TASKS (262144); "
                                     "the depth map was left unchanged");
-    decode_changed_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(keys, d->depth, n);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: decode failed");
     return PR_OK;
 }
