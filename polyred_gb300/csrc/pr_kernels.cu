@@ -28,6 +28,13 @@ namespace {
 
 constexpr float kEps = 1e-7f;  // math.Epsilon as float32 (math/math.go:31)
 
+// The approximate units, for values whose error a bound covers (PTX ISA: rcp
+// 1 ulp; rsqrt 2^-22.4, ex2 2^-22 relative; lg2 2^-22 absolute on (1/2, 2), else relative).
+PR_DEV float approx_lg2(float x) { float r; asm("lg2.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+PR_DEV float approx_ex2(float x) { float r; asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+PR_DEV float approx_rsq(float x) { float r; asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+PR_DEV float approx_rcp(float x) { float r; asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+
 PR_DEV V4 ld4(const float4 q) { return {q.x, q.y, q.z, q.w}; }
 
 // Mat4.MulM (math/mat4.go:201-220), plain float32 sums left to right.
@@ -139,8 +146,12 @@ PR_DEV void tighten_box(V4 a, V4 b, V4 c, float sabc, long long& x0, long long& 
 }
 
 // The reference's pixel box (rounded bounding box padded by one, clamped
-// to the target), narrowed by tighten_box; false: no pixel to test.
-PR_DEV bool pixel_box(V4 a, V4 b, V4 c, float sabc, int W, int H, uint32_t* bx, uint32_t* by, uint32_t* area) {
+// to the target), narrowed by tighten_box: its words and its area, 0 with no
+// pixel to test. Any coordinates, NaN and infinities included.
+struct PixBox {
+    uint32_t area, bx, by;
+};
+static __device__ __noinline__ PixBox pixel_box_any(V4 a, V4 b, V4 c, float sabc, int W, int H) {
     Box r = box3(a, b, c);
     long long xmin = go_f2i(__fsub_rn(pround(r.mnx), 1.0f));
     long long xmax = go_f2i(__fadd_rn(pround(r.mxx), 1.0f));
@@ -148,13 +159,79 @@ PR_DEV bool pixel_box(V4 a, V4 b, V4 c, float sabc, int W, int H, uint32_t* bx, 
     long long ymax = go_f2i(__fadd_rn(pround(r.mxy), 1.0f));
     long long x0 = xmin < 0 ? 0 : xmin, x1 = xmax > W - 1 ? W - 1 : xmax;
     long long y0 = ymin < 0 ? 0 : ymin, y1 = ymax > H - 1 ? H - 1 : ymax;
-    if (x0 > x1 || y0 > y1) return false;
+    if (x0 > x1 || y0 > y1) return {0u, 0u, 0u};
     tighten_box(a, b, c, sabc, x0, x1, y0, y1);
-    if (x0 > x1 || y0 > y1) return false;
-    *bx = (uint32_t)x0 | ((uint32_t)x1 << 16);
-    *by = (uint32_t)y0 | ((uint32_t)y1 << 16);
-    *area = (uint32_t)((x1 - x0 + 1) * (y1 - y0 + 1));
-    return true;
+    if (x0 > x1 || y0 > y1) return {0u, 0u, 0u};
+    return {(uint32_t)((x1 - x0 + 1) * (y1 - y0 + 1)), (uint32_t)x0 | ((uint32_t)x1 << 16), (uint32_t)y0 | ((uint32_t)y1 << 16)};
+}
+
+// The box of three finite screen vertices, where the plain minima and maxima
+// are box3's (NaN and infinities go through the general functions). The
+// setup kernels are bound by issue, and box3's special cases, the 64-bit
+// conversions of the pixel box and an IEEE quotient for its margin were a
+// third of a triangle's instructions.
+struct ScrBox {
+    float mnx, mxx, mny, mxy, mnz, mxz;
+    bool fin;
+};
+PR_DEV ScrBox scr_box(V4 a, V4 b, V4 c) {
+    const float sum = __fadd_rn(__fadd_rn(__fadd_rn(fabsf(a.x), fabsf(a.y)), __fadd_rn(fabsf(a.z), fabsf(b.x))),
+                                __fadd_rn(__fadd_rn(fabsf(b.y), fabsf(b.z)),
+                                          __fadd_rn(fabsf(c.x), __fadd_rn(fabsf(c.y), fabsf(c.z)))));
+    return {fminf(fminf(a.x, b.x), c.x), fmaxf(fmaxf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y), fmaxf(fmaxf(a.y, b.y), c.y),
+            fminf(fminf(a.z, b.z), c.z), fmaxf(fmaxf(a.z, b.z), c.z), sum < 3e38f};
+}
+static __device__ __noinline__ bool intersect_any(float ew, float eh, V4 a, V4 b, V4 c) {
+    const Box vp = {0.0f, 0.0f, -1.0f, ew, eh, 1.0f};
+    return box_intersect(vp, box3(a, b, c));
+}
+static __device__ __noinline__ bool contains_any(float ew, float eh, V4 a, V4 b, V4 c) {
+    const Box vp = {0.0f, 0.0f, -1.0f, ew, eh, 1.0f};
+    return box_contains(vp, a) && box_contains(vp, b) && box_contains(vp, c);
+}
+// box_intersect of the viewport box (0, 0, -1) .. (ew, eh, 1), the far end of z the reference's ew-by-eh Max.Y.
+PR_DEV bool scr_intersects(const ScrBox& s, float ew, float eh, V4 a, V4 b, V4 c) {
+    if (!s.fin) return intersect_any(ew, eh, a, b, c);
+    return s.mxx >= 0.0f && s.mnx <= ew && s.mxy >= 0.0f && s.mny <= eh && s.mxz >= -1.0f && s.mnz <= eh;
+}
+// box_contains of its three vertices. Above 1 and below -1 the next float is
+// already more than Epsilon away, so only the bounds at 0 keep it.
+PR_DEV bool scr_contained(const ScrBox& s, float ew, float eh, V4 a, V4 b, V4 c) {
+    if (!s.fin) return contains_any(ew, eh, a, b, c);
+    return s.mnx >= -kEps && s.mxx <= ew && s.mny >= -kEps && s.mxy <= eh && s.mnz >= -1.0f && s.mxz <= 1.0f;
+}
+
+// pixel_box_any for a finite box that reaches 0 or more, in float32 (the
+// coordinates, clamped to [0, 2^16], round exactly by additions of 2^23). A
+// reciprocal rounded up in place of tighten_box's quotient only widens its margin.
+PR_DEV PixBox pixel_box(const ScrBox& s, V4 a, V4 b, V4 c, float sabc, int W, int H) {
+    if (!(s.fin && s.mxx >= 0.0f && s.mxy >= 0.0f)) return pixel_box_any(a, b, c, sabc, W, H);
+    const float k23 = 8388608.0f;
+    auto clip = [](float v) { return fminf(fmaxf(v, 0.0f), 65536.0f); };
+    auto round_up = [&](float v) { return __fsub_rn(__fadd_rz(__fadd_rd(clip(v), 0.5f), k23), k23); };  // half away from zero
+    float x0 = fmaxf(__fsub_rn(round_up(s.mnx), 1.0f), 0.0f), x1 = fminf(__fadd_rn(round_up(s.mxx), 1.0f), (float)(W - 1));
+    float y0 = fmaxf(__fsub_rn(round_up(s.mny), 1.0f), 0.0f), y1 = fminf(__fadd_rn(round_up(s.mxy), 1.0f), (float)(H - 1));
+    // tighten_box
+    const float wx = __fsub_ru(s.mxx, s.mnx), wy = __fsub_ru(s.mxy, s.mny);
+    const float E = __fadd_ru(wx, wy), U = __fadd_ru(E, 4.0f);
+    const float k6u = 3.6e-7f;  // >= 6 * 2^-24
+    const float dS = __fmul_ru(__fmul_ru(k6u, E), U), dA = __fmul_ru(__fmul_ru(k6u, E), E);
+    const float as = fabsf(sabc), L = __fsub_rd(as, dA);
+    const float inv = __fmul_ru(approx_rcp(L), 1.0000005f);
+    const float q = __fmul_ru(__fadd_ru(dS, __fmul_ru(2.1e-7f, __fadd_ru(as, __fmul_ru(2.0f, dA)))), inv);
+    if (L > __fmul_ru(2.0f, dA) && L > 0.0f && as < 3e38f && q < 1e30f) {
+        const float mx = __fmul_ru(__fmul_ru(2.0f, wx), q), my = __fmul_ru(__fmul_ru(2.0f, wy), q);
+        auto up = [&](float v) { return __fsub_rn(__fadd_ru(clip(v), k23), k23); };                           // ceil
+        auto down = [&](float v) { return __fsub_rn(__fadd_rd(fminf(fmaxf(v, -4.0f), 65536.0f), k23), k23); };  // floor (v < 0: below 0)
+        x0 = fmaxf(x0, up(__fsub_rd(__fsub_rd(s.mnx, mx), 0.5f)));
+        x1 = fminf(x1, down(__fsub_ru(__fadd_ru(s.mxx, mx), 0.5f)));
+        y0 = fmaxf(y0, up(__fsub_rd(__fsub_rd(s.mny, my), 0.5f)));
+        y1 = fminf(y1, down(__fsub_ru(__fadd_ru(s.mxy, my), 0.5f)));
+    }
+    if (!(x0 <= x1 && y0 <= y1)) return {0u, 0u, 0u};
+    auto u16 = [&](float v) { return __float_as_uint(__fadd_rn(v, k23)) - 0x4B000000u; };
+    const uint32_t ix0 = u16(x0), ix1 = u16(x1), iy0 = u16(y0), iy1 = u16(y1);
+    return {(ix1 - ix0 + 1u) * (iy1 - iy0 + 1u), ix0 | (ix1 << 16), iy0 | (iy1 << 16)};
 }
 
 PR_DEV uint32_t find_object(const uint32_t* first, uint32_t n_obj, uint32_t t) {
@@ -346,11 +423,11 @@ PR_DEV void write_attr(const SetupParams& P, uint32_t ridx, const SubVtx* v, int
 
 // Build and store the records of one sub-triangle; returns its pixel area
 // (0 = nothing to raster, and then nothing is stored) and writes its bbox
-// words. With P.defer_attr the
+// words. sabc and box: the vertices' sabc_of and scr_box. With P.defer_attr the
 // attribute record is left to attr_kernel, which writes it only for records
 // that win a pixel.
 PR_DEV uint32_t write_sub(const SetupParams& P, uint32_t ridx, uint32_t seq, const SubVtx* v, const float* recipw,
-                          int matid, uint32_t* bx, uint32_t* by, const V4* mw = nullptr) {
+                          int matid, float sabc, const ScrBox& box, uint32_t* bx, uint32_t* by, const V4* mw = nullptr) {
     RasterRec R;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -359,24 +436,24 @@ PR_DEV uint32_t write_sub(const SetupParams& P, uint32_t ridx, uint32_t seq, con
         R.v[3 * k + 2] = v[k].pos.z;
         R.recipw[k] = recipw ? recipw[k] : 0.0f;
     }
-    R.sabc = sabc_of(R.v[0], R.v[1], R.v[3], R.v[4], R.v[6], R.v[7]);
+    R.sabc = sabc;
     R.seq = seq;
-    uint32_t area = 0;
     // no pixel to test: no task will name the record, no pixel can pick it
     // as its winner, so nothing reads it
-    if (!pixel_box(v[0].pos, v[1].pos, v[2].pos, R.sabc, P.W, P.H, &R.bx, &R.by, &area)) {
+    const PixBox pb = pixel_box(box, v[0].pos, v[1].pos, v[2].pos, sabc, P.W, P.H);
+    if (pb.area == 0) {
         if (P.attr_state) P.attr_state[ridx] = kAttrDone;
         return 0;
     }
-    *bx = R.bx;
-    *by = R.by;
+    R.bx = *bx = pb.bx;
+    R.by = *by = pb.by;
     const float4* rs = reinterpret_cast<const float4*>(&R);
     float4* rd = reinterpret_cast<float4*>(P.rrec + ridx);
 #pragma unroll
     for (int k = 0; k < 4; k++) rd[k] = rs[k];
     if (P.attr_state) P.attr_state[ridx] = P.defer_attr ? kAttrDeferred : kAttrDone;
     if (P.arec && !P.defer_attr) write_attr(P, ridx, v, matid, mw);
-    return area;
+    return pb.area;
 }
 
 // Vec4.Apply(ViewportMatrix) for a matrix of ViewportMatrix's pattern
@@ -541,10 +618,25 @@ PR_DEV bool tri_valid_of(const SetupParams& P, uint32_t t, const V4* p) {
     return tri_is_valid(p[0], p[1], p[2]);
 }
 
-// The transform and the culls of transform_main (screen positions, -1/W,
+// A vertex through trans and the viewport (render/raster.go:398-412). Its -1/W
+// and Pos()'s 1/W are one reciprocal where the viewport leaves w as it is.
+PR_DEV V4 screen_vertex(const SetupParams& P, const float* trans, V4 p, float* recipw) {
+    const V4 cp = mulv(trans, p), q = viewport_apply(P, cp);
+    float r = 1.0f;
+    *recipw = 1.0f;
+    if (P.perspective) {  // uniform
+        r = __frcp_rn(cp.w);
+        *recipw = -r;
+    }
+    if (q.w == 1.0f || q.w == 0.0f) return {q.x, q.y, q.z, 1.0f};
+    if (!P.perspective || __float_as_uint(q.w) != __float_as_uint(cp.w)) r = __frcp_rn(q.w);
+    return {__fmul_rn(q.x, r), __fmul_rn(q.y, r), __fmul_rn(q.z, r), 1.0f};
+}
+
+// The transform and the culls of draw (screen positions, -1/W, Sabc, the box,
 // the object); false when a cull drops the triangle.
 PR_DEV bool transform_main_geom(const SetupParams& P, const ObjCache* C, uint32_t t, SubVtx* v, float* recipw,
-                                uint32_t* obj, bool* contained) {
+                                uint32_t* obj, float* sabc, ScrBox* box, bool* contained) {
     V4 p[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) p[k] = ld4(P.pos[t * 3 + k]);
@@ -552,18 +644,13 @@ PR_DEV bool transform_main_geom(const SetupParams& P, const ObjCache* C, uint32_
     float trans[16];
     const uint32_t o = object_trans(P, C, t, trans);
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const V4 cp = mulv(trans, p[k]);
-        recipw[k] = P.perspective ? __fdiv_rn(-1.0f, cp.w) : 1.0f;
-        v[k].pos = pos4(viewport_apply(P, cp));
-    }
-    // cullBackFace (render/cull.go:26-28)
-    if (cross_z(__fsub_rn(v[1].pos.x, v[0].pos.x), __fsub_rn(v[1].pos.y, v[0].pos.y), __fsub_rn(v[2].pos.x, v[0].pos.x),
-                __fsub_rn(v[2].pos.y, v[0].pos.y)) < 0.0f)
-        return false;
-    const Box vp = {0.0f, 0.0f, -1.0f, ext_w(P), ext_h(P), 1.0f};
-    if (!box_intersect(vp, box3(v[0].pos, v[1].pos, v[2].pos))) return false;
-    *contained = box_contains(vp, v[0].pos) && box_contains(vp, v[1].pos) && box_contains(vp, v[2].pos);
+    for (int k = 0; k < 3; k++) v[k].pos = screen_vertex(P, trans, p[k], recipw + k);
+    // cullBackFace (render/cull.go:26-28): its cross product is Barycoord's Sabc
+    *sabc = sabc_of(v[0].pos.x, v[0].pos.y, v[1].pos.x, v[1].pos.y, v[2].pos.x, v[2].pos.y);
+    if (*sabc < 0.0f) return false;
+    *box = scr_box(v[0].pos, v[1].pos, v[2].pos);
+    if (!scr_intersects(*box, ext_w(P), ext_h(P), v[0].pos, v[1].pos, v[2].pos)) return false;
+    *contained = scr_contained(*box, ext_w(P), ext_h(P), v[0].pos, v[1].pos, v[2].pos);
     *obj = o;
     return true;
 }
@@ -593,7 +680,9 @@ PR_DEV void setup_main_one(const SetupParams& P, const ObjCache* C, uint32_t t, 
     int matid = -1;
     bool contained = false;
     uint32_t obj = 0;
-    const bool ok = t < P.n_tris && transform_main_geom(P, C, t, v, recipw, &obj, &contained);
+    float sabc = 0.0f;
+    ScrBox box = {};
+    const bool ok = t < P.n_tris && transform_main_geom(P, C, t, v, recipw, &obj, &sabc, &box, &contained);
     if (ok && !P.defer_attr) vertex_attrs(P, t, obj, v, &matid);
     if (ok && P.tri_scr) {
         float4* s = reinterpret_cast<float4*>(P.tri_scr + 12 * (size_t)t);
@@ -614,7 +703,7 @@ PR_DEV void setup_main_one(const SetupParams& P, const ObjCache* C, uint32_t t, 
             atomicMax(&P.cnt->need_rec, ridx + 1);
         } else {
             P.first_rec[t] = ridx;
-            area = write_sub(P, ridx, t * 8u, v, recipw, matid, &bx, &by);
+            area = write_sub(P, ridx, t * 8u, v, recipw, matid, sabc, box, &bx, &by);
         }
     }
     emit_tasks_warp(P, ridx, area, bx, by);
@@ -655,9 +744,8 @@ PR_DEV void clip_one_group(const SetupParams& P, const uint32_t* clip_list, uint
         const uint32_t k = min(sub, 2u);
         float trans[16];
         const uint32_t o = object_trans(P, nullptr, t, trans);
-        const V4 cp = mulv(trans, ld4(P.pos[t * 3 + k]));
-        const float rw = P.perspective ? __fdiv_rn(-1.0f, cp.w) : 1.0f;
-        const V4 sp = pos4(viewport_apply(P, cp));
+        float rw;
+        const V4 sp = screen_vertex(P, trans, ld4(P.pos[t * 3 + k]), &rw);
         const V4 nn = apply3_outline(ld4(P.nor[t * 3 + k]), P.obj_normal + o * 16);
         if (sub < 3u) {
             G.pos[k] = sp;
@@ -709,7 +797,9 @@ PR_DEV void clip_one_group(const SetupParams& P, const uint32_t* clip_list, uint
             if (sub == 0) P.first_rec[t] = ridx;
             const SubVtx s3[3] = {G.cv[0], G.cv[sub + 1], G.cv[sub + 2]};
             const V4 mw[3] = {G.mw[0], G.mw[sub + 1], G.mw[sub + 2]};
-            area = write_sub(P, ridx, t * 8u + sub, s3, recipw, matid, &bx, &by, attrs ? mw : nullptr);
+            area = write_sub(P, ridx, t * 8u + sub, s3, recipw, matid,
+                             sabc_of(s3[0].pos.x, s3[0].pos.y, s3[1].pos.x, s3[1].pos.y, s3[2].pos.x, s3[2].pos.y),
+                             scr_box(s3[0].pos, s3[1].pos, s3[2].pos), &bx, &by, attrs ? mw : nullptr);
         }
     }
     emit_tasks_warp(P, ridx, area, bx, by);
@@ -730,6 +820,8 @@ __global__ void __launch_bounds__(128) clip_kernel(const __grid_constant__ Setup
 PR_DEV void setup_shadow_one(const SetupParams& P, const ObjCache* C, uint32_t t) {
     bool ok = false;
     SubVtx v[3];
+    float sabc = 0.0f;
+    ScrBox box = {};
     if (t < P.n_tris) {
         V4 p[3];
 #pragma unroll
@@ -739,18 +831,18 @@ PR_DEV void setup_shadow_one(const SetupParams& P, const ObjCache* C, uint32_t t
             object_trans(P, C, t, trans);
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                v[k].pos = pos4(viewport_apply(P, mulv(trans, p[k])));
+                float rw;
+                v[k].pos = screen_vertex(P, trans, p[k], &rw);
                 v[k].nor = {0, 0, 0, 0};
                 v[k].u = v[k].v = 0;
                 v[k].col = 0;
             }
-            // cullBackFace (render/cull.go:26-28): culled iff cross.Z < 0
-            ok = !(cross_z(__fsub_rn(v[1].pos.x, v[0].pos.x), __fsub_rn(v[1].pos.y, v[0].pos.y),
-                           __fsub_rn(v[2].pos.x, v[0].pos.x), __fsub_rn(v[2].pos.y, v[0].pos.y)) < 0.0f);
-            // cullViewFrustum (render/cull.go:15-23): NewAABB((W,H,1),(0,0,0),(0,0,-1))
-            if (ok) {
-                const Box vp = box3(V4{ext_w(P), ext_h(P), 1.0f, 1.0f}, V4{0, 0, 0, 1}, V4{0, 0, -1.0f, 1});
-                ok = box_intersect(vp, box3(v[0].pos, v[1].pos, v[2].pos));
+            // cullBackFace (render/cull.go:26-28): culled iff cross.Z, Barycoord's Sabc, is below 0
+            sabc = sabc_of(v[0].pos.x, v[0].pos.y, v[1].pos.x, v[1].pos.y, v[2].pos.x, v[2].pos.y);
+            if (!(sabc < 0.0f)) {
+                // cullViewFrustum (render/cull.go:15-23): NewAABB((W,H,1),(0,0,0),(0,0,-1))
+                box = scr_box(v[0].pos, v[1].pos, v[2].pos);
+                ok = scr_intersects(box, ext_w(P), ext_h(P), v[0].pos, v[1].pos, v[2].pos);
             }
         }
     }
@@ -758,7 +850,7 @@ PR_DEV void setup_shadow_one(const SetupParams& P, const ObjCache* C, uint32_t t
     uint32_t area = 0, bx = 0, by = 0;
     if (ok) {
         float rw[3] = {1, 1, 1};
-        area = write_sub(P, t, t, v, rw, -1, &bx, &by);
+        area = write_sub(P, t, t, v, rw, -1, sabc, box, &bx, &by);
     }
     emit_tasks_warp(P, t, area, bx, by);
 }
@@ -1639,10 +1731,6 @@ static __device__ __noinline__ uint32_t blinn_exact_px(const ShadeParams& P, uin
     return blinn_exact(P, mat, tc, nn, frag_world(A, bc));
 }
 
-PR_DEV float approx_lg2(float x) { float r; asm("lg2.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
-PR_DEV float approx_ex2(float x) { float r; asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
-PR_DEV float approx_rsq(float x) { float r; asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
-PR_DEV float approx_rcp(float x) { float r; asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 
 // blinn_exact_px's colour from a plain float32 evaluation and a bound on its
 // distance from the reference's, when that bound decides all three bytes;
