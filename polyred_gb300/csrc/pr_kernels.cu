@@ -421,13 +421,17 @@ PR_DEV void write_attr(const SetupParams& P, uint32_t ridx, const SubVtx* v, int
     for (int k = 0; k < 8; k++) ad[k] = as[k];
 }
 
-// Build and store the records of one sub-triangle; returns its pixel area
-// (0 = nothing to raster, and then nothing is stored) and writes its bbox
-// words. sabc and box: the vertices' sabc_of and scr_box. With P.defer_attr the
-// attribute record is left to attr_kernel, which writes it only for records
-// that win a pixel.
-PR_DEV uint32_t write_sub(const SetupParams& P, uint32_t ridx, uint32_t seq, const SubVtx* v, const float* recipw,
-                          int matid, float sabc, const ScrBox& box, uint32_t* bx, uint32_t* by, const V4* mw = nullptr) {
+// Build and store the records of one sub-triangle of Sabc sabc and pixel box
+// pb. With P.defer_attr the attribute record is left to attr_kernel, which
+// writes it only for records that win a pixel.
+PR_DEV void write_sub(const SetupParams& P, uint32_t ridx, uint32_t seq, const SubVtx* v, const float* recipw, int matid,
+                      float sabc, const PixBox& pb, const V4* mw = nullptr) {
+    // no pixel to test: no task will name the record, no pixel can pick it
+    // as its winner, so nothing reads it
+    if (pb.area == 0) {
+        if (P.attr_state) P.attr_state[ridx] = kAttrDone;
+        return;
+    }
     RasterRec R;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -438,22 +442,14 @@ PR_DEV uint32_t write_sub(const SetupParams& P, uint32_t ridx, uint32_t seq, con
     }
     R.sabc = sabc;
     R.seq = seq;
-    // no pixel to test: no task will name the record, no pixel can pick it
-    // as its winner, so nothing reads it
-    const PixBox pb = pixel_box(box, v[0].pos, v[1].pos, v[2].pos, sabc, P.W, P.H);
-    if (pb.area == 0) {
-        if (P.attr_state) P.attr_state[ridx] = kAttrDone;
-        return 0;
-    }
-    R.bx = *bx = pb.bx;
-    R.by = *by = pb.by;
+    R.bx = pb.bx;
+    R.by = pb.by;
     const float4* rs = reinterpret_cast<const float4*>(&R);
     float4* rd = reinterpret_cast<float4*>(P.rrec + ridx);
 #pragma unroll
     for (int k = 0; k < 4; k++) rd[k] = rs[k];
     if (P.attr_state) P.attr_state[ridx] = P.defer_attr ? kAttrDeferred : kAttrDone;
     if (P.arec && !P.defer_attr) write_attr(P, ridx, v, matid, mw);
-    return pb.area;
 }
 
 // Vec4.Apply(ViewportMatrix) for a matrix of ViewportMatrix's pattern
@@ -498,16 +494,12 @@ PR_DEV uint32_t warp_reserve(uint32_t* counter, uint32_t n, uint32_t* total) {
 
 PR_DEV uint32_t n_tasks_of(uint32_t area, uint32_t shift) { return (area + (1u << shift) - 1u) >> shift; }
 
-// Append n (per lane) tasks (r, flag), (r, flag + 1), ... of record r to a
-// list; all lanes call. A lane with more than kWarpEmit tasks leaves their
-// writing to the whole warp, which would otherwise wait on that lane's serial
-// stores. need: the task capacity that would hold them, per task.
+// Write n (per lane) tasks (r, 0), (r, 1), ... of record r at list + o; all
+// lanes call. A lane with more than kWarpEmit tasks leaves their writing to
+// the whole warp, which would otherwise wait on that lane's serial stores.
+// need: the task capacity that would hold one of the list's tasks.
 constexpr uint32_t kWarpEmit = 8;
-PR_DEV void emit_run(const SetupParams& P, uint2* list, uint32_t cap, uint32_t* counter, uint32_t need, uint32_t r,
-                     uint32_t n, uint32_t flag) {
-    uint32_t tot;
-    uint32_t o = warp_reserve(counter, n, &tot);
-    if (tot == 0) return;  // warp-uniform
+PR_DEV void emit_run(const SetupParams& P, uint2* list, uint32_t cap, uint32_t o, uint32_t need, uint32_t r, uint32_t n) {
     const bool fits = o + n <= cap;
     if (n != 0 && !fits) {
         atomicOr(&P.cnt->overflow, 2u);
@@ -515,34 +507,70 @@ PR_DEV void emit_run(const SetupParams& P, uint2* list, uint32_t cap, uint32_t* 
     }
     const bool shared = fits && n > kWarpEmit;
     if (fits && !shared)
-        for (uint32_t c = 0; c < n; c++) list[o + c] = make_uint2(r, flag + c);
+        for (uint32_t c = 0; c < n; c++) list[o + c] = make_uint2(r, c);
     for (unsigned big = __ballot_sync(0xffffffffu, shared); big; big &= big - 1u) {
         const int l = __ffs(big) - 1;
         const uint32_t lo = __shfl_sync(0xffffffffu, o, l), ln = __shfl_sync(0xffffffffu, n, l);
         const uint32_t lr = __shfl_sync(0xffffffffu, r, l);
-        for (uint32_t c = lane_id(); c < ln; c += 32u) list[lo + c] = make_uint2(lr, flag + c);
+        for (uint32_t c = lane_id(); c < ln; c += 32u) list[lo + c] = make_uint2(lr, c);
     }
 }
 
-// Write the raster tasks of this lane's record (area 0: none); all lanes
-// call. A record whose pixel box has kBigArea pixels or more (and a pass with
+// A record whose pixel box has kBigArea pixels or more (and a pass with
 // room for them) gets one task per 32 x 32 block of its box (raster_block)
 // in place of one per 32 pixels. 20 views inside their sphere fields (bound by
 // the pixel tests' issue): raster 8.7 -> 4.2 ms, and the clip kernel no longer
 // writes a ground plane's tasks by the ten thousand (1080p: 45 -> 24 us). From
 // 1024 pixels on, a sphere of 2000-pixel boxes rastered in 18 us, from 4096 in 15.
 constexpr uint32_t kBigArea = 4096;
-PR_DEV uint32_t blocks_of(uint32_t bx, uint32_t by) {
-    return (((bx >> 16) - (bx & 0xffffu) + 32u) >> 5) * (((by >> 16) - (by & 0xffffu) + 32u) >> 5);
+PR_DEV bool is_big(const SetupParams& P, uint32_t area) { return area >= kBigArea && P.cap_big != 0u; }
+PR_DEV uint32_t small_tasks(const SetupParams& P, uint32_t area) {
+    return is_big(P, area) ? 0u : n_tasks_of(area, P.task_shift);
 }
-PR_DEV void emit_tasks_warp(const SetupParams& P, uint32_t ridx, uint32_t area, uint32_t bx, uint32_t by) {
-    const bool big = area >= kBigArea && P.cap_big != 0u;
-    const uint32_t nt = n_tasks_of(area, P.task_shift);
-    emit_run(P, P.tasks, P.cap_tasks, &P.cnt->n_tasks, 1u, ridx, big ? 0u : nt, 0u);
-    if (__any_sync(0xffffffffu, big)) {
-        emit_run(P, P.tasks + P.cap_tasks, P.cap_big, &P.cnt->n_big, 4u, ridx, big ? blocks_of(bx, by) : 0u, 0u);
-        if (big) atomicAdd(&P.cnt->n_big_px, nt);
+// The block tasks of this lane's record, if it is a large one; all lanes call.
+PR_DEV void emit_blocks(const SetupParams& P, uint32_t ridx, const PixBox& pb) {
+    const bool big = is_big(P, pb.area);
+    if (!__any_sync(0xffffffffu, big)) return;
+    const uint32_t n = big ? (((pb.bx >> 16) - (pb.bx & 0xffffu) + 32u) >> 5) * (((pb.by >> 16) - (pb.by & 0xffffu) + 32u) >> 5) : 0u;
+    uint32_t tot;
+    const uint32_t o = warp_reserve(&P.cnt->n_big, n, &tot);
+    emit_run(P, P.tasks + P.cap_tasks, P.cap_big, o, 4u, ridx, n);
+    if (big) atomicAdd(&P.cnt->n_big_px, n_tasks_of(pb.area, P.task_shift));
+}
+
+// The first record and the first small task of this thread among its block's
+// (128 threads, all call), by one 64-bit atomic per block: one per warp and
+// counter, on two words every warp of the grid adds to, were what the setup
+// kernels waited for (the 10M-triangle soup: 570 us whether a triangle took
+// 55 or 31 instructions per lane). rec: 0 or 1; nt < 2^14.
+struct ReserveSm {
+    uint32_t warp[4], rec, task;
+};
+PR_DEV void block_reserve(const SetupParams& P, ReserveSm& S, uint32_t rec, uint32_t nt, uint32_t* o_rec, uint32_t* o_task) {
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    const uint32_t v = rec | (nt << 8);  // at most 128 records, 2^21 tasks a block
+    uint32_t incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= (uint32_t)d) incl += u;
     }
+    if (lane == 31) S.warp[warp] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t tot = S.warp[0] + S.warp[1] + S.warp[2] + S.warp[3];
+        unsigned long long b = 0;
+        if (tot)
+            b = atomicAdd(reinterpret_cast<unsigned long long*>(&P.cnt->n_rec),
+                          (unsigned long long)(tot & 0xffu) | (unsigned long long)(tot >> 8) << 32);
+        S.rec = (uint32_t)b;
+        S.task = (uint32_t)(b >> 32);
+    }
+    __syncthreads();
+    uint32_t off = incl - v;
+    for (uint32_t w = 0; w < warp; w++) off += S.warp[w];
+    *o_rec = S.rec + (off & 0xffu);
+    *o_task = S.task + (off >> 8);
 }
 
 // draw's transform and culls for triangle t (render/raster.go:380-436):
@@ -674,7 +702,7 @@ PR_DEV void vertex_attrs(const SetupParams& P, uint32_t t, uint32_t o, SubVtx* v
 
 // cpuForwardPass + draw for triangles fully inside the viewport
 // (render/raster.go:257-269, 380-436); clipped ones go to clip_kernel.
-PR_DEV void setup_main_one(const SetupParams& P, const ObjCache* C, uint32_t t, uint32_t* clip_list) {
+PR_DEV void setup_main_one(const SetupParams& P, const ObjCache* C, uint32_t t, uint32_t* clip_list, ReserveSm& S) {
     SubVtx v[3];
     float recipw[3];
     int matid = -1;
@@ -692,28 +720,35 @@ PR_DEV void setup_main_one(const SetupParams& P, const ObjCache* C, uint32_t t, 
     }
     __syncwarp();
     const bool emit = ok && contained, clip = ok && !contained;
-    uint32_t tot;
-    const uint32_t ci = warp_reserve(&P.cnt->n_clipped, clip ? 1u : 0u, &tot);
-    if (clip) clip_list[ci] = t;
-    uint32_t ridx = warp_reserve(&P.cnt->n_rec, emit ? 1u : 0u, &tot);
-    uint32_t area = 0, bx = 0, by = 0;
+    if (__any_sync(0xffffffffu, clip)) {  // few triangles are
+        uint32_t tot;
+        const uint32_t ci = warp_reserve(&P.cnt->n_clipped, clip ? 1u : 0u, &tot);
+        if (clip) clip_list[ci] = t;
+    }
+    PixBox pb = {0u, 0u, 0u};
+    if (emit) pb = pixel_box(box, v[0].pos, v[1].pos, v[2].pos, sabc, P.W, P.H);
+    uint32_t ridx, o;
+    const uint32_t nt = small_tasks(P, pb.area);
+    block_reserve(P, S, emit ? 1u : 0u, nt, &ridx, &o);
     if (emit) {
         if (ridx >= P.cap_rec) {
             atomicOr(&P.cnt->overflow, 1u);
             atomicMax(&P.cnt->need_rec, ridx + 1);
         } else {
             P.first_rec[t] = ridx;
-            area = write_sub(P, ridx, t * 8u, v, recipw, matid, sabc, box, &bx, &by);
+            write_sub(P, ridx, t * 8u, v, recipw, matid, sabc, pb);
         }
     }
-    emit_tasks_warp(P, ridx, area, bx, by);
+    emit_run(P, P.tasks, P.cap_tasks, o, 1u, ridx, nt);
+    emit_blocks(P, ridx, pb);
 }
 // 8 blocks per SM (64 registers, a few spilled on rare paths): more warps to
 // hide the per-triangle loads and stores measured faster than 80 registers at 6.
 __global__ void __launch_bounds__(128, 8) setup_main_kernel(const __grid_constant__ SetupParams P, uint32_t* clip_list) {
     __shared__ ObjCache C;
+    __shared__ ReserveSm S;
     if (!P.obj_trans) obj_cache_fill(P, blockIdx.x * blockDim.x, C);  // uniform
-    setup_main_one(P, &C, blockIdx.x * blockDim.x + threadIdx.x, clip_list);
+    setup_main_one(P, &C, blockIdx.x * blockDim.x + threadIdx.x, clip_list, S);
 }
 
 // clipTriangle (render/clipping.go:70-157) for the listed triangles: fan
@@ -788,7 +823,7 @@ PR_DEV void clip_one_group(const SetupParams& P, const uint32_t* clip_list, uint
     uint32_t tot;
     Counters* crec = P.cnt_rec ? P.cnt_rec : P.cnt;
     uint32_t ridx = warp_reserve(&crec->n_rec, mine ? 1u : 0u, &tot);
-    uint32_t area = 0, bx = 0, by = 0;
+    PixBox pb = {0u, 0u, 0u};
     if (mine) {
         if (ridx >= P.cap_rec) {
             atomicOr(&P.cnt->overflow, 1u);
@@ -797,12 +832,15 @@ PR_DEV void clip_one_group(const SetupParams& P, const uint32_t* clip_list, uint
             if (sub == 0) P.first_rec[t] = ridx;
             const SubVtx s3[3] = {G.cv[0], G.cv[sub + 1], G.cv[sub + 2]};
             const V4 mw[3] = {G.mw[0], G.mw[sub + 1], G.mw[sub + 2]};
-            area = write_sub(P, ridx, t * 8u + sub, s3, recipw, matid,
-                             sabc_of(s3[0].pos.x, s3[0].pos.y, s3[1].pos.x, s3[1].pos.y, s3[2].pos.x, s3[2].pos.y),
-                             scr_box(s3[0].pos, s3[1].pos, s3[2].pos), &bx, &by, attrs ? mw : nullptr);
+            const float sabc = sabc_of(s3[0].pos.x, s3[0].pos.y, s3[1].pos.x, s3[1].pos.y, s3[2].pos.x, s3[2].pos.y);
+            pb = pixel_box(scr_box(s3[0].pos, s3[1].pos, s3[2].pos), s3[0].pos, s3[1].pos, s3[2].pos, sabc, P.W, P.H);
+            write_sub(P, ridx, t * 8u + sub, s3, recipw, matid, sabc, pb, attrs ? mw : nullptr);
         }
     }
-    emit_tasks_warp(P, ridx, area, bx, by);
+    const uint32_t nt = small_tasks(P, pb.area);
+    const uint32_t o = warp_reserve(&P.cnt->n_tasks, nt, &tot);
+    emit_run(P, P.tasks, P.cap_tasks, o, 1u, ridx, nt);
+    emit_blocks(P, ridx, pb);
 }
 __global__ void __launch_bounds__(128) clip_kernel(const __grid_constant__ SetupParams P, const uint32_t* clip_list) {
     const uint32_t n = (P.cnt_rec ? P.cnt_rec : P.cnt)->n_clipped;
@@ -817,7 +855,7 @@ __global__ void __launch_bounds__(128) clip_kernel(const __grid_constant__ Setup
 }
 
 // passShadows / drawDepth for one input triangle (render/shadow.go:137-192)
-PR_DEV void setup_shadow_one(const SetupParams& P, const ObjCache* C, uint32_t t) {
+PR_DEV void setup_shadow_one(const SetupParams& P, const ObjCache* C, uint32_t t, ReserveSm& S) {
     bool ok = false;
     SubVtx v[3];
     float sabc = 0.0f;
@@ -847,18 +885,24 @@ PR_DEV void setup_shadow_one(const SetupParams& P, const ObjCache* C, uint32_t t
         }
     }
     __syncwarp();
-    uint32_t area = 0, bx = 0, by = 0;
+    PixBox pb = {0u, 0u, 0u};
+    if (ok) pb = pixel_box(box, v[0].pos, v[1].pos, v[2].pos, sabc, P.W, P.H);
+    uint32_t none, o;
+    const uint32_t nt = small_tasks(P, pb.area);
+    block_reserve(P, S, 0u, nt, &none, &o);
     if (ok) {
-        float rw[3] = {1, 1, 1};
-        area = write_sub(P, t, t, v, rw, -1, sabc, box, &bx, &by);
+        const float rw[3] = {1, 1, 1};
+        write_sub(P, t, t, v, rw, -1, sabc, pb);
     }
-    emit_tasks_warp(P, t, area, bx, by);
+    emit_run(P, P.tasks, P.cap_tasks, o, 1u, t, nt);
+    emit_blocks(P, t, pb);
 }
 // 9 blocks per SM (56 registers): more warps than at 62 registers and 8.
 __global__ void __launch_bounds__(128, 9) setup_shadow_kernel(const __grid_constant__ SetupParams P) {
     __shared__ ObjCache C;
+    __shared__ ReserveSm S;
     if (!P.obj_trans) obj_cache_fill(P, blockIdx.x * blockDim.x, C);  // uniform
-    setup_shadow_one(P, &C, blockIdx.x * blockDim.x + threadIdx.x);
+    setup_shadow_one(P, &C, blockIdx.x * blockDim.x + threadIdx.x, S);
 }
 
 // Proj·View·Model per (pass, object), the product obj_cache_fill forms.
@@ -2663,15 +2707,17 @@ __global__ void __launch_bounds__(128) setup_shadow_batch_kernel(const SetupPara
     __shared__ ObjCache C;
     const int j = job_of(blk, n_jobs, blockIdx.x);
     const uint32_t t0 = (blockIdx.x - blk[j]) * blockDim.x;
+    __shared__ ReserveSm S;
     obj_cache_fill(jobs[j], t0, C);
-    setup_shadow_one(jobs[j], &C, t0 + threadIdx.x);
+    setup_shadow_one(jobs[j], &C, t0 + threadIdx.x, S);
 }
 __global__ void __launch_bounds__(128) setup_main_batch_kernel(const SetupParams* jobs, const uint32_t* blk, int n_jobs) {
     __shared__ ObjCache C;
     const int j = job_of(blk, n_jobs, blockIdx.x);
     const uint32_t t0 = (blockIdx.x - blk[j]) * blockDim.x;
+    __shared__ ReserveSm S;
     obj_cache_fill(jobs[j], t0, C);
-    setup_main_one(jobs[j], &C, t0 + threadIdx.x, jobs[j].clip_list);
+    setup_main_one(jobs[j], &C, t0 + threadIdx.x, jobs[j].clip_list, S);
 }
 __global__ void __launch_bounds__(128) clip_batch_kernel(const SetupParams* jobs, const uint32_t* blk, int n_jobs) {
     const int j = job_of(blk, n_jobs, blockIdx.x);

@@ -56,9 +56,9 @@ constexpr uint8_t kAttrDone = 0, kAttrDeferred = 1, kAttrWanted = 2;  // written
 // Block tasks per task capacity: a task buffer of cap tasks holds cap + big_room(cap) entries.
 inline uint32_t big_room(uint32_t cap) { return cap / 4 + 64; }
 
-struct Counters {
+struct alignas(16) Counters {
     uint32_t n_rec;       // records emitted (main view)
-    uint32_t n_tasks;     // raster tasks emitted
+    uint32_t n_tasks;     // raster tasks emitted; with n_rec one 64-bit word, which setup adds to
     uint32_t overflow;    // capacity exceeded (records or tasks)
     uint32_t n_clipped;   // input triangles that were clipped
     uint32_t nan_flag;    // a NaN-depth fragment was produced
