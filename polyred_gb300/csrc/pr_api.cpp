@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdarg>
+#include <cmath>
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
@@ -578,6 +579,35 @@ void fill_shade_frame(const Ctx* c, const pr_frame_desc* f, const M4& s2w, int S
     for (uint32_t l = 0; l < f->n_lights; l++) {
         prk::LightK& K = sp.lights[l];
         K.sfast = unit_bottom(K.lview) && unit_bottom(K.lproj) && unit_bottom(svp.m) ? 1 : 0;
+        // The reference's three Applies (four roundings a row and step) stay
+        // within 12.01 u |Vp||P||V||p| of the product's exact value (u = 2^-24,
+        // double rounding included), smap rounded to float32 and applied by
+        // float32 FMAs within 5.01 u of the same.
+        double m[16], a[16], m2[16], a2[16];
+        auto mul = [](const double* p, const double* q, double* r) {
+            for (int i = 0; i < 4; i++)
+                for (int j = 0; j < 4; j++) {
+                    r[i * 4 + j] = 0;
+                    for (int k = 0; k < 4; k++) r[i * 4 + j] += p[i * 4 + k] * q[k * 4 + j];
+                }
+        };
+        double v[16], p[16], s[16], va[16], pa[16], sa[16];
+        for (int e = 0; e < 16; e++) {
+            v[e] = K.lview[e];
+            p[e] = K.lproj[e];
+            s[e] = svp.m[e];
+            va[e] = std::fabs(v[e]);
+            pa[e] = std::fabs(p[e]);
+            sa[e] = std::fabs(s[e]);
+        }
+        mul(p, v, m);
+        mul(s, m, m2);
+        mul(pa, va, a);
+        mul(sa, a, a2);
+        for (int e = 0; e < 12; e++) {
+            K.smap[e] = (float)m2[e];
+            K.serr[e] = (float)(a2[e] * (17.5 * 5.9604644775390625e-08));  // 17.5 u: float32's own rounding included
+        }
     }
     sp.SW = SW;
     sp.SH = SH;

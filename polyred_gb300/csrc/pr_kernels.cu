@@ -1571,45 +1571,25 @@ __device__ __noinline__ bool shadow_hit_exact(const ShadeParams& P, const LightK
     return false;
 }
 
-// Vec4.Apply evaluated with single-rounding FMAs, and a bound on its distance
-// from the reference's Apply (FMAs through float64) of the exact input, given
-// a bound e on the input's distance (e.w = 0: the bottom row (0, 0, 0, 1)
-// passes w through unchanged in both). Per row, both evaluations lie within
-// g sum_j |m_ij||input_j| of their exact values (g = gamma_4 = 4u'/(1-4u'),
-// u' = 2^-24 (1 + 2^-28) covering the double rounding), so
-// |fast - reference| <= sum_j |m_ij| (e_j (1 + g) + 2g |x_j|), all in upward
-// rounding (1 + g <= 1.0000005, 2g <= 4.8e-7).
-PR_DEV V4 apply4_bounded(V4 x, V4 e, const float* m, V4* eo) {
-    const V4 y = {__fmaf_rn(m[0], x.x, __fmaf_rn(m[1], x.y, __fmaf_rn(m[2], x.z, __fmul_rn(m[3], x.w)))),
-                  __fmaf_rn(m[4], x.x, __fmaf_rn(m[5], x.y, __fmaf_rn(m[6], x.z, __fmul_rn(m[7], x.w)))),
-                  __fmaf_rn(m[8], x.x, __fmaf_rn(m[9], x.y, __fmaf_rn(m[10], x.z, __fmul_rn(m[11], x.w)))),
-                  __fmaf_rn(m[12], x.x, __fmaf_rn(m[13], x.y, __fmaf_rn(m[14], x.z, __fmul_rn(m[15], x.w))))};
-    const float c1 = 1.0000005f, c2 = 4.8e-7f;
-    const float w0 = __fmaf_ru(e.x, c1, __fmul_ru(c2, fabsf(x.x))), w1 = __fmaf_ru(e.y, c1, __fmul_ru(c2, fabsf(x.y)));
-    const float w2 = __fmaf_ru(e.z, c1, __fmul_ru(c2, fabsf(x.z))), w3 = __fmul_ru(c2, fabsf(x.w));
-    *eo = V4{__fmaf_ru(fabsf(m[0]), w0, __fmaf_ru(fabsf(m[1]), w1, __fmaf_ru(fabsf(m[2]), w2, __fmul_ru(fabsf(m[3]), w3)))),
-             __fmaf_ru(fabsf(m[4]), w0, __fmaf_ru(fabsf(m[5]), w1, __fmaf_ru(fabsf(m[6]), w2, __fmul_ru(fabsf(m[7]), w3)))),
-             __fmaf_ru(fabsf(m[8]), w0, __fmaf_ru(fabsf(m[9]), w1, __fmaf_ru(fabsf(m[10]), w2, __fmul_ru(fabsf(m[11]), w3)))),
-             0.0f};
-    return y;
-}
-
-// shadow_hit_exact from the single-rounding transform, when its bound
-// decides every outcome (both truncated map coordinates and the depth
-// compare); false: undecided, the caller runs the exact test. The division
-// by w uses the same iw = RN(1/w) in both, so it scales the bound by |iw|
-// and adds two roundings (2u |sc| < 2.4e-7 |sc|); 1e-30 covers underflow.
+// shadow_hit_exact from one single-rounding transform (LightK::smap), when
+// its bound (LightK::serr) decides every outcome (both truncated map
+// coordinates and the depth compare); false: undecided, the caller runs the
+// exact test. w passes through the three bottom rows (0, 0, 0, 1) unchanged,
+// so the division uses the same iw = RN(1/w) in both; it scales the bound by
+// |iw| and adds two roundings (2u |sc| < 2.4e-7 |sc|); 1e-30 covers underflow.
 PR_DEV bool shadow_hit_fast(const ShadeParams& P, const LightK& L, V4 ws, size_t plane, int li, bool* hit) {
-    V4 e = {0.0f, 0.0f, 0.0f, 0.0f};
-    V4 v = apply4_bounded(ws, e, L.lview, &e);
-    v = apply4_bounded(v, e, L.lproj, &e);
-    v = apply4_bounded(v, e, P.shadow_vp, &e);
-    float sx = v.x, sy = v.y, sz = v.z, ia = 1.0f;
-    if (!(v.w == 1.0f || v.w == 0.0f)) {  // pos4
-        const float iw = __fdiv_rn(1.0f, v.w);
-        sx = __fmul_rn(v.x, iw);
-        sy = __fmul_rn(v.y, iw);
-        sz = __fmul_rn(v.z, iw);
+    const float* m = L.smap;
+    const float* q = L.serr;
+    const float ax = fabsf(ws.x), ay = fabsf(ws.y), az = fabsf(ws.z), aw = fabsf(ws.w);
+    auto row = [&](const float* r) { return __fmaf_rn(r[0], ws.x, __fmaf_rn(r[1], ws.y, __fmaf_rn(r[2], ws.z, __fmul_rn(r[3], ws.w)))); };
+    auto err = [&](const float* r) { return __fmaf_ru(r[0], ax, __fmaf_ru(r[1], ay, __fmaf_ru(r[2], az, __fmul_ru(r[3], aw)))); };
+    const V4 e = {err(q), err(q + 4), err(q + 8), 0.0f};
+    float sx = row(m), sy = row(m + 4), sz = row(m + 8), ia = 1.0f;
+    if (!(ws.w == 1.0f || ws.w == 0.0f)) {  // pos4
+        const float iw = __frcp_rn(ws.w);
+        sx = __fmul_rn(sx, iw);
+        sy = __fmul_rn(sy, iw);
+        sz = __fmul_rn(sz, iw);
         ia = __fmul_ru(fabsf(iw), 1.0000002f);
     }
     const float dx = __fadd_ru(__fmaf_ru(ia, e.x, __fmul_ru(2.4e-7f, fabsf(sx))), 1e-30f);

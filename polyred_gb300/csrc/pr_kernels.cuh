@@ -79,7 +79,8 @@ struct LightK {
     float color[3];
     float lview[16], lproj[16];
     int32_t sfast;    // 1: the bottom rows of lview, lproj and the map viewport are exactly (0, 0, 0, 1)
-    int32_t pad_[3];
+    float smap[12];   // with sfast: the rows x, y, z of map viewport * lproj * lview,
+    float serr[12];   // and of the bound on a single-rounded smap * p against the reference's three Applies, per |p|
 };
 
 // Per-view setup parameters (passed by value).
