@@ -182,6 +182,7 @@ struct Ctx {
     // submitted frames: scene uploads and host-output copies on their own streams
     cudaStream_t stream_u = nullptr, stream_d = nullptr;
     cudaEvent_t ev_frame = nullptr, ev_d2h = nullptr;
+    bool submitted = false;  // ev_d2h has been recorded
     // raster work space
     DevBuf<prk::RasterRec> rrec;
     DevBuf<prk::AttrRec> arec;
@@ -216,18 +217,16 @@ struct Ctx {
     DevBuf<float4> d_vcol;                 // scene colours / 255, when the caller gives none
     DevBuf<double> d_acc;
     pr_stats stats{};
-    cudaEvent_t ev[6] = {};
+    cudaEvent_t ev[3] = {};  // the frame: start, shadow maps complete, end
     // shadow passes run on their own stream, with their own records and tasks
     cudaStream_t stream_s = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    bool shadows_ran = false;  // the last frame drew a shadow pass (ev[0] to ev[1])
     DevBuf<prk::RasterRec> rrec_s;
     DevBuf<uint2> tasks_s;
-    // clipped sub-triangles: clipped and rasterised on a third stream beside the main raster
-    cudaStream_t stream_c = nullptr;
-    cudaEvent_t ev_setup = nullptr, ev_clip = nullptr;
-    DevBuf<uint2> tasks_c;
+    DevBuf<uint2> tasks_c;  // the clipped sub-triangles' tasks
     // AO's march on stream 3 beside attributes and shading: after resolve,
     // joined before the AO colour scaling
+    cudaStream_t stream_c = nullptr;
     cudaEvent_t ev_resolved = nullptr, ev_ao0 = nullptr, ev_ao = nullptr;
     bool ao_marched = false;  // the last frame ran the AO march (ev_ao0, ev_ao hold it)
     DevBuf<float> ao_T;
@@ -463,6 +462,21 @@ int inverses_std(const float* vp_inv, const float* proj_inv) {
     return 1;
 }
 
+// The raster parameters of light l's shadow pass (counters cnt), without mode and queue.
+prk::RasterParams shadow_raster(Ctx* c, prk::Counters* cnt, int SW, int SH, int l) {
+    prk::RasterParams rp{};
+    rp.rrec = c->rrec_s.p;
+    rp.tasks = c->tasks_s.p;
+    rp.big = rp.tasks + c->cap_tasks;
+    rp.cnt = cnt;
+    rp.cnt_w = cnt;
+    rp.W = SW;
+    rp.H = SH;
+    rp.smap = c->smap.p + (size_t)SW * SH * l;
+    rp.lastnan = c->lastnan.p;
+    return rp;
+}
+
 void fill_scene_ptrs(Ctx* c, prk::SetupParams& p) {
     p.pos = c->sb.pos.p;
     p.nor = c->sb.nor.p;
@@ -524,11 +538,17 @@ void collect_stats(Ctx* c) {
         }
         return ms;
     };
-    c->stats.ms_shadow = span(c->ev[0], c->ev[1]);
-    c->stats.ms_setup = span(c->ev[0], c->ev[2]);  // concurrent with the shadow passes
-    c->stats.ms_raster = span(c->ev[2], c->ev[3]);
-    c->stats.ms_shade = span(c->ev[3], c->ev[4]);
-    c->stats.ms_total = span(c->ev[0], c->ev[4]);
+    // the main pass's phases by the device clock its kernels wrote (an event
+    // between two kernels would keep the second from starting early)
+    auto since = [&](int k) {
+        const unsigned long long t0 = c->h_cnt[0].stamp[0], t = c->h_cnt[0].stamp[k];
+        return t > t0 ? (float)((double)(t - t0) * 1e-6) : 0.0f;
+    };
+    c->stats.ms_shadow = c->shadows_ran ? span(c->ev[0], c->ev[1]) : 0.0f;
+    c->stats.ms_total = span(c->ev[0], c->ev[2]);
+    c->stats.ms_setup = since(1);  // concurrent with the shadow passes
+    c->stats.ms_raster = std::max(since(2) - since(1), 0.0f);
+    c->stats.ms_shade = std::max(c->stats.ms_total - since(2), 0.0f);
     c->stats.ms_ao = c->ao_marched ? span(c->ev_ao0, c->ev_ao) : 0.0f;  // the march, beside shading
     c->stats.n_ao_pixels = c->h_cnt[0].n_ao;
 }
@@ -724,76 +744,94 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
     uint32_t launches = 0;
 
     {
-        CUDA_TRY(cudaMemsetAsync(dcnt, 0, sizeof(prk::Counters) * prk::kNumCounters, st));
         CUDA_TRY(cudaEventRecord(c->ev[0], st));
-        // Proj·View·Model of every object for the main pass (0) and each light (1 + l)
         const uint32_t n_obj = (uint32_t)c->sb.objects.size();
-        const int n_pass = shadows ? 1 + NL : 1;
+        bool casts = false;
+        for (int l = 0; shadows && l < NL; l++) casts = casts || f->lights[l].cast_shadow;
+        c->shadows_ran = casts;
+        if ((rc = c->obj_trans.ensure((size_t)(1 + NL) * std::max<uint32_t>(n_obj, 1) * 16))) return rc;
+        // The counter rows of the shadow passes start on their stream, every
+        // other row here, with Proj·View·Model of every object.
+        const uint32_t light_rows = casts ? ((1u << NL) - 1u) << 1 : 0u;
         {
             prk::PassMats pm;
             std::memcpy(pm.pv[0], pv.m, 64);
-            for (int l = 0; shadows && l < NL; l++) {
-                const M4 lpv = prh::mulm(loadm(f->lights[l].shadow_proj), loadm(f->lights[l].shadow_view));
-                std::memcpy(pm.pv[1 + l], lpv.m, 64);
-            }
-            if ((rc = c->obj_trans.ensure((size_t)n_pass * std::max<uint32_t>(n_obj, 1) * 16))) return rc;
-            KTRY(prk::launch_obj_trans(pm, n_pass, c->sb.obj_model.p, n_obj, c->obj_trans.p, st));
+            KTRY(prk::launch_pass_init(pm, 1, c->sb.obj_model.p, n_obj, c->obj_trans.p, dcnt, ~light_rows, st));
             launches += 1;
         }
         // ---- shadow passes (render/raster.go:176-184), on their own stream:
-        // only the deferred pass reads the maps ----
+        // only the deferred pass reads the maps. The host submits them behind
+        // the main pass's raster, in two parts: a launch costs it 3.4 us, as
+        // long as a small frame's kernels, and the main chain is the longer.
         cudaStream_t ss = c->stream_s;
-        CUDA_TRY(cudaEventRecord(c->ev_fork, st));
-        CUDA_TRY(cudaStreamWaitEvent(ss, c->ev_fork, 0));
-        if (shadows) {
-            M4 svp = prh::viewport((float)SW, (float)SH);
+        const M4 svp = prh::viewport((float)SW, (float)SH);
+        auto shadow_draw = [&](int l) -> int {
+            prk::SetupParams sp{};
+            fill_scene_ptrs(c, sp);
+            sp.W = SW;
+            sp.H = SH;
+            sp.msaa = M;
+            sp.perspective = 0;
+            M4 lpv = prh::mulm(loadm(f->lights[l].shadow_proj), loadm(f->lights[l].shadow_view));
+            std::memcpy(sp.pv, lpv.m, 64);
+            std::memcpy(sp.viewport, svp.m, 64);
+            sp.vp_std = viewport_std(sp.viewport);
+            sp.rrec = c->rrec_s.p;
+            sp.arec = nullptr;
+            sp.cap_rec = c->cap_rec;
+            sp.tasks = c->tasks_s.p;
+            sp.cap_tasks = c->cap_tasks;
+            sp.cap_big = prk::big_room(c->cap_tasks);
+            sp.first_rec = nullptr;
+            sp.cnt = dcnt + 1 + l;
+            sp.obj_trans = c->obj_trans.p + (size_t)(1 + l) * n_obj * 16;
+            KTRY(prk::launch_setup_shadow(sp, ss));
+            prk::RasterParams rp = shadow_raster(c, dcnt + 1 + l, SW, SH, l);
+            rp.mode = prk::kShadow;
+            rp.take = &dcnt[1 + l].take[0];
+            KTRY(prk::launch_raster(rp, c->n_sms * 8, ss));
+            launches += 2;
+            return PR_OK;
+        };
+        // the NaN fix-up (each kernel returns at once without a NaN fragment)
+        auto shadow_nan = [&](int l) -> int {
+            prk::RasterParams rp = shadow_raster(c, dcnt + 1 + l, SW, SH, l);
+            KTRY(prk::launch_shadow_fixup_reset(SW, SH, c->lastnan.p, rp.smap, dcnt + 1 + l, ss));
+            rp.mode = prk::kShadowFixup;
+            rp.take = &dcnt[1 + l].take[1];
+            KTRY(prk::launch_raster(rp, c->n_sms * 8, ss));
+            KTRY(prk::launch_nan_cleanup((size_t)SW * SH, c->lastnan.p, 0u, nullptr, 0u, dcnt + 1 + l, ss));
+            launches += 3;
+            return PR_OK;
+        };
+        auto shadows_begin = [&]() -> int {
+            if (!casts) return PR_OK;
+            if (c->sb.n_tris > c->cap_rec) return fail(PR_ERR_OVERFLOW, "record capacity below triangle count");
+            CUDA_TRY(cudaStreamWaitEvent(ss, c->ev[0], 0));
+            prk::PassMats pm;
+            for (int l = 0; l < NL; l++) {
+                const M4 lpv = prh::mulm(loadm(f->lights[l].shadow_proj), loadm(f->lights[l].shadow_view));
+                std::memcpy(pm.pv[l], lpv.m, 64);
+            }
+            KTRY(prk::launch_pass_init(pm, NL, c->sb.obj_model.p, n_obj, c->obj_trans.p + (size_t)n_obj * 16, dcnt,
+                                       light_rows, ss));
+            launches += 1;
+            for (int l = 0; l < NL; l++)
+                if (f->lights[l].cast_shadow) return shadow_draw(l);
+            return PR_OK;
+        };
+        auto shadows_finish = [&]() -> int {
+            if (!casts) return PR_OK;
+            bool drawn = true;  // the first casting light is
             for (int l = 0; l < NL; l++) {
                 if (!f->lights[l].cast_shadow) continue;
-                prk::SetupParams sp{};
-                fill_scene_ptrs(c, sp);
-                sp.W = SW;
-                sp.H = SH;
-                sp.msaa = M;
-                sp.perspective = 0;
-                M4 lpv = prh::mulm(loadm(f->lights[l].shadow_proj), loadm(f->lights[l].shadow_view));
-                std::memcpy(sp.pv, lpv.m, 64);
-                std::memcpy(sp.viewport, svp.m, 64);
-                sp.vp_std = viewport_std(sp.viewport);
-                sp.rrec = c->rrec_s.p;
-                sp.arec = nullptr;
-                sp.cap_rec = c->cap_rec;
-                sp.tasks = c->tasks_s.p;
-                sp.cap_tasks = c->cap_tasks;
-                sp.cap_big = prk::big_room(c->cap_tasks);
-                sp.first_rec = nullptr;
-                sp.cnt = dcnt + 1 + l;
-                sp.obj_trans = c->obj_trans.p + (size_t)(1 + l) * n_obj * 16;
-                if (c->sb.n_tris > c->cap_rec) return fail(PR_ERR_OVERFLOW, "record capacity below triangle count");
-                uint32_t* plane = c->smap.p + (size_t)SW * SH * l;
-                KTRY(prk::launch_setup_shadow(sp, ss));
-                prk::RasterParams rp{};
-                rp.rrec = c->rrec_s.p;
-                rp.tasks = c->tasks_s.p;
-                rp.big = rp.tasks + c->cap_tasks;
-                rp.cnt = dcnt + 1 + l;
-                rp.cnt_w = dcnt + 1 + l;
-                rp.W = SW;
-                rp.H = SH;
-                rp.mode = prk::kShadow;
-                rp.smap = plane;
-                rp.lastnan = c->lastnan.p;
-                rp.take = &dcnt[1 + l].take[0];
-                KTRY(prk::launch_raster(rp, c->n_sms * 8, ss));
-                KTRY(prk::launch_shadow_fixup_reset(SW, SH, c->lastnan.p, plane, dcnt + 1 + l, ss));
-                rp.mode = prk::kShadowFixup;
-                rp.take = &dcnt[1 + l].take[1];
-                KTRY(prk::launch_raster(rp, c->n_sms * 8, ss));
-                KTRY(prk::launch_nan_cleanup((size_t)SW * SH, c->lastnan.p, 0u, nullptr, 0u, dcnt + 1 + l, ss));
-                launches += 5;
+                int rc2 = drawn ? PR_OK : shadow_draw(l);
+                if (rc2 || (rc2 = shadow_nan(l))) return rc2;
+                drawn = false;
             }
-        }
-        CUDA_TRY(cudaEventRecord(c->ev[1], ss));
-        CUDA_TRY(cudaEventRecord(c->ev_join, ss));
+            CUDA_TRY(cudaEventRecord(c->ev[1], ss));
+            return PR_OK;
+        };
         // ---- forward pass (render/raster.go:226-273) ----
         prk::SetupParams mp{};
         fill_scene_ptrs(c, mp);
@@ -823,21 +861,20 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             if ((rc = c->tri_scr.ensure((size_t)std::max<uint32_t>(c->sb.n_tris, 1) * 12))) return rc;
             mp.tri_scr = c->tri_scr.p;
         }
-        CUDA_TRY(cudaMemsetAsync(c->keys.p, 0, npx * 8, st));
+        mp.clear = c->keys.p;
+        mp.n_clear = npx;
         KTRY(prk::launch_setup_main_only(mp, c->clip_list.p, st));
-        CUDA_TRY(cudaEventRecord(c->ev[2], st));
-        // clipped triangles: their own task list and stream; records and the
-        // NaN flag stay the main pass's (visibility is order-independent)
-        cudaStream_t sc = c->stream_c;
+        // clipped triangles: their own task list; records and the NaN flag
+        // stay the main pass's (visibility is order-independent). The raster
+        // of the others is released as soon as every clipping block has
+        // started, and the clipped ones' follows it.
         prk::Counters* dclip = dcnt + prk::kClipCnt;
-        CUDA_TRY(cudaEventRecord(c->ev_setup, st));
-        CUDA_TRY(cudaStreamWaitEvent(sc, c->ev_setup, 0));
         prk::SetupParams cp = mp;
         cp.defer_attr = 0;  // clipped sub-triangles carry interpolated attributes: written at once
         cp.cnt = dclip;
         cp.cnt_rec = dcnt;
         cp.tasks = c->tasks_c.p;
-        KTRY(prk::launch_clip(cp, c->clip_list.p, sc));
+        KTRY(prk::launch_clip(cp, c->clip_list.p, st));
         prk::RasterParams rp{};
         rp.rrec = c->rrec.p;
         rp.tasks = c->tasks.p;
@@ -851,36 +888,38 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         rp.nanseq = c->nanseq.p;
         rp.beaten = c->beaten.p;
         rp.take = &dcnt[0].take[0];
+        rp.after_clip = 1;
+        KTRY(prk::launch_raster(rp, c->n_sms * 8, st));
         prk::RasterParams rc_ = rp;
+        rc_.after_clip = 0;
         rc_.tasks = c->tasks_c.p;
         rc_.big = rc_.tasks + c->cap_tasks;
         rc_.cnt = dclip;
         rc_.take = &dclip->take[0];
         rc_.grab = 32;  // a short list (the frame's clipped triangles): spread it over warps
-        KTRY(prk::launch_raster(rc_, c->n_sms * 8, sc));
-        CUDA_TRY(cudaEventRecord(c->ev_clip, sc));
-        KTRY(prk::launch_raster(rp, c->n_sms * 8, st));
-        CUDA_TRY(cudaStreamWaitEvent(st, c->ev_clip, 0));
-        // the NaN fix-up of both lists in one launch (it returns at once
-        // without a NaN fragment)
+        KTRY(prk::launch_raster(rc_, c->n_sms * 8, st));
+        if ((rc = shadows_begin())) return rc;
+        // the NaN fix-up of both lists (it returns at once without a NaN fragment)
+        rp.after_clip = 0;
         rp.mode = prk::kMainFixup;
         rp.take = &dcnt[0].take[1];
-        rp.tasks2 = c->tasks_c.p;
+        rp.tasks2 = rc_.tasks;
         rp.big2 = rc_.big;
         rp.cnt2 = dclip;
         rp.take2 = &dclip->take[1];
         KTRY(prk::launch_raster(rp, c->n_sms * 8, st));
         // AmbientOcclusionShade's march needs only the resolved depths: resolve
-        // lists its pixels, and they are marched on stream 3 (free after the
-        // clipped raster) while stream 1 writes attributes and shades; the
-        // colour scaling joins after shading. A scene without an AO material
-        // lists no pixel, and both launches are left out.
+        // lists its pixels, and they are marched on stream 3 while stream 1
+        // writes attributes and shades; the colour scaling joins after shading.
+        // A scene without an AO material lists no pixel, and both launches are
+        // left out.
         const bool with_ao = out && out->rgba && c->sb.has_ao;
         c->ao_marched = with_ao;
         if (with_ao && ((rc = c->ao_T.ensure(npx)) || (rc = c->linemax.ensure(4 * npx)))) return rc;
         KTRY(prk::launch_resolve(W, H, c->keys.p, c->nanseq.p, c->beaten.p, dcnt, c->win.p, c->depth_ao.p, c->first_rec.p,
                                  c->attr_state.p, c->sb.tri_flags.p, with_ao ? c->ao_list.p : nullptr, c->linemax.p, st));
         prk::AoParams ap{};
+        cudaStream_t sc = c->stream_c;
         if (with_ao) {
             CUDA_TRY(cudaEventRecord(c->ev_resolved, st));
             CUDA_TRY(cudaStreamWaitEvent(sc, c->ev_resolved, 0));
@@ -909,9 +948,9 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             CUDA_TRY(cudaEventRecord(c->ev_ao, sc));
             launches += 1;
         }
-        KTRY(prk::launch_attr(mp, st));
-        CUDA_TRY(cudaEventRecord(c->ev[3], st));
+        KTRY(prk::launch_attr(mp, !with_ao, st));
         launches += 7;
+        if ((rc = shadows_finish())) return rc;
 
         // ---- deferred shading + gamma (render/raster.go:275-378) ----
         std::unique_ptr<prk::ShadeParams> sp_owner(new (std::nothrow) prk::ShadeParams());
@@ -957,12 +996,10 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             sp.rgba = (uchar4*)c->o_msaa.p;  // the framebuffer's colours
         }
         sp.ao_listed = 1;  // listed by resolve
-        CUDA_TRY(cudaStreamWaitEvent(st, c->ev_join, 0));  // the shadow maps are complete
-        CUDA_TRY(cudaStreamWaitEvent(st, c->ev_d2h, 0));   // a submitted frame's outputs left the staging
-        KTRY(prk::launch_shade(sp, st));
+        if (casts) CUDA_TRY(cudaStreamWaitEvent(st, c->ev[1], 0));          // the shadow maps are complete
+        if (c->submitted) CUDA_TRY(cudaStreamWaitEvent(st, c->ev_d2h, 0));  // a submitted frame's outputs left the staging
+        KTRY(prk::launch_shade(sp, !casts && !c->submitted, st));
         launches += 1;
-        CUDA_TRY(cudaEventRecord(c->sb.ev_released, st));  // the scene buffers are read no more
-        CUDA_TRY(cudaEventRecord(c->ev[5], st));
         if (sp.rgba) {
             if (with_ao) {
                 // AmbientOcclusionShade's colour scaling and gamma of the listed
@@ -979,7 +1016,8 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
                 launches += 1;
             }
         }
-        CUDA_TRY(cudaEventRecord(c->ev[4], st));
+        CUDA_TRY(cudaEventRecord(c->ev[2], st));
+        CUDA_TRY(cudaEventRecord(c->sb.ev_released, st));  // the scene buffers are read no more
         CUDA_TRY(cudaMemcpyAsync(c->h_cnt, dcnt, sizeof(prk::Counters) * prk::kNumCounters, cudaMemcpyDeviceToHost, st));
         if (!sync) {
             c->stats.n_kernel_launches = launches;
@@ -989,6 +1027,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
                 CUDA_TRY(cudaStreamWaitEvent(c->stream_d, c->ev_frame, 0));
                 if ((rc = copy_host_outputs(c, out, npx, npx_img, c->stream_d))) return rc;
                 CUDA_TRY(cudaEventRecord(c->ev_d2h, c->stream_d));
+                c->submitted = true;
             }
             return PR_OK;
         }
@@ -1070,9 +1109,10 @@ int pr_create(int device, void** out_ctx) {
     c->device = device;
     int rc = set_device(c);
     if (rc) { delete c; return rc; }
-    // Stream 3 (clipped raster, then AO's march: the frame's longest chain
-    // after resolve) takes the device's highest priority, so that its blocks
-    // go first and shading and the shadow passes fill the rest.
+    // Stream 3 (AO's march: the frame's longest chain after resolve) takes the
+    // device's highest priority, so that its blocks go first and shading and
+    // the shadow passes fill the rest (shading or shadows above it: 1M-triangle
+    // field at 1080p 573 -> 590 us and more).
     int prio_lo = 0, prio_hi = 0;
     if (cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) != cudaSuccess) prio_hi = 0;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
@@ -1081,11 +1121,7 @@ int pr_create(int device, void** out_ctx) {
     }
     for (auto& ev : c->ev) cudaEventCreate(&ev);
     if (cudaStreamCreateWithFlags(&c->stream_s, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithPriority(&c->stream_c, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_setup, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_clip, cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream_u, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream_d, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_frame, cudaEventDisableTiming) != cudaSuccess ||
@@ -1142,8 +1178,6 @@ int pr_destroy(void* ctx) {
     c->tri_scr.release(); c->d_kd.release(); c->d_ks.release(); c->d_shin.release(); c->d_vcol.release();
     c->d_acc.release();
     c->rrec_s.release(); c->tasks_s.release(); c->tasks_c.release();
-    if (c->ev_setup) cudaEventDestroy(c->ev_setup);
-    if (c->ev_clip) cudaEventDestroy(c->ev_clip);
     if (c->ev_resolved) cudaEventDestroy(c->ev_resolved);
     if (c->ev_ao0) cudaEventDestroy(c->ev_ao0);
     if (c->ev_ao) cudaEventDestroy(c->ev_ao);
@@ -1155,8 +1189,6 @@ int pr_destroy(void* ctx) {
     if (c->h_cnt) cudaFreeHost(c->h_cnt);
     for (auto& ev : c->ev)
         if (ev) cudaEventDestroy(ev);
-    if (c->ev_fork) cudaEventDestroy(c->ev_fork);
-    if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->stream_s) {
         cudaStreamSynchronize(c->stream_s);
         cudaStreamDestroy(c->stream_s);

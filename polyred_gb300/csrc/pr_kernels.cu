@@ -35,6 +35,22 @@ PR_DEV float approx_ex2(float x) { float r; asm("ex2.approx.f32 %0, %1;" : "=f"(
 PR_DEV float approx_rsq(float x) { float r; asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 PR_DEV float approx_rcp(float x) { float r; asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 
+// A frame's dependent launches are programmatic: a kernel's blocks become
+// resident while its predecessor drains, and wait here for it to complete (and
+// its writes to be seen) before their first access. Between plain launches of
+// a small frame the device idled 3 to 4 us each (frames of 800x500 to
+// 1280x720: 96, 164 and 192 us, so 69, 131 and 152). A kernel releases its
+// successor only past its own wait, so that completion stays transitive, and
+// only a short one does so before its end: waiting blocks hold registers that
+// another stream's kernels could use.
+PR_DEV void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+PR_DEV void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+PR_DEV unsigned long long device_clock() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
 PR_DEV V4 ld4(const float4 q) { return {q.x, q.y, q.z, q.w}; }
 
 // Mat4.MulM (math/mat4.go:201-220), plain float32 sums left to right.
@@ -298,23 +314,26 @@ PR_DEV V4 intersect_segment(V4 P, V4 N, V4 v0, V4 v1) {
 // own, as the reference's loop does at step i, and places its 0, 1 or 2 output
 // vertices at the exclusive prefix sum of the counts, so each output polygon
 // is the loop's, vertex for vertex; an overflow check at step i would see the
-// same prefix count. All 32 lanes of the warp call; a lane outside [0, n) holds
-// nothing. Returns the vertex count (or -1) to every lane of the group, and
-// lane i < count gets vertex i in *v. ring: the group's 2 x 10 vertices of
-// shared scratch.
+// same prefix count. One copy of a plane's code, and a plane that cuts nothing
+// is left at once: the instructions a small frame's few warps fetch are what
+// the clip kernel waits for (planes 6.4 -> 3.6 us of 18 in a 641x479 frame).
+// All 32 lanes of the warp call; a lane outside [0, n) holds nothing. Returns
+// the vertex count (or -1) to every lane of the group, and lane i < count gets
+// vertex i in *v. ring: the group's 2 x 10 vertices of shared scratch.
 constexpr int kClipLanes = 16;  // >= 9 polygon vertices
 PR_DEV int sutherland_hodgman_group(V4* v, int n, float w, float h, uint32_t sub, V4 (*ring)[10]) {
     const unsigned full = 0xffffffffu;
     const uint32_t gbase = (threadIdx.x & 31u) & ~(uint32_t)(kClipLanes - 1);
-    const float pp[6][4] = {{w, 0, 0, 1}, {0, 0, 0, 1}, {0, h, 0, 1}, {0, 0, 0, 1}, {0, 0, 1, 1}, {0, 0, -1, 1}};
-    const float pn[6][4] = {{-1, 0, 0, 1}, {1, 0, 0, 1}, {0, -1, 0, 1}, {0, 1, 0, 1}, {0, 0, -1, 1}, {0, 0, 1, 1}};
     int res = n;
+#pragma unroll 1
     for (int pl = 0; pl < 6; pl++) {
-        const V4 P = {pp[pl][0], pp[pl][1], pp[pl][2], pp[pl][3]};
-        const V4 N = {pn[pl][0], pn[pl][1], pn[pl][2], pn[pl][3]};
+        const V4 P = {pl == 0 ? w : 0.0f, pl == 2 ? h : 0.0f, pl == 4 ? 1.0f : pl == 5 ? -1.0f : 0.0f, 1.0f};
+        const V4 N = {pl == 0 ? -1.0f : pl == 1 ? 1.0f : 0.0f, pl == 2 ? -1.0f : pl == 3 ? 1.0f : 0.0f,
+                      pl == 4 ? -1.0f : pl == 5 ? 1.0f : 0.0f, 1.0f};
         const bool act = (int)sub < n;  // n == 0 (an empty polygon, or a finished group): no lane acts
         const V4 e = *v;
         const bool fe = act && dot4(sub4(e, P), N) > 0.0f;
+        if (!__any_sync(full, act && !fe)) continue;  // every vertex inside: the polygons stay (res holds n)
         const int src = sub == 0u ? n - 1 : (int)sub - 1;  // the previous vertex (the last one for vertex 0)
         V4 sv;
         sv.x = __shfl_sync(full, e.x, src < 0 ? 0 : src, kClipLanes);
@@ -747,6 +766,23 @@ PR_DEV void setup_main_one(const SetupParams& P, const ObjCache* C, uint32_t t, 
 __global__ void __launch_bounds__(128, 8) setup_main_kernel(const __grid_constant__ SetupParams P, uint32_t* clip_list) {
     __shared__ ObjCache C;
     __shared__ ReserveSm S;
+    const uint32_t tri_blocks = (P.n_tris + 127u) / 128u;
+    if (blockIdx.x >= tri_blocks) {
+        // The raster's keys to 0, beside the triangles' latency-bound chains
+        // (a memset before them: 12 us of a 4K frame).
+        const size_t at = ((size_t)(blockIdx.x - tri_blocks) * 128u + threadIdx.x) * 2u;
+        const size_t step = (size_t)(gridDim.x - tri_blocks) * 256u;
+        for (size_t i = at; i < P.n_clear; i += step) {
+            if (i + 1u < P.n_clear)
+                *reinterpret_cast<ulonglong2*>(P.clear + i) = make_ulonglong2(0ull, 0ull);
+            else
+                P.clear[i] = 0ull;
+        }
+        after_previous();
+        return;
+    }
+    after_previous();
+    release_next();
     if (!P.obj_trans) obj_cache_fill(P, blockIdx.x * blockDim.x, C);  // uniform
     setup_main_one(P, &C, blockIdx.x * blockDim.x + threadIdx.x, clip_list, S);
 }
@@ -843,6 +879,8 @@ PR_DEV void clip_one_group(const SetupParams& P, const uint32_t* clip_list, uint
     emit_blocks(P, ridx, pb);
 }
 __global__ void __launch_bounds__(128) clip_kernel(const __grid_constant__ SetupParams P, const uint32_t* clip_list) {
+    after_previous();
+    release_next();  // the raster starts on the unclipped triangles' tasks
     const uint32_t n = (P.cnt_rec ? P.cnt_rec : P.cnt)->n_clipped;
     constexpr uint32_t kPerBlock = 128 / kClipLanes;
     __shared__ ClipGroupSm s_g[kPerBlock];
@@ -901,13 +939,23 @@ PR_DEV void setup_shadow_one(const SetupParams& P, const ObjCache* C, uint32_t t
 __global__ void __launch_bounds__(128, 9) setup_shadow_kernel(const __grid_constant__ SetupParams P) {
     __shared__ ObjCache C;
     __shared__ ReserveSm S;
+    after_previous();
     if (!P.obj_trans) obj_cache_fill(P, blockIdx.x * blockDim.x, C);  // uniform
     setup_shadow_one(P, &C, blockIdx.x * blockDim.x + threadIdx.x, S);
 }
 
+// What a frame's passes start from: the counter rows of `rows` at zero, and
 // Proj·View·Model per (pass, object), the product obj_cache_fill forms.
-__global__ void obj_trans_kernel(const __grid_constant__ PassMats pm, int n_pass, const float* obj_model,
-                                 uint32_t n_objects, float* out) {
+__global__ void pass_init_kernel(const __grid_constant__ PassMats pm, int n_pass, const float* obj_model,
+                                 uint32_t n_objects, float* out, Counters* cnt, uint32_t rows) {
+    release_next();  // launched in full order itself
+    if (blockIdx.x == 0) {
+        constexpr uint32_t kWords = sizeof(Counters) / 4;
+        for (uint32_t e = threadIdx.x; e < kWords * (uint32_t)kNumCounters; e += blockDim.x)
+            if ((rows >> (e / kWords)) & 1u) reinterpret_cast<uint32_t*>(cnt)[e] = 0u;
+        __syncthreads();
+        if (threadIdx.x == 0 && (rows & 1u)) cnt->stamp[0] = device_clock();
+    }
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (size_t)n_pass * n_objects * 16) return;
     const size_t po = e >> 4;
@@ -1228,12 +1276,25 @@ PR_DEV void raster_block(const RasterParams& P, uint2 task, uint32_t part, uint3
 constexpr uint32_t kSpreadShare = 33;  // lists with fewer tasks per warp than this (and than grab) are spread
 __global__ void __launch_bounds__(kRasterWarps * 32, 6) raster_kernel(const __grid_constant__ RasterParams P) {
     __shared__ RasterWarpSm s_w[kRasterWarps];
+    // after_clip: clip_kernel released this one past its own wait for setup, so
+    // the list is complete. One block waits for clip_kernel, so that the next
+    // kernel finds the clipped list complete; more of them would only keep the
+    // shadow passes off the device.
+    if (P.after_clip) {
+        __threadfence();  // acquire setup's writes: no stale line in this SM's L1
+        if (blockIdx.x == 0 && threadIdx.x == 0) P.cnt_w->stamp[1] = device_clock();
+    } else {
+        after_previous();
+    }
     if (P.mode == kMainFixup || P.mode == kShadowFixup) {
         if (P.cnt_w->nan_flag == 0) return;  // flags of every list of the pass meet in cnt_w
     }
     const Counters* c = P.cnt;
     const uint32_t n_tasks = c->n_tasks;
-    if (c->overflow) return;
+    if (c->overflow) {
+        if (P.after_clip && blockIdx.x == 0) after_previous();
+        return;
+    }
     const int warp = threadIdx.x >> 5;
     const uint32_t nw = gridDim.x * kRasterWarps;
     // Block tasks by warp index (a few per warp), after the small ones (before
@@ -1279,6 +1340,7 @@ __global__ void __launch_bounds__(kRasterWarps * 32, 6) raster_kernel(const __gr
     };
     drain(P.tasks, P.take, n_tasks);
     if (P.big) drain_big(P.big, c->n_big);
+    if (P.after_clip && blockIdx.x == 0) after_previous();
     if (P.tasks2 && !P.cnt2->overflow) {
         drain(P.tasks2, P.take2, P.cnt2->n_tasks);
         drain_big(P.big2, P.cnt2->n_big);
@@ -1359,6 +1421,8 @@ __global__ void __launch_bounds__(256) resolve_kernel(int W, int H, const unsign
                                                       uint32_t* beaten, Counters* cnt, uint32_t* win, float* depth_ao,
                                                       const uint32_t* first_rec, uint8_t* attr_state,
                                                       const uint8_t* tri_flags, uint32_t* ao_list, float* linemax) {
+    after_previous();
+    release_next();
     const int x = (int)(blockIdx.x * 32 + tile_x(threadIdx.x)), r = (int)(blockIdx.y * 8 + tile_y(threadIdx.x));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     bool ao = false;
@@ -1418,6 +1482,8 @@ constexpr int kAttrRun = 128;
 __global__ void __launch_bounds__(128) attr_kernel(const __grid_constant__ SetupParams P) {
     __shared__ __align__(16) float s_rec[4][10][36];  // each warp's ten records (36: their words in different banks)
     __shared__ uint32_t s_idx[4][kAttrRun];
+    after_previous();
+    release_next();
     const uint32_t n = min(P.cnt->n_rec, P.cap_rec);  // setup and clip wrote the state of each
     const int lane = threadIdx.x & 31, r = lane / 3, k = lane - 3 * r, warp = threadIdx.x >> 5;
     const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -1494,6 +1560,8 @@ __global__ void __launch_bounds__(128) attr_kernel(const __grid_constant__ Setup
 // (A small persistent grid: with no NaN fragment, the usual case, every block
 // reads the flag and leaves.)
 __global__ void shadow_fixup_reset_kernel(size_t n, const uint32_t* lastnan, uint32_t* smap, const Counters* cnt) {
+    after_previous();
+    release_next();
     if (cnt->nan_flag == 0) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         if (lastnan[i] != 0u) smap[i] = 0u;
@@ -1503,6 +1571,8 @@ __global__ void shadow_fixup_reset_kernel(size_t n, const uint32_t* lastnan, uin
 // the state a pass starts from (a[] = va, b[] = vb); untouched otherwise, as
 // only NaN fragments write it.
 __global__ void nan_cleanup_kernel(size_t n, uint32_t* a, uint32_t va, uint32_t* b, uint32_t vb, const Counters* cnt) {
+    after_previous();
+    release_next();
     if (cnt->nan_flag == 0) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         a[i] = va;
@@ -2085,6 +2155,9 @@ template <bool kTex, bool kFast>
 // 4 blocks per SM (64 registers, a few spilled): 32 warps to hide the
 // record, attribute and shadow-map loads measured faster than 80 registers at 3.
 __global__ void __launch_bounds__(256, 4) shade_kernel(const __grid_constant__ ShadeParams P) {
+    after_previous();
+    release_next();
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) P.cnt_w->stamp[2] = device_clock();
     const int x = (int)(blockIdx.x * 32 + tile_x(threadIdx.x)), r = (int)(blockIdx.y * 8 + tile_y(threadIdx.x));
     const bool pending = shade_one<kTex, kFast>(P, x, r);
     if (P.ao_list && !P.ao_listed) ao_append_tile(P, pending, (uint32_t)r * (uint32_t)P.W + (uint32_t)x);
@@ -2652,6 +2725,8 @@ __global__ void __launch_bounds__(kAoThreads) ao_tables_kernel(const __grid_cons
 
 // The colour scaling of every listed pixel from its stored total.
 __global__ void ao_apply_kernel(const __grid_constant__ AoParams P) {
+    after_previous();
+    release_next();
     const uint32_t n = P.cnt->n_ao;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
         ao_finish(P, P.list[j], P.T[j]);
@@ -2871,77 +2946,80 @@ __global__ void fma_probe_kernel(const float* a, const float* b, const float* c,
 
 int check(cudaError_t e) { return e == cudaSuccess ? 0 : (int)e; }
 
+// k on the stream; with `overlap` as a programmatic launch behind the kernel
+// before it there (k begins with after_previous).
+template <class... K, class... A>
+int launch(bool overlap, void (*k)(K...), dim3 grid, dim3 block, void* stream, const A&... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute a = {};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = overlap ? 1 : 0;
+    return check(cudaLaunchKernelEx(&c, k, K(args)...));
+}
+
 }  // namespace
 
 int launch_setup_main_only(const SetupParams& p, uint32_t* clip_list, void* stream) {
-    if (p.n_tris == 0) return 0;
-    setup_main_kernel<<<(p.n_tris + 127) / 128, 128, 0, (cudaStream_t)stream>>>(p, clip_list);
-    return check(cudaGetLastError());
+    // a clearing block per 2048 keys
+    const unsigned nb = (p.n_tris + 127) / 128 + (unsigned)((p.n_clear + 2047) / 2048);
+    if (nb == 0) return 0;
+    return launch(true, setup_main_kernel, nb, 128, stream, p, clip_list);
 }
 int launch_resolve(int W, int H, const unsigned long long* keys, uint32_t* nanseq, uint32_t* beaten, Counters* cnt,
                    uint32_t* win, float* depth_ao, const uint32_t* first_rec, uint8_t* attr_state,
                    const uint8_t* tri_flags, uint32_t* ao_list, float* linemax, void* stream) {
     if (W <= 0 || H <= 0) return 0;
     const dim3 grd((unsigned)((W + 31) / 32), (unsigned)((H + 7) / 8));
-    resolve_kernel<<<grd, 256, 0, (cudaStream_t)stream>>>(W, H, keys, nanseq, beaten, cnt, win, depth_ao, first_rec,
-                                                         attr_state, tri_flags, ao_list, linemax);
-    return check(cudaGetLastError());
+    return launch(true, resolve_kernel, grd, 256, stream, W, H, keys, nanseq, beaten, cnt, win, depth_ao, first_rec,
+                  attr_state, tri_flags, ao_list, linemax);
 }
-int launch_attr(const SetupParams& p, void* stream) {
-    attr_kernel<<<(unsigned)sm_count() * 8u, 128, 0, (cudaStream_t)stream>>>(p);
-    return check(cudaGetLastError());
+int launch_attr(const SetupParams& p, bool overlap, void* stream) {
+    return launch(overlap, attr_kernel, (unsigned)sm_count() * 8u, 128, stream, p);
 }
-int launch_obj_trans(const PassMats& pm, int n_pass, const float* obj_model, uint32_t n_objects, float* out,
-                     void* stream) {
+int launch_pass_init(const PassMats& pm, int n_pass, const float* obj_model, uint32_t n_objects, float* out,
+                     Counters* cnt, uint32_t rows, void* stream) {
+    static_assert(kNumCounters <= 32, "a bit per counter row");
     const size_t n = (size_t)n_pass * n_objects * 16;
-    if (n == 0) return 0;
-    obj_trans_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(pm, n_pass, obj_model, n_objects, out);
-    return check(cudaGetLastError());
+    return launch(false, pass_init_kernel, (unsigned)std::max<size_t>((n + 255) / 256, 1), 256, stream, pm, n_pass,
+                  obj_model, n_objects, out, cnt, rows);
 }
 int launch_clip(const SetupParams& p, const uint32_t* clip_list, void* stream) {
-    if (p.n_tris == 0) return 0;
     // the list's length is known only on the device: a few blocks per SM stride over it
     const unsigned nb = std::min((p.n_tris + 15) / 16, (unsigned)sm_count() * 4u);
-    clip_kernel<<<nb, 128, 0, (cudaStream_t)stream>>>(p, clip_list);
-    return check(cudaGetLastError());
+    return launch(true, clip_kernel, std::max(nb, 1u), 128, stream, p, clip_list);
 }
 int launch_setup_shadow(const SetupParams& p, void* stream) {
     if (p.n_tris == 0) return 0;
-    unsigned nb = (p.n_tris + 127) / 128;
-    setup_shadow_kernel<<<nb, 128, 0, (cudaStream_t)stream>>>(p);
-    return check(cudaGetLastError());
+    return launch(true, setup_shadow_kernel, (p.n_tris + 127) / 128, 128, stream, p);
 }
 int launch_raster(const RasterParams& p, int n_blocks, void* stream) {
-    raster_kernel<<<n_blocks, kRasterWarps * 32, 0, (cudaStream_t)stream>>>(p);
-    return check(cudaGetLastError());
+    return launch(true, raster_kernel, (unsigned)n_blocks, kRasterWarps * 32, stream, p);
 }
 int launch_shadow_fixup_reset(int W, int H, const uint32_t* lastnan, uint32_t* smap, const Counters* cnt,
                               void* stream) {
     size_t n = (size_t)W * H;
     const unsigned nb = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 8);
-    shadow_fixup_reset_kernel<<<std::max(nb, 1u), 256, 0, (cudaStream_t)stream>>>(n, lastnan, smap, cnt);
-    return check(cudaGetLastError());
+    return launch(true, shadow_fixup_reset_kernel, std::max(nb, 1u), 256, stream, n, lastnan, smap, cnt);
 }
 int launch_nan_cleanup(size_t n, uint32_t* a, uint32_t va, uint32_t* b, uint32_t vb, const Counters* cnt,
                        void* stream) {
     const unsigned nb = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 8);
-    nan_cleanup_kernel<<<std::max(nb, 1u), 256, 0, (cudaStream_t)stream>>>(n, a, va, b, vb, cnt);
-    return check(cudaGetLastError());
+    return launch(true, nan_cleanup_kernel, std::max(nb, 1u), 256, stream, n, a, va, b, vb, cnt);
 }
 // No output asks for the fragment's own attributes.
 bool shade_is_fast(const ShadeParams& p) { return !p.gnor && !p.gfnor && !p.gwpos && !p.guvd && !p.gvcol && !p.dgb; }
-int launch_shade(const ShadeParams& p, void* stream) {
-    const dim3 blk(256), grd((p.W + 31) / 32, (p.H + 7) / 8);
+int launch_shade(const ShadeParams& p, bool overlap, void* stream) {
+    const dim3 grd((p.W + 31) / 32, (p.H + 7) / 8);
     const bool fast = shade_is_fast(p);
-    if (p.mat_tex && fast)
-        shade_kernel<true, true><<<grd, blk, 0, (cudaStream_t)stream>>>(p);
-    else if (p.mat_tex)
-        shade_kernel<true, false><<<grd, blk, 0, (cudaStream_t)stream>>>(p);
-    else if (fast)
-        shade_kernel<false, true><<<grd, blk, 0, (cudaStream_t)stream>>>(p);
-    else
-        shade_kernel<false, false><<<grd, blk, 0, (cudaStream_t)stream>>>(p);
-    return check(cudaGetLastError());
+    return launch(overlap,
+                  p.mat_tex ? (fast ? shade_kernel<true, true> : shade_kernel<true, false>)
+                            : (fast ? shade_kernel<false, true> : shade_kernel<false, false>),
+                  grd, 256, stream, p);
 }
 int launch_tri_flags(const float4* pos, uint32_t n, uint8_t* flags, const int32_t* mat, const uint32_t* obj_first,
                      const uint32_t* blk_obj, const int32_t* obj_matbase, uint32_t n_objects, const pr_material* mats,
@@ -3023,8 +3101,8 @@ PR_DEV uint8_t resize_div(int32_t acc, int32_t sum) {
 // imageutil.Resize's two passes for one output pixel: the horizontal pass
 // (into the reference's transposed uint8 temporary) for every input row the
 // vertical taps reach, then the vertical pass over those values.
-__global__ void msaa_resize_kernel(const uchar4* __restrict__ in, int in_w, int in_h, uchar4* __restrict__ out, int w,
-                                   int h) {
+__global__ void msaa_resize_kernel(const uchar4* in, int in_w, int in_h, uchar4* out, int w, int h) {
+    after_previous();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= w || y >= h) return;
@@ -3059,8 +3137,7 @@ __global__ void msaa_resize_kernel(const uchar4* __restrict__ in, int in_w, int 
 int launch_msaa_resize(const uchar4* in, int in_w, int in_h, uchar4* out, int w, int h, void* stream) {
     if (w <= 0 || h <= 0 || in_w < w || in_h < h || in_w > w * kMaxMsaa || in_h > h * kMaxMsaa) return -1;
     const dim3 block(32, 8), grid((unsigned)((w + 31) / 32), (unsigned)((h + 7) / 8));
-    msaa_resize_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(in, in_w, in_h, out, w, h);
-    return check(cudaGetLastError());
+    return launch(true, msaa_resize_kernel, grid, block, stream, in, in_w, in_h, out, w, h);
 }
 
 size_t ao_tables_bytes() { return sizeof(AoTables); }
@@ -3083,8 +3160,7 @@ int launch_ao_T(const AoParams& p, void* stream) {
     return check(cudaGetLastError());
 }
 int launch_ao_apply(const AoParams& p, int n_blocks, void* stream) {
-    ao_apply_kernel<<<n_blocks, 256, 0, (cudaStream_t)stream>>>(p);
-    return check(cudaGetLastError());
+    return launch(false, ao_apply_kernel, (unsigned)n_blocks, 256, stream, p);
 }
 int set_ao_tables(const float* cosv, const float* sinv, int n, void* stream) {
     float d[2][8] = {};
@@ -3184,6 +3260,7 @@ __global__ void __launch_bounds__(256) noalloc_init_kernel(const float* depth, u
                                                            Counters* cnt, uint32_t* obj_first, float* obj_trans,
                                                            uint32_t* blk_obj, uint32_t n_tris,
                                                            const __grid_constant__ NaObjects O) {
+    release_next();  // launched in full order itself
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         const float d = depth[i];
@@ -3209,6 +3286,7 @@ __global__ void __launch_bounds__(256) noalloc_init_kernel(const float* depth, u
 // fragment replaced stays as it was, as in the reference's map.
 // After a task overflow the map stays as it was.
 __global__ void decode_changed_kernel(const uint32_t* keys, float* depth, size_t n, const Counters* cnt) {
+    after_previous();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || cnt->overflow) return;
     const float d = depth[i];
@@ -3350,9 +3428,8 @@ extern "C" int pr_depth_map_noalloc(const pr_depth_map_desc* d) {
     rp.take = &cnt->take[1];
     if (!rc) rc = launch_raster(rp, sm_count() * 8, st);
     if (rc) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: kernel launch failed");
-    decode_changed_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(keys, d->depth, n, cnt);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: kernel launch failed");
+    rc = launch(true, decode_changed_kernel, (unsigned)((n + 255) / 256), 256, st, keys, d->depth, n, cnt);
+    if (rc) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: kernel launch failed");
     Counters h{};
     e = cudaMemcpyAsync(&h, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);

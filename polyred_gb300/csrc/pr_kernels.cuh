@@ -70,7 +70,7 @@ struct alignas(16) Counters {
     uint32_t take_attr;   // work-queue head of the attribute records
     uint32_t n_big;       // block tasks of large records (raster_block)
     uint32_t n_big_px;    // ... counted as tasks of 2^task_shift pixels
-    uint32_t pad[2];
+    unsigned long long stamp[3];  // device clock (ns) at the start of: the frame, its main raster, its shading
 };
 
 struct LightK {
@@ -120,6 +120,8 @@ struct SetupParams {
     uint32_t* clip_list;         // batched main setup: this view's clip list
     const uint8_t* tri_flags;    // [n_tris] Triangle.IsValid, or null (computed inline)
     Counters* cnt_rec;           // clip: the main pass's counters (records, clip list); null: cnt
+    unsigned long long* clear;   // main setup: the depth keys its blocks past the triangles' set to 0
+    size_t n_clear;
 };
 
 enum RasterMode { kMain = 0, kMainFixup = 1, kShadow = 2, kShadowFixup = 3 };
@@ -138,6 +140,7 @@ struct RasterParams {
     uint32_t* lastnan;         // shadow: 1 + max seq of NaN-depth fragments, 0 if none
     uint32_t task_shift = kTaskShift;  // as the setup that wrote the tasks
     uint32_t* take = nullptr;          // zeroed work-queue head (warps take grab tasks at a time; unused by batches)
+    int after_clip = 0;                // 1: launched behind clip_kernel, whose tasks are another list
     uint32_t grab = 0;                 // tasks per queue grab, a multiple of 32; 0: from the task count
                                        // (64 below 256 tasks per warp of the grid, else 128)
     // a second task list drained after the first (its own counters and
@@ -247,14 +250,15 @@ struct DiffParamsK {
 namespace prk {
 int launch_setup_main_only(const SetupParams& p, uint32_t* clip_list, void* stream);
 int launch_clip(const SetupParams& p, const uint32_t* clip_list, void* stream);
-// Proj·View·Model of every object for n_pass passes: out[pass][o][16] from
-// the passes' Proj·View (pv[pass]) in Mat4.MulM's order.
+// The counter rows of the bit set `rows` to zero, and Proj·View·Model of every
+// object for n_pass passes: out[pass][o][16] from the passes' Proj·View
+// (pv[pass]) in Mat4.MulM's order.
 constexpr int kMaxPasses = kMaxLights + 1;
 struct PassMats {
     float pv[kMaxPasses][16];
 };
-int launch_obj_trans(const PassMats& pm, int n_pass, const float* obj_model, uint32_t n_objects, float* out,
-                     void* stream);
+int launch_pass_init(const PassMats& pm, int n_pass, const float* obj_model, uint32_t n_objects, float* out,
+                     Counters* cnt, uint32_t rows, void* stream);
 // Resolve that also marks the winning records whose attributes were deferred
 // (attr_state kAttrDeferred -> kAttrWanted), puts the NaN bookkeeping
 // (nanseq, beaten) back to kNone / 0 after a frame that used it, and, with
@@ -265,7 +269,8 @@ int launch_resolve(int W, int H, const unsigned long long* keys, uint32_t* nanse
                    uint32_t* win, float* depth_ao, const uint32_t* first_rec, uint8_t* attr_state,
                    const uint8_t* tri_flags, uint32_t* ao_list, float* linemax, void* stream);
 // The attribute records of the records resolve marked (P: the main view's setup parameters).
-int launch_attr(const SetupParams& p, void* stream);
+// overlap: the operation before it on the stream is a kernel of the frame.
+int launch_attr(const SetupParams& p, bool overlap, void* stream);
 int launch_setup_shadow(const SetupParams& p, void* stream);
 int launch_raster(const RasterParams& p, int n_blocks, void* stream);
 int launch_shadow_fixup_reset(int W, int H, const uint32_t* lastnan, uint32_t* smap, const Counters* cnt,
@@ -273,7 +278,7 @@ int launch_shadow_fixup_reset(int W, int H, const uint32_t* lastnan, uint32_t* s
 // After a pass that saw a NaN fragment (cnt->nan_flag): a[0..n) = va and, if b, b[0..n) = vb.
 int launch_nan_cleanup(size_t n, uint32_t* a, uint32_t va, uint32_t* b, uint32_t vb, const Counters* cnt,
                        void* stream);
-int launch_shade(const ShadeParams& p, void* stream);
+int launch_shade(const ShadeParams& p, bool overlap, void* stream);
 bool shade_is_fast(const ShadeParams& p);  // colours and depths alone: certified lighting
 // AO split so that its march overlaps shading: the list (made by resolve),
 // the march writing p.T (after resolve), and the colour scaling and gamma
