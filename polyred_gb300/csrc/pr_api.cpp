@@ -144,12 +144,13 @@ struct SceneBufs {
     DevBuf<float2> uv;
     DevBuf<uchar4> col;
     DevBuf<int32_t> mat;
-    DevBuf<uint32_t> obj_first;
+    DevBuf<uint8_t> d_tables;   // the small tables, one copy; in it:
+    float *obj_model = nullptr, *obj_normal = nullptr;
+    pr_material* dmats = nullptr;
+    uint32_t* obj_first = nullptr;
+    int32_t* obj_matbase = nullptr;
+    uint32_t* blk_obj = nullptr;  // object of the first triangle of each 128-triangle block
     DevBuf<uint8_t> tri_flags;  // Triangle.IsValid per input triangle
-    DevBuf<float> obj_model, obj_normal;
-    DevBuf<int32_t> obj_matbase;
-    DevBuf<pr_material> dmats;
-    DevBuf<uint32_t> blk_obj;              // object of the first triangle of each 128-triangle block
     DevBuf<uint32_t> texels;               // image textures: every mipmap level, packed RGBA8
     DevBuf<prt::TexDesc> tex;
     DevBuf<int32_t> mat_tex;               // [n_materials] texture of each material, -1: uniform
@@ -157,18 +158,18 @@ struct SceneBufs {
     bool has_ao = false;                   // a material has ambient occlusion
     HostBuf tables;                        // page-locked staging of the small tables (submitted uploads)
     cudaEvent_t ev_uploaded = nullptr;     // the upload into these buffers has landed
-    cudaEvent_t ev_released = nullptr;     // the last frame that read them is past shading
-    cudaEvent_t ev_released_ao = nullptr;  // ... and past the frame's AO stream work (stream 3)
+    // of the last frame that read them and was not waited for by the host:
+    cudaEvent_t ev_geometry = nullptr;  // past setup, clipping, shadow passes and attributes: only shading is left
+    cudaEvent_t ev_released = nullptr;  // past shading
     void release() {
         pos.release(); nor.release(); uv.release(); col.release(); mat.release();
-        obj_first.release(); tri_flags.release(); obj_model.release(); obj_normal.release();
-        obj_matbase.release(); dmats.release(); blk_obj.release(); tables.release();
+        tri_flags.release(); d_tables.release(); tables.release();
         texels.release(); tex.release(); mat_tex.release();
         has_tex = has_ao = false;
         if (ev_uploaded) cudaEventDestroy(ev_uploaded);
         if (ev_released) cudaEventDestroy(ev_released);
-        if (ev_released_ao) cudaEventDestroy(ev_released_ao);
-        ev_uploaded = ev_released = ev_released_ao = nullptr;
+        if (ev_geometry) cudaEventDestroy(ev_geometry);
+        ev_uploaded = ev_released = ev_geometry = nullptr;
     }
 };
 
@@ -299,74 +300,64 @@ int upload(DevBuf<T>& b, const void* src, size_t n, bool dev_src, cudaStream_t s
 }
 
 // Copy a scene into b on stream st: the triangle arrays, the per-object
-// Model and Normal = Model.Inv().T() (render/raster.go:242-243), the
-// material table, and the Triangle.IsValid flags. staged: the small host
+// Model and Normal = Model.Inv().T() (render/raster.go:242-243) and the
+// material table; scene_flags follows on the frames' stream. staged: the small
 // tables go through b's page-locked staging, so nothing waits for the copy;
-// otherwise the caller synchronises st before they go out of scope.
+// otherwise from pageable memory (copied when cudaMemcpyAsync returns). They
+// are one copy: each of six kept a submitted scene's bulk waiting, as did a
+// flags kernel on the uploading stream behind the frame in flight (1M triangles
+// anew each 1080p frame: 766 -> 711 us a frame, 655 of them the bare copies).
 int scene_fill(SceneBufs& b, const pr_scene_desc* s, cudaStream_t st, bool staged) {
     int rc;
     const bool dev = (s->flags & PR_SCENE_DEVICE_PTRS) != 0;
     const uint32_t n = s->n_tris, no = s->n_objects, nm = s->n_materials;
-    std::vector<uint32_t> first(no + 1);
-    std::vector<float> model((size_t)no * 16), normal((size_t)no * 16);
-    std::vector<int32_t> mb(no);
+    const uint32_t nblk = std::max<uint32_t>((n + 127) / 128, 1);
+    auto al = [](size_t v) { return (v + 15) & ~(size_t)15; };
+    const size_t o_model = 0, o_normal = o_model + (size_t)no * 64, o_mats = o_normal + (size_t)no * 64,
+                 o_first = al(o_mats + (size_t)nm * sizeof(pr_material)), o_mb = o_first + ((size_t)no + 1) * 4,
+                 o_blk = o_mb + (size_t)no * 4, total = o_blk + (size_t)nblk * 4;
+    std::vector<uint8_t> pageable;
+    if (staged) {
+        if ((rc = b.tables.ensure(total))) return rc;
+    } else {
+        pageable.resize(total);
+    }
+    uint8_t* h = staged ? b.tables.p : pageable.data();
+    uint32_t* first = (uint32_t*)(h + o_first);
     for (uint32_t o = 0; o < no; o++) {
         first[o] = s->objects[o].first_tri;
         M4 m = loadm(s->objects[o].model), mi;
         if (!prh::inv(m, &mi)) return fail(PR_ERR_SINGULAR, "object %u: model matrix is singular", o);
         M4 nm4 = prh::transpose(mi);
-        std::memcpy(&model[(size_t)o * 16], m.m, 64);
-        std::memcpy(&normal[(size_t)o * 16], nm4.m, 64);
-        mb[o] = s->objects[o].mat_base;
+        std::memcpy(h + o_model + (size_t)o * 64, m.m, 64);
+        std::memcpy(h + o_normal + (size_t)o * 64, nm4.m, 64);
+        ((int32_t*)(h + o_mb))[o] = s->objects[o].mat_base;
     }
     first[no] = n;
     // object of each 128-triangle block's first triangle (the last object starting at or before it)
-    const uint32_t nblk = (n + 127) / 128;
-    std::vector<uint32_t> blk(std::max<uint32_t>(nblk, 1), 0u);
+    uint32_t* blk = (uint32_t*)(h + o_blk);
     for (uint32_t k = 0, o = 0; k < nblk; k++) {
         while (o + 1 < no && first[o + 1] <= k * 128u) o++;
         blk[k] = o;
     }
+    if (nm) std::memcpy(h + o_mats, s->materials, (size_t)nm * sizeof(pr_material));
     if ((rc = upload(b.pos, s->pos, (size_t)n * 3, dev, st))) return rc;
     if ((rc = upload(b.nor, s->nor, (size_t)n * 3, dev, st))) return rc;
     if ((rc = upload(b.uv, s->uv, (size_t)n * 3, dev, st))) return rc;
     if ((rc = upload(b.col, s->col, (size_t)n * 3, dev, st))) return rc;
     if ((rc = upload(b.mat, s->mat_id, (size_t)n, dev, st))) return rc;
-    const void* t_first = first.data();
-    const void* t_model = model.data();
-    const void* t_normal = normal.data();
-    const void* t_mb = mb.data();
-    const void* t_mats = s->materials;
-    const void* t_blk = blk.data();
-    if (staged) {
-        auto al = [](size_t v) { return (v + 15) & ~(size_t)15; };
-        const size_t o_first = 0, o_model = al(o_first + first.size() * 4), o_normal = o_model + model.size() * 4,
-                     o_mb = o_normal + normal.size() * 4, o_mats = al(o_mb + mb.size() * 4),
-                     o_blk = al(o_mats + (size_t)nm * sizeof(pr_material)), total = o_blk + blk.size() * 4;
-        if ((rc = b.tables.ensure(total))) return rc;
-        uint8_t* h = b.tables.p;
-        std::memcpy(h + o_first, first.data(), first.size() * 4);
-        std::memcpy(h + o_model, model.data(), model.size() * 4);
-        std::memcpy(h + o_normal, normal.data(), normal.size() * 4);
-        std::memcpy(h + o_mb, mb.data(), mb.size() * 4);
-        if (nm) std::memcpy(h + o_mats, s->materials, (size_t)nm * sizeof(pr_material));
-        std::memcpy(h + o_blk, blk.data(), blk.size() * 4);
-        t_blk = h + o_blk;
-        t_first = h + o_first;
-        t_model = h + o_model;
-        t_normal = h + o_normal;
-        t_mb = h + o_mb;
-        t_mats = h + o_mats;
-    }
-    if ((rc = upload(b.obj_first, t_first, first.size(), false, st))) return rc;
-    if ((rc = upload(b.obj_model, t_model, model.size(), false, st))) return rc;
-    if ((rc = upload(b.obj_normal, t_normal, normal.size(), false, st))) return rc;
-    if ((rc = upload(b.obj_matbase, t_mb, mb.size(), false, st))) return rc;
-    if ((rc = upload(b.dmats, t_mats, nm, false, st))) return rc;
-    if ((rc = upload(b.blk_obj, t_blk, blk.size(), false, st))) return rc;
+    // From here on also what shading reads: materials and images. The triangles
+    // above, the bulk of an upload, need not wait for the frame's last phase.
+    if (staged) CUDA_TRY(cudaStreamWaitEvent(st, b.ev_released, 0));
+    if ((rc = upload(b.d_tables, h, total, false, st))) return rc;
+    uint8_t* d = b.d_tables.p;
+    b.obj_model = (float*)(d + o_model);
+    b.obj_normal = (float*)(d + o_normal);
+    b.dmats = (pr_material*)(d + o_mats);
+    b.obj_first = (uint32_t*)(d + o_first);
+    b.obj_matbase = (int32_t*)(d + o_mb);
+    b.blk_obj = (uint32_t*)(d + o_blk);
     if ((rc = b.tri_flags.ensure(std::max<uint32_t>(n, 1)))) return rc;
-    KTRY(prk::launch_tri_flags(b.pos.p, n, b.tri_flags.p, b.mat.p, b.obj_first.p, b.blk_obj.p, b.obj_matbase.p, no,
-                               b.dmats.p, nm, st));
     // image textures: NewTexture's levels built here, once per upload
     b.has_tex = false;
     if (scene_has_images(s)) {
@@ -399,6 +390,13 @@ int scene_fill(SceneBufs& b, const pr_scene_desc* s, cudaStream_t st, bool stage
     b.has_ao = false;
     for (uint32_t m = 0; m < nm; m++) b.has_ao |= (s->materials[m].flags & PR_MAT_AO) != 0;
     b.n_tris = n;
+    return PR_OK;
+}
+
+// The Triangle.IsValid flags of a filled scene, on the stream whose frames read them.
+int scene_flags(SceneBufs& b, cudaStream_t st) {
+    KTRY(prk::launch_tri_flags(b.pos.p, b.n_tris, b.tri_flags.p, b.mat.p, b.obj_first, b.blk_obj, b.obj_matbase,
+                               (uint32_t)b.objects.size(), b.dmats, (uint32_t)b.materials.size(), st));
     return PR_OK;
 }
 
@@ -483,12 +481,12 @@ void fill_scene_ptrs(Ctx* c, prk::SetupParams& p) {
     p.uv = c->sb.uv.p;
     p.col = c->sb.col.p;
     p.mat = c->sb.mat.p;
-    p.obj_first = c->sb.obj_first.p;
-    p.obj_model = c->sb.obj_model.p;
-    p.obj_normal = c->sb.obj_normal.p;
-    p.obj_matbase = c->sb.obj_matbase.p;
+    p.obj_first = c->sb.obj_first;
+    p.obj_model = c->sb.obj_model;
+    p.obj_normal = c->sb.obj_normal;
+    p.obj_matbase = c->sb.obj_matbase;
     p.tri_flags = c->sb.tri_flags.p;
-    p.blk_obj = c->sb.blk_obj.p;
+    p.blk_obj = c->sb.blk_obj;
     p.n_tris = c->sb.n_tris;
     p.n_objects = (uint32_t)c->sb.objects.size();
 }
@@ -571,7 +569,7 @@ void fill_shade_frame(const Ctx* c, const pr_frame_desc* f, const M4& s2w, int S
     sp.W = f->width;
     sp.H = f->height;
     sp.flags = f->flags;
-    sp.mats = c->sb.dmats.p;
+    sp.mats = c->sb.dmats;
     sp.n_mats = (uint32_t)c->sb.materials.size();
     sp.n_lights = (int)f->n_lights;
     sp.n_ambient = (int)f->n_ambient;
@@ -756,7 +754,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         {
             prk::PassMats pm;
             std::memcpy(pm.pv[0], pv.m, 64);
-            KTRY(prk::launch_pass_init(pm, 1, c->sb.obj_model.p, n_obj, c->obj_trans.p, dcnt, ~light_rows, st));
+            KTRY(prk::launch_pass_init(pm, 1, c->sb.obj_model, n_obj, c->obj_trans.p, dcnt, ~light_rows, st));
             launches += 1;
         }
         // ---- shadow passes (render/raster.go:176-184), on their own stream:
@@ -813,7 +811,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
                 const M4 lpv = prh::mulm(loadm(f->lights[l].shadow_proj), loadm(f->lights[l].shadow_view));
                 std::memcpy(pm.pv[l], lpv.m, 64);
             }
-            KTRY(prk::launch_pass_init(pm, NL, c->sb.obj_model.p, n_obj, c->obj_trans.p + (size_t)n_obj * 16, dcnt,
+            KTRY(prk::launch_pass_init(pm, NL, c->sb.obj_model, n_obj, c->obj_trans.p + (size_t)n_obj * 16, dcnt,
                                        light_rows, ss));
             launches += 1;
             for (int l = 0; l < NL; l++)
@@ -924,7 +922,6 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             CUDA_TRY(cudaEventRecord(c->ev_resolved, st));
             CUDA_TRY(cudaStreamWaitEvent(sc, c->ev_resolved, 0));
             CUDA_TRY(cudaEventRecord(c->ev_ao0, sc));
-            CUDA_TRY(cudaEventRecord(c->sb.ev_released_ao, sc));  // stream 3 reads no scene buffer
             ap.W = W;
             ap.H = H;
             ap.gamma_on = (f->flags & PR_FRAME_GAMMA) ? 1 : 0;
@@ -998,8 +995,10 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         sp.ao_listed = 1;  // listed by resolve
         if (casts) CUDA_TRY(cudaStreamWaitEvent(st, c->ev[1], 0));          // the shadow maps are complete
         if (c->submitted) CUDA_TRY(cudaStreamWaitEvent(st, c->ev_d2h, 0));  // a submitted frame's outputs left the staging
-        KTRY(prk::launch_shade(sp, !casts && !c->submitted, st));
+        if (!sync) CUDA_TRY(cudaEventRecord(c->sb.ev_geometry, st));
+        KTRY(prk::launch_shade(sp, !casts && !c->submitted && sync, st));
         launches += 1;
+        if (!sync) CUDA_TRY(cudaEventRecord(c->sb.ev_released, st));
         if (sp.rgba) {
             if (with_ao) {
                 // AmbientOcclusionShade's colour scaling and gamma of the listed
@@ -1017,7 +1016,6 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             }
         }
         CUDA_TRY(cudaEventRecord(c->ev[2], st));
-        CUDA_TRY(cudaEventRecord(c->sb.ev_released, st));  // the scene buffers are read no more
         CUDA_TRY(cudaMemcpyAsync(c->h_cnt, dcnt, sizeof(prk::Counters) * prk::kNumCounters, cudaMemcpyDeviceToHost, st));
         if (!sync) {
             c->stats.n_kernel_launches = launches;
@@ -1130,8 +1128,8 @@ int pr_create(int device, void** out_ctx) {
         cudaEventCreateWithFlags(&c->sb.ev_released, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->sb_back.ev_uploaded, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->sb_back.ev_released, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->sb.ev_released_ao, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->sb_back.ev_released_ao, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->sb.ev_geometry, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->sb_back.ev_geometry, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_resolved, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreate(&c->ev_ao0) != cudaSuccess || cudaEventCreate(&c->ev_ao) != cudaSuccess) {
         pr_destroy(c);
@@ -1211,7 +1209,7 @@ int pr_scene_upload(void* ctx, const pr_scene_desc* s) {
     CUDA_TRY(cudaStreamSynchronize(c->stream_d));
     clear_stale_error();
     c->has_scene = false;  // until the new scene is complete (a failed upload leaves none)
-    if ((rc = scene_fill(c->sb, s, c->stream, false))) return rc;
+    if ((rc = scene_fill(c->sb, s, c->stream, false)) || (rc = scene_flags(c->sb, c->stream))) return rc;
     CUDA_TRY(cudaStreamSynchronize(c->stream));  // host tables go out of scope
     c->has_scene = true;
     c->smap_valid = false;
@@ -1229,14 +1227,16 @@ int pr_frame_submit(void* ctx, const pr_scene_desc* scene, const pr_frame_desc* 
     SceneBufs& b = c->sb_back;
     clear_stale_error();
     CUDA_TRY(cudaEventSynchronize(b.ev_uploaded));                 // its staging is free again
-    CUDA_TRY(cudaStreamWaitEvent(c->stream_u, b.ev_released, 0));  // no frame reads it any more
-    CUDA_TRY(cudaStreamWaitEvent(c->stream_u, b.ev_released_ao, 0));
+    // no frame reads its triangles and objects any more (scene_fill waits for
+    // shading before it touches the materials)
+    CUDA_TRY(cudaStreamWaitEvent(c->stream_u, b.ev_geometry, 0));
     if ((rc = scene_fill(b, scene, c->stream_u, true))) return rc;
     CUDA_TRY(cudaEventRecord(b.ev_uploaded, c->stream_u));
     std::swap(c->sb, c->sb_back);
     c->has_scene = true;
     c->smap_valid = false;  // as pr_scene_upload
     CUDA_TRY(cudaStreamWaitEvent(c->stream, c->sb.ev_uploaded, 0));
+    if ((rc = scene_flags(c->sb, c->stream))) return rc;
     return render_impl(c, frame, out, false, nullptr, true);
 }
 
@@ -1463,14 +1463,14 @@ int diff_setup(Ctx* c, const pr_frame_desc* f, const pr_diff_params* prm, prk::D
     K.H = f->height;
     K.vcol = vcol;
     K.vnor = (prm && prm->vertex_normal) ? (const float4*)prm->vertex_normal : c->sb.nor.p;
-    K.obj_first = c->sb.obj_first.p;
+    K.obj_first = c->sb.obj_first;
     K.n_objects = (uint32_t)c->sb.objects.size();
-    K.obj_normal = c->sb.obj_normal.p;
+    K.obj_normal = c->sb.obj_normal;
     K.n_mats = (int)nm;
     K.kd = c->d_kd.p;
     K.ks = c->d_ks.p;
     K.shin = c->d_shin.p;
-    K.mats = c->sb.dmats.p;
+    K.mats = c->sb.dmats;
     K.n_lights = (int)f->n_lights;
     K.n_ambient = (int)f->n_ambient;
     for (uint32_t l = 0; l < f->n_lights; l++) {
