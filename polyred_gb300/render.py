@@ -12,6 +12,7 @@ Usage::
     img = r.Render()          # (H, W, 4) uint8, top-down rows like *image.RGBA
     ids, depth = r.tri_id(), r.depth()
 """
+import collections
 import ctypes as C
 import weakref
 
@@ -269,6 +270,43 @@ def host_array(shape, dtype):
     return a
 
 
+class _Spare:
+    """Host memory of one renderer's images, used again once the program has
+    dropped them. A fresh 1.6 MB array is fresh pages, and the faults of three
+    took longer than a frame of 800x500 (Render(): 1300 -> 230 us). An array is
+    handed out over a buffer of its own; when its last view goes, the buffer
+    comes back, at most `keep` of a size stay, and they go with the renderer.
+    Plain memory: it survives a fork, as the arrays before did. deque's append
+    and pop are atomic, and the callback that returns a buffer may run on any
+    thread, inside a collection, so there is no lock to hold."""
+
+    def __init__(self, keep):
+        self.keep = keep
+        self.free = {}
+
+    def _give(self, n, buf):
+        q = self.free.get(n)
+        if q is not None and len(q) < self.keep:
+            q.append(buf)
+
+    def only(self, sizes):
+        """Forget the sizes that the next frame does not ask for."""
+        self.free = {n: self.free.get(n) or collections.deque() for n in sizes}
+
+    def array(self, shape, dtype):
+        """An array that the caller overwrites whole."""
+        n = int(np.prod(shape)) * np.dtype(dtype).itemsize
+        if n == 0:
+            return np.zeros(shape, dtype)
+        try:
+            buf = self.free[n].pop()
+        except (KeyError, IndexError):
+            buf = np.empty(n, np.uint8)
+        lease = (C.c_uint8 * n).from_buffer(buf)
+        weakref.finalize(lease, self._give, n, buf).atexit = False
+        return np.frombuffer(lease, dtype).reshape(shape)
+
+
 class Outputs:
     """Host arrays a frame writes (pr_outputs); pinned=True places them in
     page-locked memory (pr_host_alloc), which the device writes at full link
@@ -278,22 +316,31 @@ class Outputs:
               "face_nor": (4, F32), "world_pos": (4, F32), "uvd": (4, F32), "vcol": (4, np.uint8),
               "mat_id": (1, np.int32)}
 
-    def __init__(self, width, height, want=("rgba",), n_shadow=0, shadow_size=None, pinned=False, msaa=1):
+    def __init__(self, width, height, want=("rgba",), n_shadow=0, shadow_size=None, pinned=False, msaa=1,
+                 spare=None):
         """rgba is (height, width, 4); with msaa > 1 every other field has
-        the framebuffer's msaa*height x msaa*width pixels."""
+        the framebuffer's msaa*height x msaa*width pixels. spare: the _Spare
+        that the arrays come from (a frame writes every element of them; the
+        single plane that stands for no shadow map stays zero)."""
         self.arrays = {}
         o = _abi.pr_outputs()
         o.size = C.sizeof(_abi.pr_outputs)
         o.flags = 0
         alloc = host_array if pinned else np.zeros
+        form = {}
         for name in want:
             if name == "shadow_maps":
                 sw, sh = shadow_size
-                a = alloc((max(n_shadow, 1), sh, sw), F32)
+                form[name] = (max(n_shadow, 1), sh, sw), F32
             else:
                 k, dt = self.FIELDS[name]
                 h, w = (height, width) if name == "rgba" else (height * msaa, width * msaa)
-                a = alloc((h, w, k) if k > 1 else (h, w), dt)
+                form[name] = (h, w, k) if k > 1 else (h, w), dt
+        if spare is not None:
+            spare.only({int(np.prod(shape)) * np.dtype(dt).itemsize for shape, dt in form.values()})
+        for name, (shape, dt) in form.items():
+            written = name != "shadow_maps" or n_shadow > 0
+            a = (spare.array if spare is not None and written else alloc)(shape, dt)
             self.arrays[name] = a
             setattr(o, name, a.ctypes.data)
         self.desc = o
@@ -310,6 +357,7 @@ class Renderer:
                           device=None, shadow_size=None, directional_shadows=False,
                           outputs=("rgba", "tri_id", "depth"))
         self._own_device = None
+        self._spare = _Spare(len(Outputs.FIELDS) + 1)
         self._lib = native.load()
         self._apply(opts)
         self._last = None
@@ -380,7 +428,8 @@ class Renderer:
         src, _ = o["scene"].lights()
         m = o["msaa"]
         sw, sh = o["shadow_size"] or (o["width"] * m, o["height"] * m)
-        out = Outputs(o["width"], o["height"], o["outputs"], n_shadow=len(src), shadow_size=(sw, sh), msaa=m)
+        out = Outputs(o["width"], o["height"], o["outputs"], n_shadow=len(src), shadow_size=(sw, sh), msaa=m,
+                      spare=self._spare)
         native.check(self._lib.pr_render(self.device.handle, C.byref(fd.desc), C.byref(out.desc)))
         st = _abi.pr_stats()
         st.size = C.sizeof(_abi.pr_stats)
