@@ -232,6 +232,7 @@ struct Ctx {
     bool ao_marched = false;  // the last frame ran the AO march (ev_ao0, ev_ao hold it)
     DevBuf<float> ao_T;
     DevBuf<float> linemax;  // [4][H][W], AO's line maxima
+    DevBuf<uint8_t> gamma;   // GammaCorrection's table (prh::gamma_table)
     DevBuf<uint8_t> ao_tab;  // AO's tap tables for frames of width ao_tab_w and rounding ao_tab_ulp
     int ao_tab_w = 0;
     float ao_tab_ulp = 0.0f;
@@ -629,7 +630,7 @@ void fill_shade_frame(const Ctx* c, const pr_frame_desc* f, const M4& s2w, int S
     }
     sp.SW = SW;
     sp.SH = SH;
-    prh::gamma_table(sp.gamma);
+    sp.gamma = c->gamma.p;
 }
 
 // Matrices of a frame (render/raster.go:232-246, 281-295).
@@ -1006,7 +1007,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
                 CUDA_TRY(cudaStreamWaitEvent(st, c->ev_ao, 0));
                 ap.rgba = sp.rgba;
                 ap.dgb = dh ? dh->dgb : nullptr;
-                std::memcpy(ap.gamma, sp.gamma, 256);
+                ap.gamma = sp.gamma;
                 KTRY(prk::launch_ao_apply(ap, c->n_sms * 4, st));
                 launches += 1;
             }
@@ -1149,6 +1150,16 @@ int pr_create(int device, void** out_ctx) {
             return fail(PR_ERR_CUDA, "AO table upload: %s", cudaGetErrorString((cudaError_t)e));
         }
     }
+    {
+        uint8_t table[256];
+        prh::gamma_table(table);
+        if ((rc = upload(c->gamma, table, 256, false, c->stream))) { pr_destroy(c); return rc; }
+        cudaError_t e = cudaStreamSynchronize(c->stream);
+        if (e != cudaSuccess) {
+            pr_destroy(c);
+            return fail(PR_ERR_CUDA, "gamma table upload: %s", cudaGetErrorString(e));
+        }
+    }
     *out_ctx = c;
     return PR_OK;
 }
@@ -1179,7 +1190,7 @@ int pr_destroy(void* ctx) {
     if (c->ev_resolved) cudaEventDestroy(c->ev_resolved);
     if (c->ev_ao0) cudaEventDestroy(c->ev_ao0);
     if (c->ev_ao) cudaEventDestroy(c->ev_ao);
-    c->ao_T.release(); c->linemax.release(); c->ao_tab.release();
+    c->ao_T.release(); c->linemax.release(); c->ao_tab.release(); c->gamma.release();
     if (c->stream_c) {
         cudaStreamSynchronize(c->stream_c);
         cudaStreamDestroy(c->stream_c);
@@ -1902,7 +1913,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
         ap.linemax = b->linemax.p + (any_ao ? 4 * o : 0);
         ap.cnt = mp.cnt;
         ap.rgba = sp.rgba;
-        std::memcpy(ap.gamma, sp.gamma, 256);
+        ap.gamma = sp.gamma;
     }
     p.nb_m = p.blk.back();
     const size_t orr = p.blk.size();

@@ -174,7 +174,7 @@ struct ShadeParams {
     float shadow_vp[16];        // ViewportMatrix(SW, SH)
     int SW, SH;
     const uint32_t* smaps;      // [n_lights][SH*SW] orderable keys
-    uint8_t gamma[256];
+    const uint8_t* gamma;       // [256]; in global memory: lanes' different entries of a parameter array are read one by one
     // outputs (device pointers, may be null)
     uchar4* rgba;
     uint32_t* tri_id;
@@ -204,7 +204,7 @@ struct AoParams {
     const uint32_t* list;
     const Counters* cnt;
     uchar4* rgba;
-    uint8_t gamma[256];
+    const uint8_t* gamma;  // [256]
     int8_t dir_fast[8];  // 1: the tap offset table is exact for this frame size
     int8_t dir_tiny[8];  // 1 / 2: the x / y component lies in (-1/99, 0)
     float ao_half_ulp;   // half an ulp of float32 at max(W, H) + 100
