@@ -2797,7 +2797,7 @@ PR_DEV void ao_finish(const AoParams& P, uint32_t i, float T) {
 // 4 blocks per SM (64 registers). The tap tables come from the context
 // (ao_tables_kernel): building them cost each block of 256 pixels 7% of its
 // instructions. Bound by issue (71% active): 713k pixels at 1920x1080 take
-// 218 us and 171 M warp instructions; every tap compared by itself, eight to
+// 206 us and 160 M warp instructions; every tap compared by itself, eight to
 // a unit, took 286 us and 227 M.
 __global__ void __launch_bounds__(kAoThreads, 4) ao_kernel(const __grid_constant__ AoParams P) {
     __shared__ AoTables S;
