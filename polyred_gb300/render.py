@@ -448,6 +448,7 @@ class Renderer:
         return None if self._last is None else self._last.get("depth")
 
     def close(self):
+        self._spare.only(())
         if self._own_device is not None:
             self._own_device.close()
             self._own_device = None

@@ -27,6 +27,8 @@ def test_in_use_is_not_shared(shape):
     assert len(s.free[n]) == 3  # bounded
     s.only({n + 4})
     assert n not in s.free
+    s.only(())  # what Renderer.close does
+    assert not s.free
 
 
 def test_other_sizes_and_a_dropped_pool():
