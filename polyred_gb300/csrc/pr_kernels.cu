@@ -185,11 +185,13 @@ static __device__ __noinline__ PixBox pixel_box_any(V4 a, V4 b, V4 c, float sabc
     return {(uint32_t)((x1 - x0 + 1) * (y1 - y0 + 1)), (uint32_t)x0 | ((uint32_t)x1 << 16), (uint32_t)y0 | ((uint32_t)y1 << 16)};
 }
 
-// The box of three finite screen vertices, where the plain minima and maxima
-// are box3's (NaN and infinities go through the general functions). The
-// setup kernels are bound by issue, and box3's special cases, the 64-bit
-// conversions of the pixel box and an IEEE quotient for its margin were a
-// third of a triangle's instructions.
+// The box of three screen vertices. fin: every coordinate is finite, where the
+// plain minima and maxima are box3's, and below 2^62, where the reference's
+// int() of a rounded coordinate is its value (from 2^63 on it is the smallest
+// int64, which leaves a box empty). The others go through the general
+// functions. The setup kernels are bound by issue, and box3's special cases,
+// the 64-bit conversions of the pixel box and an IEEE quotient for its margin
+// were a third of a triangle's instructions.
 struct ScrBox {
     float mnx, mxx, mny, mxy, mnz, mxz;
     bool fin;
@@ -199,7 +201,7 @@ PR_DEV ScrBox scr_box(V4 a, V4 b, V4 c) {
                                 __fadd_rn(__fadd_rn(fabsf(b.y), fabsf(b.z)),
                                           __fadd_rn(fabsf(c.x), __fadd_rn(fabsf(c.y), fabsf(c.z)))));
     return {fminf(fminf(a.x, b.x), c.x), fmaxf(fmaxf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y), fmaxf(fmaxf(a.y, b.y), c.y),
-            fminf(fminf(a.z, b.z), c.z), fmaxf(fmaxf(a.z, b.z), c.z), sum < 3e38f};
+            fminf(fminf(a.z, b.z), c.z), fmaxf(fmaxf(a.z, b.z), c.z), sum < 4e18f};
 }
 static __device__ __noinline__ bool intersect_any(float ew, float eh, V4 a, V4 b, V4 c) {
     const Box vp = {0.0f, 0.0f, -1.0f, ew, eh, 1.0f};
@@ -221,7 +223,7 @@ PR_DEV bool scr_contained(const ScrBox& s, float ew, float eh, V4 a, V4 b, V4 c)
     return s.mnx >= -kEps && s.mxx <= ew && s.mny >= -kEps && s.mxy <= eh && s.mnz >= -1.0f && s.mxz <= 1.0f;
 }
 
-// pixel_box_any for a finite box that reaches 0 or more, in float32 (the
+// pixel_box_any for a box (fin) that reaches 0 or more, in float32 (the
 // coordinates, clamped to [0, 2^16], round exactly by additions of 2^23). A
 // reciprocal rounded up in place of tighten_box's quotient only widens its margin.
 PR_DEV PixBox pixel_box(const ScrBox& s, V4 a, V4 b, V4 c, float sabc, int W, int H) {
