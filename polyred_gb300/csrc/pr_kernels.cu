@@ -45,9 +45,11 @@ PR_DEV float approx_rcp(float x) { float r; asm("rcp.approx.f32 %0, %1;" : "=f"(
 // another stream's kernels could use.
 PR_DEV void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 PR_DEV void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-PR_DEV void acquire(const uint32_t* p) {
+PR_DEV void publish(uint32_t* p) { asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(p), "r"(1u) : "memory"); }
+PR_DEV bool published(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v != 0u;
 }
 PR_DEV unsigned long long device_clock() {
     unsigned long long t;
@@ -886,8 +888,13 @@ PR_DEV void clip_one_group(const SetupParams& P, const uint32_t* clip_list, uint
 }
 __global__ void __launch_bounds__(128) clip_kernel(const __grid_constant__ SetupParams P, const uint32_t* clip_list) {
     after_previous();
-    release_next();  // the raster starts on the unclipped triangles' tasks
-    const uint32_t n = (P.cnt_rec ? P.cnt_rec : P.cnt)->n_clipped;
+    Counters* cnt = P.cnt_rec ? P.cnt_rec : P.cnt;
+    if (threadIdx.x == 0) {  // the raster starts on the unclipped triangles' tasks
+        // release_next gives no order: it finds setup's writes by this word
+        if (blockIdx.x == 0) publish(&cnt->set_up);
+        release_next();
+    }
+    const uint32_t n = cnt->n_clipped;
     constexpr uint32_t kPerBlock = 128 / kClipLanes;
     __shared__ ClipGroupSm s_g[kPerBlock];
     // grid-stride over the list (uniform per block, so every warp calls clip_one_group whole)
@@ -1282,15 +1289,15 @@ PR_DEV void raster_block(const RasterParams& P, uint2 task, uint32_t part, uint3
 constexpr uint32_t kSpreadShare = 33;  // lists with fewer tasks per warp than this (and than grab) are spread
 __global__ void __launch_bounds__(kRasterWarps * 32, 6) raster_kernel(const __grid_constant__ RasterParams P) {
     __shared__ RasterWarpSm s_w[kRasterWarps];
-    // after_clip: clip_kernel released this one past its own wait for setup, so
-    // the list is complete. One block waits for clip_kernel, so that the next
-    // kernel finds the clipped list complete; more of them would only keep the
-    // shadow passes off the device.
+    // after_clip: clip_kernel released this one past its own wait for setup. It
+    // published setup's writes before (an acquire load per block finds them: a
+    // fence here took 8 us of the 1M-triangle field's 67 and 15 of the soup's
+    // 270); a block that does not find the word set waits. One block waits for
+    // clip_kernel at the end, so that the next kernel finds the clipped list
+    // complete; more of them would only keep the shadow passes off the device.
     if (P.after_clip) {
-        // acquire setup's writes: no stale line in this SM's L1 (a fence here
-        // took 8 us of the 1M-triangle field's 67 and 15 of the soup's 270)
         if (threadIdx.x == 0) {
-            acquire(&P.cnt->n_tasks);
+            if (!published(&P.cnt->set_up)) after_previous();
             if (blockIdx.x == 0) P.cnt_w->stamp[1] = device_clock();
         }
         __syncthreads();

@@ -70,6 +70,7 @@ struct alignas(16) Counters {
     uint32_t take_attr;   // work-queue head of the attribute records
     uint32_t n_big;       // block tasks of large records (raster_block)
     uint32_t n_big_px;    // ... counted as tasks of 2^task_shift pixels
+    uint32_t set_up;      // 1: the main setup is complete, published by clip_kernel for the raster it releases
     unsigned long long stamp[3];  // device clock (ns) at the start of: the frame, its main raster, its shading
 };
 
