@@ -338,8 +338,9 @@ int pr_shadow_camera(const float light_pos[3], const float scene_center[3],
  * Limits (larger inputs are rejected with PR_ERR_INVALID_ARG, or
  * PR_ERR_OVERFLOW for the task count, leaving the map unchanged):
  * n_tris <= PR_NOALLOC_MAX_TRIS, n_objects <= PR_NOALLOC_MAX_OBJECTS,
- * width*height <= PR_NOALLOC_MAX_TEXELS, raster tasks (1024-pixel chunks of
- * the triangles' pixel boxes) <= PR_NOALLOC_MAX_TASKS.
+ * width*height <= PR_NOALLOC_MAX_TEXELS (of any shape; sides above 65000
+ * go through slower kernels), raster tasks (1024-pixel chunks of the
+ * triangles' pixel boxes) <= PR_NOALLOC_MAX_TASKS.
  *
  * The first call on a device looks up the array's device address. Every
  * call uses the same array: calls

@@ -160,7 +160,7 @@ PR_DEV void tighten_box(V4 a, V4 b, V4 c, float sabc, long long& x0, long long& 
         x1 = 0;
         return;
     }
-    // within the reference box (|coordinates| < 2^16 there): float compares, then exact conversions
+    // within the reference box (|coordinates| < 2^24 there): float compares, then exact conversions
     if (lx > (float)x0) x0 = (long long)lx;
     if (hx < (float)x1) x1 = (long long)hx;
     if (ly > (float)y0) y0 = (long long)ly;
@@ -173,17 +173,21 @@ PR_DEV void tighten_box(V4 a, V4 b, V4 c, float sabc, long long& x0, long long& 
 struct PixBox {
     uint32_t area, bx, by;
 };
-static __device__ __noinline__ PixBox pixel_box_any(V4 a, V4 b, V4 c, float sabc, int W, int H) {
+PR_DEV bool pixel_range(V4 a, V4 b, V4 c, float sabc, int W, int H, long long& x0, long long& x1, long long& y0, long long& y1) {
     Box r = box3(a, b, c);
     long long xmin = go_f2i(__fsub_rn(pround(r.mnx), 1.0f));
     long long xmax = go_f2i(__fadd_rn(pround(r.mxx), 1.0f));
     long long ymin = go_f2i(__fsub_rn(pround(r.mny), 1.0f));
     long long ymax = go_f2i(__fadd_rn(pround(r.mxy), 1.0f));
-    long long x0 = xmin < 0 ? 0 : xmin, x1 = xmax > W - 1 ? W - 1 : xmax;
-    long long y0 = ymin < 0 ? 0 : ymin, y1 = ymax > H - 1 ? H - 1 : ymax;
-    if (x0 > x1 || y0 > y1) return {0u, 0u, 0u};
+    x0 = xmin < 0 ? 0 : xmin, x1 = xmax > W - 1 ? W - 1 : xmax;
+    y0 = ymin < 0 ? 0 : ymin, y1 = ymax > H - 1 ? H - 1 : ymax;
+    if (x0 > x1 || y0 > y1) return false;
     tighten_box(a, b, c, sabc, x0, x1, y0, y1);
-    if (x0 > x1 || y0 > y1) return {0u, 0u, 0u};
+    return x0 <= x1 && y0 <= y1;
+}
+static __device__ __noinline__ PixBox pixel_box_any(V4 a, V4 b, V4 c, float sabc, int W, int H) {
+    long long x0, x1, y0, y1;
+    if (!pixel_range(a, b, c, sabc, W, H, x0, x1, y0, y1)) return {0u, 0u, 0u};
     return {(uint32_t)((x1 - x0 + 1) * (y1 - y0 + 1)), (uint32_t)x0 | ((uint32_t)x1 << 16), (uint32_t)y0 | ((uint32_t)y1 << 16)};
 }
 
@@ -905,36 +909,35 @@ __global__ void __launch_bounds__(128) clip_kernel(const __grid_constant__ Setup
     }
 }
 
-// passShadows / drawDepth for one input triangle (render/shadow.go:137-192)
+// The transform and the culls of drawDepth for one input triangle
+// (render/shadow.go:137-192); false: dropped.
+PR_DEV bool shadow_geom(const SetupParams& P, const ObjCache* C, uint32_t t, SubVtx* v, float* sabc, ScrBox* box) {
+    V4 p[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) p[k] = ld4(P.pos[t * 3 + k]);
+    if (!tri_valid_of(P, t, p)) return false;
+    float trans[16];
+    object_trans(P, C, t, trans);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        float rw;
+        v[k].pos = screen_vertex(P, trans, p[k], &rw);
+        v[k].nor = {0, 0, 0, 0};
+        v[k].u = v[k].v = 0;
+        v[k].col = 0;
+    }
+    // cullBackFace (render/cull.go:26-28): culled iff cross.Z, Barycoord's Sabc, is below 0
+    *sabc = sabc_of(v[0].pos.x, v[0].pos.y, v[1].pos.x, v[1].pos.y, v[2].pos.x, v[2].pos.y);
+    if (*sabc < 0.0f) return false;
+    // cullViewFrustum (render/cull.go:15-23): NewAABB((W,H,1),(0,0,0),(0,0,-1))
+    *box = scr_box(v[0].pos, v[1].pos, v[2].pos);
+    return scr_intersects(*box, ext_w(P), ext_h(P), v[0].pos, v[1].pos, v[2].pos);
+}
 PR_DEV void setup_shadow_one(const SetupParams& P, const ObjCache* C, uint32_t t, ReserveSm& S) {
-    bool ok = false;
     SubVtx v[3];
     float sabc = 0.0f;
     ScrBox box = {};
-    if (t < P.n_tris) {
-        V4 p[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) p[k] = ld4(P.pos[t * 3 + k]);
-        if (tri_valid_of(P, t, p)) {
-            float trans[16];
-            object_trans(P, C, t, trans);
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                float rw;
-                v[k].pos = screen_vertex(P, trans, p[k], &rw);
-                v[k].nor = {0, 0, 0, 0};
-                v[k].u = v[k].v = 0;
-                v[k].col = 0;
-            }
-            // cullBackFace (render/cull.go:26-28): culled iff cross.Z, Barycoord's Sabc, is below 0
-            sabc = sabc_of(v[0].pos.x, v[0].pos.y, v[1].pos.x, v[1].pos.y, v[2].pos.x, v[2].pos.y);
-            if (!(sabc < 0.0f)) {
-                // cullViewFrustum (render/cull.go:15-23): NewAABB((W,H,1),(0,0,0),(0,0,-1))
-                box = scr_box(v[0].pos, v[1].pos, v[2].pos);
-                ok = scr_intersects(box, ext_w(P), ext_h(P), v[0].pos, v[1].pos, v[2].pos);
-            }
-        }
-    }
+    const bool ok = t < P.n_tris && shadow_geom(P, C, t, v, &sabc, &box);
     __syncwarp();
     PixBox pb = {0u, 0u, 0u};
     if (ok) pb = pixel_box(box, v[0].pos, v[1].pos, v[2].pos, sabc, P.W, P.H);
@@ -1076,14 +1079,8 @@ PR_DEV bool pixel_depth(const SmRec& r, int px, int py, float* zout) {
     return true;
 }
 
-// The exact test and the depth write of one queued pixel.
-PR_DEV void raster_pixel(const RasterParams& P, const RasterWarpSm& S, uint32_t ent) {
-    const SmRec& r = S.rec[ent >> 27];
-    int px, py;
-    rec_pixel(r.bb, ent & 0x7FFFFFFu, &px, &py);
-    float z;
-    if (!pixel_depth(r, px, py, &z)) return;
-    const uint32_t seq = __float_as_uint(r.zs.w);
+// The depth write of a covered pixel.
+PR_DEV void put_fragment(const RasterParams& P, int px, int py, float z, uint32_t seq) {
     const bool zn = isnan(z);
     if (P.mode == kMain) {
         size_t i = (size_t)(P.H - 1 - py) * P.W + px;
@@ -1115,6 +1112,14 @@ PR_DEV void raster_pixel(const RasterParams& P, const RasterWarpSm& S, uint32_t 
         uint32_t ln = P.lastnan[i];
         if (!zn && ln != 0u && seq + 1u > ln) atomicMax(&P.smap[i], fkey(z));
     }
+}
+// The exact test and the depth write of one queued pixel.
+PR_DEV void raster_pixel(const RasterParams& P, const RasterWarpSm& S, uint32_t ent) {
+    const SmRec& r = S.rec[ent >> 27];
+    int px, py;
+    rec_pixel(r.bb, ent & 0x7FFFFFFu, &px, &py);
+    float z;
+    if (pixel_depth(r, px, py, &z)) put_fragment(P, px, py, z, __float_as_uint(r.zs.w));
 }
 
 // Tasks [base, base + 32) of one pass, one per lane, pixels spread over the
@@ -3364,6 +3369,10 @@ constexpr uint32_t kNoAllocMaxObjects = 256;
 constexpr uint32_t kNoAllocMaxTexels = 1u << 20;  // e.g. 1024 x 1024
 constexpr uint32_t kNoAllocMaxTasks = 4u * kNoAllocMaxTris;
 constexpr uint32_t kNoAllocTaskShift = 10;  // 1024-pixel tasks: the fixed task table covers large triangles
+// The longest side that setup_shadow_kernel and raster_kernel take: corners are
+// 16 bits, and rec_pixel's quotient of an index below bw + 2^10 is exact while
+// (bw + 2^10) bw < 2^32. Longer maps go through the kernels below.
+constexpr int kNoAllocMaxSide = 65000;
 
 constexpr size_t kNaCounters = 0;                                   // Counters
 constexpr size_t kNaObjFirst = 256;                                 // u32 [max_objects + 1]
@@ -3428,6 +3437,60 @@ __global__ void decode_changed_kernel(const uint32_t* keys, float* depth, size_t
     const float d = depth[i];
     const uint32_t k0 = isnan(d) ? 0u : fkey(d), k = keys[i];
     if (k != k0) depth[i] = fkey_decode(k);
+}
+
+// Maps with a side above kNoAllocMaxSide (so at most 16 texels across):
+// records whose box is four whole words, and a warp per record. Every texel of
+// a box takes the exact test; the tasks the other path would have made are
+// counted, for the same limit.
+__global__ void __launch_bounds__(128) long_map_setup_kernel(const __grid_constant__ SetupParams P) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= P.n_tris) return;
+    SubVtx v[3];
+    float sabc = 0.0f;
+    ScrBox box = {};
+    long long x0 = 1, x1 = 0, y0 = 0, y1 = -1;
+    RasterRec& R = P.rrec[t];
+    if (shadow_geom(P, nullptr, t, v, &sabc, &box) && pixel_range(v[0].pos, v[1].pos, v[2].pos, sabc, P.W, P.H, x0, x1, y0, y1)) {
+        for (int k = 0; k < 3; k++) {
+            R.v[3 * k] = v[k].pos.x;
+            R.v[3 * k + 1] = v[k].pos.y;
+            R.v[3 * k + 2] = v[k].pos.z;
+        }
+        R.sabc = sabc;
+        atomicAdd(&P.cnt->n_tasks, n_tasks_of((uint32_t)((x1 - x0 + 1) * (y1 - y0 + 1)), P.task_shift));
+    } else {
+        x0 = 1, x1 = 0;
+    }
+    R.bx = (uint32_t)x0;
+    R.by = (uint32_t)x1;
+    R.recipw[0] = __uint_as_float((uint32_t)y0);
+    R.recipw[1] = __uint_as_float((uint32_t)y1);
+}
+__global__ void __launch_bounds__(256) long_map_raster_kernel(const __grid_constant__ RasterParams P, uint32_t n) {
+    if (P.cnt->n_tasks > kNoAllocMaxTasks) {
+        atomicOr(&P.cnt_w->overflow, 2u);
+        return;
+    }
+    if (P.mode == kShadowFixup && P.cnt_w->nan_flag == 0) return;
+    const uint32_t lane = threadIdx.x & 31u, nw = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < n; t += nw) {
+        const RasterRec& R = P.rrec[t];
+        const int x0 = (int)R.bx, x1 = (int)R.by, y0 = __float_as_int(R.recipw[0]), y1 = __float_as_int(R.recipw[1]);
+        if (x0 > x1) continue;
+        SmRec r;
+        r.ab = make_float4(R.v[0], R.v[1], R.v[3], R.v[4]);
+        r.e0 = make_float4(__fsub_rn(R.v[3], R.v[0]), __fsub_rn(R.v[4], R.v[1]), __fsub_rn(R.v[6], R.v[0]), __fsub_rn(R.v[7], R.v[1]));
+        r.e1 = make_float4(__fsub_rn(R.v[6], R.v[3]), __fsub_rn(R.v[7], R.v[4]), 0.0f, R.sabc);
+        r.zs = make_float4(R.v[2], R.v[5], R.v[8], 0.0f);
+        const uint32_t bw = (uint32_t)(x1 - x0 + 1), area = bw * (uint32_t)(y1 - y0 + 1);  // at most 2^20
+        for (uint32_t k = lane; k < area; k += 32u) {
+            const uint32_t row = k / bw;
+            const int px = x0 + (int)(k - row * bw), py = y0 + (int)row;
+            float z;
+            if (pixel_depth(r, px, py, &z)) put_fragment(P, px, py, z, t);
+        }
+    }
 }
 
 std::mutex g_noalloc_mu;
@@ -3545,7 +3608,7 @@ extern "C" int pr_depth_map_noalloc(const pr_depth_map_desc* d) {
     sp.cap_tasks = kNoAllocMaxTasks;
     sp.cnt = cnt;
     sp.task_shift = kNoAllocTaskShift;
-    int rc = launch_setup_shadow(sp, st);
+    const bool long_map = d->width > kNoAllocMaxSide || d->height > kNoAllocMaxSide;
     RasterParams rp{};
     rp.task_shift = kNoAllocTaskShift;
     rp.rrec = rrec;
@@ -3554,15 +3617,19 @@ extern "C" int pr_depth_map_noalloc(const pr_depth_map_desc* d) {
     rp.cnt_w = cnt;
     rp.W = d->width;
     rp.H = d->height;
-    rp.mode = kShadow;
     rp.smap = keys;
     rp.lastnan = lastnan;
-    rp.take = &cnt->take[0];
-    if (!rc) rc = launch_raster(rp, sm_count() * 8, st);
+    auto raster = [&](RasterMode mode, uint32_t* take) {
+        rp.mode = mode;
+        rp.take = take;
+        return long_map ? launch(false, long_map_raster_kernel, (unsigned)sm_count() * 8u, 256, st, rp, d->n_tris)
+                        : launch_raster(rp, sm_count() * 8, st);
+    };
+    int rc = !long_map ? launch_setup_shadow(sp, st)
+                       : d->n_tris ? launch(false, long_map_setup_kernel, (d->n_tris + 127u) / 128u, 128, st, sp) : 0;
+    if (!rc) rc = raster(kShadow, &cnt->take[0]);
     if (!rc) rc = launch_shadow_fixup_reset(d->width, d->height, lastnan, keys, cnt, st);
-    rp.mode = kShadowFixup;
-    rp.take = &cnt->take[1];
-    if (!rc) rc = launch_raster(rp, sm_count() * 8, st);
+    if (!rc) rc = raster(kShadowFixup, &cnt->take[1]);
     if (rc) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: kernel launch failed");
     rc = launch(true, decode_changed_kernel, (unsigned)((n + 255) / 256), 256, st, keys, d->depth, n, cnt);
     if (rc) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: kernel launch failed");

@@ -1,5 +1,6 @@
 """pr_depth_map_noalloc against the oracle's drawDepth: vertices so far out that
-the reference's int64 pixel bounds overflow."""
+the reference's int64 pixel bounds overflow; maps up to 2^20 texels long, whose
+corners do not fit 16 bits."""
 import ctypes as C
 
 import numpy as np
@@ -73,3 +74,40 @@ def test_far_vertices(native_lib, axis, sign):
         tris.append(t if axis == 0 else t[:, [1, 0, 2]])
     want = check(native_lib, _soup(both_windings(tris)), 64, 64)
     assert 50 < (want != 0).sum() < 64 * 64
+
+
+def long_triangles(w, h):
+    """Small and long triangles along the whole map and past its ends; every 16th edge-on along a line of texel
+    centres (0 / 0 barycentrics: NaN depths)."""
+    g = np.random.default_rng(w + 3 * h)
+    long, short = max(w, h), min(w, h)
+    k = 400
+    at = g.uniform(-2.05, 2.05, (k, 1)) + np.where(g.random((k, 3)) < 0.5, 6.0 / long, g.choice([1e-3, 3e-2, 0.5], (k, 1))) * g.normal(0, 1, (k, 3))
+    across = g.uniform(-2, 2, (k, 1)) + g.normal(0, 0.8, (k, 3))
+    across[::16] = -2 + 4 * (g.integers(0, short, (k // 16, 1)) + 0.5) / short
+    z = g.uniform(-2, 2, (k, 1)) + g.normal(0, 0.3, (k, 3))
+    return np.stack([at, across, z] if w > h else [across, at, z], 2)
+
+
+@pytest.mark.parametrize("w,h", [(1 << 20, 1), (1, 1 << 20), (131072, 8), (8, 131072), (65537, 15), (65001, 16), (65000, 16), (16, 65000), (16385, 60)])
+def test_long_maps(native_lib, w, h):
+    want = check(native_lib, _soup(both_windings(long_triangles(w, h))), w, h)
+    row = want.any(0) if w > h else want.any(1)
+    n = len(row)
+    assert row[: n // 16].any() and row[-(n // 16):].any()
+    if min(w, h) & (min(w, h) - 1) == 0:  # texel centres are float32 numbers
+        assert np.isnan(want).any()
+
+
+def test_long_map_overflow_leaves_the_map_unchanged(native_lib):
+    """260 triangles that cover 131072 x 8 texels need 1024 tasks apiece: refused as on a square map; 200 are not."""
+    tris = [[[-9, -9, -1 + k / 260], [9, -9, -1 + k / 260], [0, 12, -1 + k / 260]] for k in range(260)]
+    soup = _soup(both_windings(tris))
+    view, proj = _ortho()
+    init = np.random.default_rng(7).uniform(-1, 1, (8, 131072)).astype(np.float32)
+    init.view(np.uint32)[:, ::13] = 0x7FA00001
+    for n, ok in ((260, False), (200, True)):
+        _, flat = oracle_map(soup[: 2 * n], 4, 4, view, proj)
+        rc, got = device_map(native_lib, flat, 131072, 8, view, proj, init)
+        same = np.array_equal(got.view(np.uint32), init.view(np.uint32))
+        assert (rc, same) == ((_abi.PR_OK, False) if ok else (_abi.PR_ERR_OVERFLOW, True))
