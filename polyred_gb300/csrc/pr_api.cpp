@@ -82,6 +82,9 @@ cudaError_t host_malloc(void** p, size_t bytes) {
     return cudaHostAlloc(p, bytes, cudaHostAllocDefault);
 }
 
+// Frees device memory that the running call can do without (MayYield).
+bool free_spare();
+
 // A device allocation that only grows. A failed growth leaves it empty
 // (p == nullptr, n == 0): the old buffer is freed first, so that the peak
 // holds one buffer, and callers keep no capacity derived from it.
@@ -96,6 +99,7 @@ struct DevBuf {
         n = 0;
         size_t alloc = std::max<size_t>(want, 1);
         cudaError_t e = dev_malloc((void**)&p, alloc * sizeof(T));
+        if (e != cudaSuccess && free_spare()) e = dev_malloc((void**)&p, alloc * sizeof(T));
         if (e != cudaSuccess) {
             p = nullptr;
             return fail(PR_ERR_OOM, "cudaMalloc(%zu bytes): %s", alloc * sizeof(T), cudaGetErrorString(e));
@@ -109,6 +113,34 @@ struct DevBuf {
         n = 0;
     }
 };
+
+// While it lives, a device allocation of this thread that finds no memory frees
+// b and tries again (cudaFree waits for the kernels that may use it).
+struct MayYield;
+thread_local MayYield* g_yield = nullptr;
+struct MayYield {
+    DevBuf<float>& b;
+    MayYield* prev;
+    explicit MayYield(DevBuf<float>& buf) : b(buf), prev(g_yield) { g_yield = this; }
+    ~MayYield() { g_yield = prev; }
+    MayYield(const MayYield&) = delete;
+};
+bool free_spare() {
+    for (MayYield* y = g_yield; y; y = y->prev)
+        if (y->b.p) {
+            y->b.release();
+            (void)cudaGetLastError();  // the failed allocation's
+            return true;
+        }
+    return false;
+}
+
+// Grows b if there is memory; without, b is empty (p == nullptr).
+void ensure_optional(DevBuf<float>& b, size_t want) {
+    if (want <= b.n) return;
+    b.release();
+    if (b.ensure(want)) (void)cudaGetLastError();  // not a later launch's failure
+}
 
 // Page-locked host memory that grows on demand.
 struct HostBuf {
@@ -231,7 +263,7 @@ struct Ctx {
     cudaEvent_t ev_resolved = nullptr, ev_ao0 = nullptr, ev_ao = nullptr;
     bool ao_marched = false;  // the last frame ran the AO march (ev_ao0, ev_ao hold it)
     DevBuf<float> ao_T;
-    DevBuf<float> linemax;  // [4][H][W], AO's line maxima
+    DevBuf<float> linemax;  // [4][H][W], AO's line maxima; empty without memory for them
     DevBuf<uint8_t> gamma;   // GammaCorrection's table (prh::gamma_table)
     DevBuf<uint8_t> ao_tab;  // AO's tap tables for frames of width ao_tab_w and rounding ao_tab_ulp
     int ao_tab_w = 0;
@@ -709,6 +741,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
     M4 s2w = prh::mulm(prh::mulm(view_inv, proj_inv), vp_inv);
 
     if ((rc = set_device(c))) return rc;
+    const MayYield yield(c->linemax);
     if ((rc = ensure_frame(c, W, H))) return rc;
     uint32_t need_rec0 = c->sb.n_tris + c->sb.n_tris / 8 + 1024;
     if ((rc = ensure_work(c, need_rec0, need_rec0))) return rc;
@@ -735,8 +768,44 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         if (c->lastnan.n != l0) CUDA_TRY(cudaMemsetAsync(c->lastnan.p, 0, c->lastnan.n * 4, st));
     }
 
+    const size_t npx = (size_t)W * H;
+    // What AO and shading need; then the line maxima, from memory that the
+    // frame can do without.
+    const bool with_ao = out && out->rgba && c->sb.has_ao;
+    if (with_ao && ((rc = c->ao_T.ensure(npx)) || (rc = c->ao_tab.ensure(prk::ao_tables_bytes())))) return rc;
+    std::unique_ptr<prk::ShadeParams> sp_owner(new (std::nothrow) prk::ShadeParams());
+    if (!sp_owner) return fail(PR_ERR_OOM, "host allocation failed");
+    prk::ShadeParams& sp = *sp_owner;
+    // outputs: device pointers directly, or ctx staging buffers
+    if (out_dev) {
+        sp.rgba = (uchar4*)out->rgba;
+        sp.tri_id = out->tri_id;
+        sp.depth = out->depth;
+        sp.gnor = (float4*)out->nor;
+        sp.gfnor = (float4*)out->face_nor;
+        sp.gwpos = (float4*)out->world_pos;
+        sp.guvd = (float4*)out->uvd;
+        sp.gvcol = (uchar4*)out->vcol;
+        sp.gmat = out->mat_id;
+    } else if (out) {
+        if (out->rgba) { if ((rc = c->o_rgba.ensure(npx * 4))) return rc; sp.rgba = (uchar4*)c->o_rgba.p; }
+        if (out->tri_id) { if ((rc = c->o_tri.ensure(npx))) return rc; sp.tri_id = c->o_tri.p; }
+        if (out->depth) { if ((rc = c->o_depth.ensure(npx))) return rc; sp.depth = c->o_depth.p; }
+        if (out->nor) { if ((rc = c->o_nor.ensure(npx))) return rc; sp.gnor = c->o_nor.p; }
+        if (out->face_nor) { if ((rc = c->o_fnor.ensure(npx))) return rc; sp.gfnor = c->o_fnor.p; }
+        if (out->world_pos) { if ((rc = c->o_wpos.ensure(npx))) return rc; sp.gwpos = c->o_wpos.p; }
+        if (out->uvd) { if ((rc = c->o_uvd.ensure(npx))) return rc; sp.guvd = c->o_uvd.p; }
+        if (out->vcol) { if ((rc = c->o_vcol.ensure(npx * 4))) return rc; sp.gvcol = (uchar4*)c->o_vcol.p; }
+        if (out->mat_id) { if ((rc = c->o_mat.ensure(npx))) return rc; sp.gmat = c->o_mat.p; }
+    }
+    uchar4* rgba_img = sp.rgba;  // the image Render() returns
+    if (M > 1 && sp.rgba) {
+        if ((rc = c->o_msaa.ensure(npx * 4))) return rc;
+        sp.rgba = (uchar4*)c->o_msaa.p;  // the framebuffer's colours
+    }
+    if (with_ao) ensure_optional(c->linemax, 4 * npx);
+
     prk::Counters* dcnt = c->cnt.p;
-    size_t npx = (size_t)W * H;
     c->stats = pr_stats{};
     c->stats.size = sizeof(pr_stats);
     c->stats.n_tris_in = c->sb.n_tris;
@@ -912,9 +981,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         // writes attributes and shades; the colour scaling joins after shading.
         // A scene without an AO material lists no pixel, and both launches are
         // left out.
-        const bool with_ao = out && out->rgba && c->sb.has_ao;
         c->ao_marched = with_ao;
-        if (with_ao && ((rc = c->ao_T.ensure(npx)) || (rc = c->linemax.ensure(4 * npx)))) return rc;
         KTRY(prk::launch_resolve(W, H, c->keys.p, c->nanseq.p, c->beaten.p, dcnt, c->win.p, c->depth_ao.p, c->first_rec.p,
                                  c->attr_state.p, c->sb.tri_flags.p, with_ao ? c->ao_list.p : nullptr, c->linemax.p, st));
         prk::AoParams ap{};
@@ -936,7 +1003,6 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             ap.exact_T = dh ? 1 : 0;
             if (c->ao_tab_w != W || c->ao_tab_ulp != ap.ao_half_ulp) {
                 c->ao_tab_w = 0;
-                if ((rc = c->ao_tab.ensure(prk::ao_tables_bytes()))) return rc;
                 KTRY(prk::launch_ao_tables(ap, c->ao_tab.p, sc));
                 c->ao_tab_w = W;
                 c->ao_tab_ulp = ap.ao_half_ulp;
@@ -951,9 +1017,6 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         if ((rc = shadows_finish())) return rc;
 
         // ---- deferred shading + gamma (render/raster.go:275-378) ----
-        std::unique_ptr<prk::ShadeParams> sp_owner(new (std::nothrow) prk::ShadeParams());
-        if (!sp_owner) return fail(PR_ERR_OOM, "host allocation failed");
-        prk::ShadeParams& sp = *sp_owner;
         fill_shade_frame(c, f, s2w, SW, SH, sp);
         sp.win = c->win.p;
         sp.depth_ao = c->depth_ao.p;
@@ -965,33 +1028,6 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         if (dh) {
             sp.tri_scr = c->tri_scr.p;
             sp.dgb = dh->dgb;
-        }
-        // outputs: device pointers directly, or ctx staging buffers
-        if (out_dev) {
-            sp.rgba = (uchar4*)out->rgba;
-            sp.tri_id = out->tri_id;
-            sp.depth = out->depth;
-            sp.gnor = (float4*)out->nor;
-            sp.gfnor = (float4*)out->face_nor;
-            sp.gwpos = (float4*)out->world_pos;
-            sp.guvd = (float4*)out->uvd;
-            sp.gvcol = (uchar4*)out->vcol;
-            sp.gmat = out->mat_id;
-        } else if (out) {
-            if (out->rgba) { if ((rc = c->o_rgba.ensure(npx * 4))) return rc; sp.rgba = (uchar4*)c->o_rgba.p; }
-            if (out->tri_id) { if ((rc = c->o_tri.ensure(npx))) return rc; sp.tri_id = c->o_tri.p; }
-            if (out->depth) { if ((rc = c->o_depth.ensure(npx))) return rc; sp.depth = c->o_depth.p; }
-            if (out->nor) { if ((rc = c->o_nor.ensure(npx))) return rc; sp.gnor = c->o_nor.p; }
-            if (out->face_nor) { if ((rc = c->o_fnor.ensure(npx))) return rc; sp.gfnor = c->o_fnor.p; }
-            if (out->world_pos) { if ((rc = c->o_wpos.ensure(npx))) return rc; sp.gwpos = c->o_wpos.p; }
-            if (out->uvd) { if ((rc = c->o_uvd.ensure(npx))) return rc; sp.guvd = c->o_uvd.p; }
-            if (out->vcol) { if ((rc = c->o_vcol.ensure(npx * 4))) return rc; sp.gvcol = (uchar4*)c->o_vcol.p; }
-            if (out->mat_id) { if ((rc = c->o_mat.ensure(npx))) return rc; sp.gmat = c->o_mat.p; }
-        }
-        uchar4* rgba_img = sp.rgba;  // the image Render() returns
-        if (M > 1 && sp.rgba) {
-            if ((rc = c->o_msaa.ensure(npx * 4))) return rc;
-            sp.rgba = (uchar4*)c->o_msaa.p;  // the framebuffer's colours
         }
         sp.ao_listed = 1;  // listed by resolve
         if (casts) CUDA_TRY(cudaStreamWaitEvent(st, c->ev[1], 0));          // the shadow maps are complete
@@ -1220,6 +1256,7 @@ int pr_scene_upload(void* ctx, const pr_scene_desc* s) {
     CUDA_TRY(cudaStreamSynchronize(c->stream_d));
     clear_stale_error();
     c->has_scene = false;  // until the new scene is complete (a failed upload leaves none)
+    const MayYield yield(c->linemax);
     if ((rc = scene_fill(c->sb, s, c->stream, false)) || (rc = scene_flags(c->sb, c->stream))) return rc;
     CUDA_TRY(cudaStreamSynchronize(c->stream));  // host tables go out of scope
     c->has_scene = true;
@@ -1241,7 +1278,10 @@ int pr_frame_submit(void* ctx, const pr_scene_desc* scene, const pr_frame_desc* 
     // no frame reads its triangles and objects any more (scene_fill waits for
     // shading before it touches the materials)
     CUDA_TRY(cudaStreamWaitEvent(c->stream_u, b.ev_geometry, 0));
-    if ((rc = scene_fill(b, scene, c->stream_u, true))) return rc;
+    {
+        const MayYield yield(c->linemax);
+        if ((rc = scene_fill(b, scene, c->stream_u, true))) return rc;
+    }
     CUDA_TRY(cudaEventRecord(b.ev_uploaded, c->stream_u));
     std::swap(c->sb, c->sb_back);
     c->has_scene = true;
@@ -1441,6 +1481,7 @@ namespace {
 // Device parameters of a differentiable call: the caller's or the scene's.
 int diff_setup(Ctx* c, const pr_frame_desc* f, const pr_diff_params* prm, prk::DiffParamsK& K) {
     int rc;
+    const MayYield yield(c->linemax);
     const uint32_t nm = (uint32_t)c->sb.materials.size();
     if (c->sb.has_tex) return fail(PR_ERR_UNSUPPORTED, "image textures are not available in the adjoint");
     if (prm && prm->size < sizeof(pr_diff_params)) return fail(PR_ERR_INVALID_ARG, "params->size too small");
@@ -1753,13 +1794,18 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
     int rc;
     bool any_ao = false;
     for (uint32_t v = 0; v < nv; v++) any_ao |= b->scenes[views[v].scene]->sb.has_ao;
-    if ((rc = b->rrec.ensure(std::max<size_t>(rec, 1))) || (rc = b->arec.ensure(std::max<size_t>(p.n_rec_main, 1))) ||
-        (rc = b->tasks.ensure(std::max<size_t>(task, 1))) || (rc = b->first_rec.ensure(nfirst)) ||
-        (rc = b->clip_list.ensure(nfirst)) || (rc = b->cnt.ensure(nv + p.S)) || (rc = b->keys.ensure(npx)) ||
-        (rc = b->nanseq.ensure(npx)) || (rc = b->beaten.ensure(npx)) || (rc = b->win.ensure(npx)) ||
-        (rc = b->ao_list.ensure(npx)) || (rc = b->depth_ao.ensure(npx)) || (rc = b->linemax.ensure(any_ao ? 4 * npx : 1)) || (rc = b->chunk.ensure(nv)) ||
-        (rc = b->smaps.ensure(std::max<size_t>(nsm, 1))))
-        return rc;
+    {
+        const MayYield yield(b->linemax);
+        if ((rc = b->rrec.ensure(std::max<size_t>(rec, 1))) || (rc = b->arec.ensure(std::max<size_t>(p.n_rec_main, 1))) ||
+            (rc = b->tasks.ensure(std::max<size_t>(task, 1))) || (rc = b->first_rec.ensure(nfirst)) ||
+            (rc = b->clip_list.ensure(nfirst)) || (rc = b->cnt.ensure(nv + p.S)) || (rc = b->keys.ensure(npx)) ||
+            (rc = b->nanseq.ensure(npx)) || (rc = b->beaten.ensure(npx)) || (rc = b->win.ensure(npx)) ||
+            (rc = b->ao_list.ensure(npx)) || (rc = b->depth_ao.ensure(npx)) || (rc = b->chunk.ensure(nv)) ||
+            (rc = b->smaps.ensure(std::max<size_t>(nsm, 1))))
+            return rc;
+    }
+    // 16 of a pixel's 44 bytes: a batch that fits only without them marches by taps
+    if (any_ao) ensure_optional(b->linemax, 4 * npx);
     if (b->h_cnt_n < nv + p.S) {
         if (b->h_cnt) cudaFreeHost(b->h_cnt);
         b->h_cnt = nullptr;
@@ -1910,7 +1956,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
                                           ap.dir_tiny);
         ap.depth = R.depth_ao;
         ap.list = sp.ao_list;
-        ap.linemax = b->linemax.p + (any_ao ? 4 * o : 0);
+        ap.linemax = any_ao && b->linemax.p ? b->linemax.p + 4 * o : nullptr;
         ap.cnt = mp.cnt;
         ap.rgba = sp.rgba;
         ap.gamma = sp.gamma;
@@ -2097,6 +2143,7 @@ int batch_run(Batch* b, uint32_t nv, const pr_batch_view* views) {
             continue;
         }
         // NaN depth in a shadow pass needs the per-texel fix-up of the single-view path
+        const MayYield yield(b->linemax);
         for (uint32_t v = 0; v < nv; v++) {
             if (!redo[v]) continue;
             Ctx* c = b->scenes[views[v].scene];
@@ -2173,6 +2220,7 @@ int pr_batch_add_scene(void* batch, const pr_scene_desc* scene, uint32_t* out_in
     if (scene->size >= PR_SCENE_DESC_SIZE_V1 && scene_has_images(scene))
         return fail(PR_ERR_UNSUPPORTED, "image textures are not available in batches");
     std::lock_guard<std::mutex> lk(b->mu);
+    const MayYield yield(b->linemax);
     void* c = nullptr;
     int rc = pr_create(b->device, &c);
     if (rc) return rc;

@@ -1481,7 +1481,7 @@ __global__ void __launch_bounds__(256) resolve_kernel(int W, int H, const unsign
         for (int q = 0; q < warp; q++) o += s_cnt[q];
         ao_list[o] = (uint32_t)i;
     }
-    if (!cnt->nan_flag)  // uniform; a frame with NaN depths marches without them
+    if (linemax && !cnt->nan_flag)  // uniform; a frame with NaN depths marches without them
         ao_linemax_tile(W, H, blockIdx.x * 32, blockIdx.y * 8, linemax, [&](int cx, int cr) {
             const unsigned long long key = keys[(size_t)cr * W + cx];
             return key != 0ull ? fkey_decode((uint32_t)(key >> 32)) : -1.0f;
@@ -2690,8 +2690,9 @@ PR_DEV int ao_tiny_cross(float c, float p) {
     return lo;
 }
 
-// Pixel i's total T in a frame with NaN depths (NaN: a direction met one).
-__device__ __noinline__ float ao_total_nan(const AoParams& P, uint32_t i, const AoTables& S) {
+// Pixel i's total T in a frame with NaN depths (NaN: a direction met one), or
+// without line maxima (no memory for them): every tap by itself.
+__device__ __noinline__ float ao_total_taps(const AoParams& P, uint32_t i, const AoTables& S) {
     const int W = P.W, H = P.H, r = (int)(i / (uint32_t)W), x = (int)i - r * W, y = H - 1 - r;
     const float* p0 = P.depth + i;
     const float z = *p0;
@@ -2732,8 +2733,8 @@ PR_DEV void ao_one(const AoParams& P, uint32_t j, uint32_t n, const AoTables& S)
     const bool mine = j < n;
     const uint32_t i = P.list[min(j, n - 1u)];
     float T;
-    if (P.cnt->nan_flag != 0u) {  // some NaN-depth fragment reached this frame (the raster flags every one)
-        T = ao_total_nan(P, i, S);
+    if (P.cnt->nan_flag != 0u || !P.linemax) {  // some NaN-depth fragment reached this frame (the raster flags every one)
+        T = ao_total_taps(P, i, S);
     } else {
         const int W = P.W, H = P.H, r = (int)(i / (uint32_t)W), x = (int)i - r * W, y = H - 1 - r;
         const float z = P.depth[i];
@@ -2988,7 +2989,7 @@ __global__ void __launch_bounds__(256) shade_batch_kernel(const ShadeParams* vie
 __global__ void __launch_bounds__(256) ao_linemax_batch_kernel(const AoParams* views, const uint32_t* blk, int n_views) {
     const int v = job_of(blk, n_views, blockIdx.x);
     const AoParams& P = views[v];
-    if (P.cnt->nan_flag || P.cnt->n_ao == 0) return;
+    if (!P.linemax || P.cnt->nan_flag || P.cnt->n_ao == 0) return;
     const uint32_t b = blockIdx.x - blk[v], tiles_x = (uint32_t)(P.W + 31) / 32u;
     const uint32_t ty = b / tiles_x;
     ao_linemax_tile(P.W, P.H, (int)((b - ty * tiles_x) * 32u), (int)(ty * 8u), P.linemax,

@@ -213,7 +213,7 @@ struct AoParams {
     float* T;            // [list] the AO total of each listed pixel (ao_T_kernel -> ao_apply_kernel)
     int exact_T;         // 1: T itself is wanted (differentiation); 0: only the colours it gives
     const void* tables;  // the frame size's tap tables (launch_ao_tables); batches build their own
-    float* linemax;      // [4][H][W] maxima of four depths along x, rows, diagonal, antidiagonal
+    float* linemax;      // [4][H][W] maxima of four depths along x, rows, diagonal, antidiagonal; null: march without
 };
 
 
@@ -265,7 +265,7 @@ int launch_pass_init(const PassMats& pm, int n_pass, const float* obj_model, uin
 // (nanseq, beaten) back to kNone / 0 after a frame that used it, and, with
 // ao_list, lists the pixels whose winner's material has AO (tri_flags kTriAO)
 // in ao_list (count in cnt->n_ao), tile by tile (32 x 8), with the depths'
-// line maxima ([4][H][W], AoParams::linemax) in linemax.
+// line maxima ([4][H][W], AoParams::linemax) in linemax unless that is null.
 int launch_resolve(int W, int H, const unsigned long long* keys, uint32_t* nanseq, uint32_t* beaten, Counters* cnt,
                    uint32_t* win, float* depth_ao, const uint32_t* first_rec, uint8_t* attr_state,
                    const uint8_t* tri_flags, uint32_t* ao_list, float* linemax, void* stream);
