@@ -438,11 +438,12 @@ int ensure_frame(Ctx* c, int W, int H) {
     int rc;
     if ((rc = c->keys.ensure(n))) return rc;
     // nanseq / beaten start all-kNone / all-0 and are put back so after any
-    // frame that used them, so a new allocation is set once
+    // frame that used them, so a new allocation is set once (each at once: a
+    // failure of the next must not leave one unset)
     const size_t n0 = c->nanseq.n, b0 = c->beaten.n;
     if ((rc = c->nanseq.ensure(n))) return rc;
-    if ((rc = c->beaten.ensure(n))) return rc;
     if (c->nanseq.n != n0) CUDA_TRY(cudaMemsetAsync(c->nanseq.p, 0xff, c->nanseq.n * 4, c->stream));
+    if ((rc = c->beaten.ensure(n))) return rc;
     if (c->beaten.n != b0) CUDA_TRY(cudaMemsetAsync(c->beaten.p, 0, c->beaten.n * 4, c->stream));
     if ((rc = c->win.ensure(n))) return rc;
     if ((rc = c->depth_ao.ensure(n))) return rc;
