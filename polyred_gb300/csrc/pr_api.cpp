@@ -228,6 +228,7 @@ struct Ctx {
     DevBuf<float> obj_trans;  // [1 + lights][n_objects][16]: Proj·View·Model per pass and object
     DevBuf<unsigned long long> keys;
     DevBuf<uint32_t> nanseq, beaten, win;
+    bool nan_in_use = false;  // a frame's raster was queued, but not the resolve that puts nanseq and beaten back
     DevBuf<float> depth_ao;
     DevBuf<uint32_t> ao_list;
     int n_ao_dirs = 0;
@@ -437,14 +438,16 @@ int ensure_frame(Ctx* c, int W, int H) {
     size_t n = (size_t)W * H;
     int rc;
     if ((rc = c->keys.ensure(n))) return rc;
-    // nanseq / beaten start all-kNone / all-0 and are put back so after any
-    // frame that used them, so a new allocation is set once (each at once: a
-    // failure of the next must not leave one unset)
+    // nanseq / beaten start all-kNone / all-0 and are put back so by resolve
+    // after any frame that used them, so a new allocation is set once (each at
+    // once: a failure of the next must not leave one unset), and again after a
+    // frame that failed between its raster and resolve
     const size_t n0 = c->nanseq.n, b0 = c->beaten.n;
     if ((rc = c->nanseq.ensure(n))) return rc;
-    if (c->nanseq.n != n0) CUDA_TRY(cudaMemsetAsync(c->nanseq.p, 0xff, c->nanseq.n * 4, c->stream));
+    if (c->nanseq.n != n0 || c->nan_in_use) CUDA_TRY(cudaMemsetAsync(c->nanseq.p, 0xff, c->nanseq.n * 4, c->stream));
     if ((rc = c->beaten.ensure(n))) return rc;
-    if (c->beaten.n != b0) CUDA_TRY(cudaMemsetAsync(c->beaten.p, 0, c->beaten.n * 4, c->stream));
+    if (c->beaten.n != b0 || c->nan_in_use) CUDA_TRY(cudaMemsetAsync(c->beaten.p, 0, c->beaten.n * 4, c->stream));
+    c->nan_in_use = false;
     if ((rc = c->win.ensure(n))) return rc;
     if ((rc = c->depth_ao.ensure(n))) return rc;
     if ((rc = c->ao_list.ensure(n))) return rc;
@@ -455,6 +458,7 @@ int ensure_frame(Ctx* c, int W, int H) {
 
 int ensure_work(Ctx* c, uint32_t need_rec, uint32_t need_tasks) {
     int rc;
+    const MayYield yield(c->linemax);
     if (need_rec > c->cap_rec) {
         uint32_t cap = std::max(need_rec, c->cap_rec * 2);
         c->cap_rec = 0;  // until every buffer holds cap (a failed growth empties one)
@@ -770,42 +774,6 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
     }
 
     const size_t npx = (size_t)W * H;
-    // What AO and shading need; then the line maxima, from memory that the
-    // frame can do without.
-    const bool with_ao = out && out->rgba && c->sb.has_ao;
-    if (with_ao && ((rc = c->ao_T.ensure(npx)) || (rc = c->ao_tab.ensure(prk::ao_tables_bytes())))) return rc;
-    std::unique_ptr<prk::ShadeParams> sp_owner(new (std::nothrow) prk::ShadeParams());
-    if (!sp_owner) return fail(PR_ERR_OOM, "host allocation failed");
-    prk::ShadeParams& sp = *sp_owner;
-    // outputs: device pointers directly, or ctx staging buffers
-    if (out_dev) {
-        sp.rgba = (uchar4*)out->rgba;
-        sp.tri_id = out->tri_id;
-        sp.depth = out->depth;
-        sp.gnor = (float4*)out->nor;
-        sp.gfnor = (float4*)out->face_nor;
-        sp.gwpos = (float4*)out->world_pos;
-        sp.guvd = (float4*)out->uvd;
-        sp.gvcol = (uchar4*)out->vcol;
-        sp.gmat = out->mat_id;
-    } else if (out) {
-        if (out->rgba) { if ((rc = c->o_rgba.ensure(npx * 4))) return rc; sp.rgba = (uchar4*)c->o_rgba.p; }
-        if (out->tri_id) { if ((rc = c->o_tri.ensure(npx))) return rc; sp.tri_id = c->o_tri.p; }
-        if (out->depth) { if ((rc = c->o_depth.ensure(npx))) return rc; sp.depth = c->o_depth.p; }
-        if (out->nor) { if ((rc = c->o_nor.ensure(npx))) return rc; sp.gnor = c->o_nor.p; }
-        if (out->face_nor) { if ((rc = c->o_fnor.ensure(npx))) return rc; sp.gfnor = c->o_fnor.p; }
-        if (out->world_pos) { if ((rc = c->o_wpos.ensure(npx))) return rc; sp.gwpos = c->o_wpos.p; }
-        if (out->uvd) { if ((rc = c->o_uvd.ensure(npx))) return rc; sp.guvd = c->o_uvd.p; }
-        if (out->vcol) { if ((rc = c->o_vcol.ensure(npx * 4))) return rc; sp.gvcol = (uchar4*)c->o_vcol.p; }
-        if (out->mat_id) { if ((rc = c->o_mat.ensure(npx))) return rc; sp.gmat = c->o_mat.p; }
-    }
-    uchar4* rgba_img = sp.rgba;  // the image Render() returns
-    if (M > 1 && sp.rgba) {
-        if ((rc = c->o_msaa.ensure(npx * 4))) return rc;
-        sp.rgba = (uchar4*)c->o_msaa.p;  // the framebuffer's colours
-    }
-    if (with_ao) ensure_optional(c->linemax, 4 * npx);
-
     prk::Counters* dcnt = c->cnt.p;
     c->stats = pr_stats{};
     c->stats.size = sizeof(pr_stats);
@@ -958,6 +926,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         rp.beaten = c->beaten.p;
         rp.take = &dcnt[0].take[0];
         rp.after_clip = 1;
+        c->nan_in_use = true;
         KTRY(prk::launch_raster(rp, c->n_sms * 8, st));
         prk::RasterParams rc_ = rp;
         rc_.after_clip = 0;
@@ -982,9 +951,15 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         // writes attributes and shades; the colour scaling joins after shading.
         // A scene without an AO material lists no pixel, and both launches are
         // left out.
+        const bool with_ao = out && out->rgba && c->sb.has_ao;
         c->ao_marched = with_ao;
+        if (with_ao) {
+            if ((rc = c->ao_T.ensure(npx))) return rc;
+            ensure_optional(c->linemax, 4 * npx);
+        }
         KTRY(prk::launch_resolve(W, H, c->keys.p, c->nanseq.p, c->beaten.p, dcnt, c->win.p, c->depth_ao.p, c->first_rec.p,
                                  c->attr_state.p, c->sb.tri_flags.p, with_ao ? c->ao_list.p : nullptr, c->linemax.p, st));
+        c->nan_in_use = false;
         prk::AoParams ap{};
         cudaStream_t sc = c->stream_c;
         if (with_ao) {
@@ -1000,15 +975,16 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             ap.list = c->ao_list.p;
             ap.cnt = dcnt;
             ap.T = c->ao_T.p;
-            ap.linemax = c->linemax.p;
             ap.exact_T = dh ? 1 : 0;
             if (c->ao_tab_w != W || c->ao_tab_ulp != ap.ao_half_ulp) {
                 c->ao_tab_w = 0;
+                if ((rc = c->ao_tab.ensure(prk::ao_tables_bytes()))) return rc;
                 KTRY(prk::launch_ao_tables(ap, c->ao_tab.p, sc));
                 c->ao_tab_w = W;
                 c->ao_tab_ulp = ap.ao_half_ulp;
             }
             ap.tables = c->ao_tab.p;
+            ap.linemax = c->linemax.p;  // here: an allocation since resolve may have taken their memory
             KTRY(prk::launch_ao_T(ap, sc));
             CUDA_TRY(cudaEventRecord(c->ev_ao, sc));
             launches += 1;
@@ -1018,6 +994,9 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         if ((rc = shadows_finish())) return rc;
 
         // ---- deferred shading + gamma (render/raster.go:275-378) ----
+        std::unique_ptr<prk::ShadeParams> sp_owner(new (std::nothrow) prk::ShadeParams());
+        if (!sp_owner) return fail(PR_ERR_OOM, "host allocation failed");
+        prk::ShadeParams& sp = *sp_owner;
         fill_shade_frame(c, f, s2w, SW, SH, sp);
         sp.win = c->win.p;
         sp.depth_ao = c->depth_ao.p;
@@ -1029,6 +1008,33 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         if (dh) {
             sp.tri_scr = c->tri_scr.p;
             sp.dgb = dh->dgb;
+        }
+        // outputs: device pointers directly, or ctx staging buffers
+        if (out_dev) {
+            sp.rgba = (uchar4*)out->rgba;
+            sp.tri_id = out->tri_id;
+            sp.depth = out->depth;
+            sp.gnor = (float4*)out->nor;
+            sp.gfnor = (float4*)out->face_nor;
+            sp.gwpos = (float4*)out->world_pos;
+            sp.guvd = (float4*)out->uvd;
+            sp.gvcol = (uchar4*)out->vcol;
+            sp.gmat = out->mat_id;
+        } else if (out) {
+            if (out->rgba) { if ((rc = c->o_rgba.ensure(npx * 4))) return rc; sp.rgba = (uchar4*)c->o_rgba.p; }
+            if (out->tri_id) { if ((rc = c->o_tri.ensure(npx))) return rc; sp.tri_id = c->o_tri.p; }
+            if (out->depth) { if ((rc = c->o_depth.ensure(npx))) return rc; sp.depth = c->o_depth.p; }
+            if (out->nor) { if ((rc = c->o_nor.ensure(npx))) return rc; sp.gnor = c->o_nor.p; }
+            if (out->face_nor) { if ((rc = c->o_fnor.ensure(npx))) return rc; sp.gfnor = c->o_fnor.p; }
+            if (out->world_pos) { if ((rc = c->o_wpos.ensure(npx))) return rc; sp.gwpos = c->o_wpos.p; }
+            if (out->uvd) { if ((rc = c->o_uvd.ensure(npx))) return rc; sp.guvd = c->o_uvd.p; }
+            if (out->vcol) { if ((rc = c->o_vcol.ensure(npx * 4))) return rc; sp.gvcol = (uchar4*)c->o_vcol.p; }
+            if (out->mat_id) { if ((rc = c->o_mat.ensure(npx))) return rc; sp.gmat = c->o_mat.p; }
+        }
+        uchar4* rgba_img = sp.rgba;  // the image Render() returns
+        if (M > 1 && sp.rgba) {
+            if ((rc = c->o_msaa.ensure(npx * 4))) return rc;
+            sp.rgba = (uchar4*)c->o_msaa.p;  // the framebuffer's colours
         }
         sp.ao_listed = 1;  // listed by resolve
         if (casts) CUDA_TRY(cudaStreamWaitEvent(st, c->ev[1], 0));          // the shadow maps are complete
@@ -1567,6 +1573,7 @@ int pr_diff_forward(void* ctx, const pr_frame_desc* frame, const pr_diff_params*
     o.flags = PR_OUT_DEVICE_PTRS;
     const size_t npx = (size_t)frame->width * frame->height;
     if (!o.rgba) {
+        const MayYield yield(c->linemax);
         if ((rc = c->o_rgba.ensure(npx * 4))) return rc;
         o.rgba = c->o_rgba.p;
     }
@@ -1731,6 +1738,7 @@ struct BatchPlan {
     std::vector<uint32_t> blk;             // blk_s[S+1] blk_m[V+1] blk_r[V+1] blk_sh[V+1]
     uint32_t nb_s = 0, nb_m = 0, nb_r = 0, nb_sh = 0;
     bool fast = true;                      // every view's shading is shade_is_fast
+    bool lines = false;                    // AO marches with line maxima
     std::vector<int> shadow_view;          // view of each shadow pass
     size_t n_rec = 0, n_rec_main = 0, n_tasks = 0, n_px = 0, n_smap = 0, n_first = 0;
     std::string key;
@@ -1807,6 +1815,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
     }
     // 16 of a pixel's 44 bytes: a batch that fits only without them marches by taps
     if (any_ao) ensure_optional(b->linemax, 4 * npx);
+    p.lines = any_ao && b->linemax.p;
     if (b->h_cnt_n < nv + p.S) {
         if (b->h_cnt) cudaFreeHost(b->h_cnt);
         b->h_cnt = nullptr;
@@ -1957,7 +1966,7 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
                                           ap.dir_tiny);
         ap.depth = R.depth_ao;
         ap.list = sp.ao_list;
-        ap.linemax = any_ao && b->linemax.p ? b->linemax.p + 4 * o : nullptr;
+        ap.linemax = p.lines ? b->linemax.p + 4 * o : nullptr;
         ap.cnt = mp.cnt;
         ap.rgba = sp.rgba;
         ap.gamma = sp.gamma;
@@ -1980,8 +1989,8 @@ int batch_plan(Batch* b, uint32_t nv, const pr_batch_view* views, BatchPlan& p) 
     (void)osh;
     // the graph's shape: everything a captured launch depends on
     char kb[128];
-    snprintf(kb, sizeof(kb), "%u/%u/%u/%u/%u/%u/%d/%zu/%zu/%d|", nv, p.S, p.nb_s, p.nb_m, p.nb_r, p.nb_sh, b->raster_bps,
-             p.n_px, p.n_smap, (int)p.fast);
+    snprintf(kb, sizeof(kb), "%u/%u/%u/%u/%u/%u/%d/%zu/%zu/%d/%d|", nv, p.S, p.nb_s, p.nb_m, p.nb_r, p.nb_sh, b->raster_bps,
+             p.n_px, p.n_smap, (int)p.fast, (int)p.lines);
     p.key = kb;
     // every pointer the captured launches take as an argument
     const void* args[] = {b->cnt.p, b->keys.p, b->nanseq.p, b->beaten.p, b->chunk.p, b->smaps.p, b->h_cnt,
@@ -2031,9 +2040,9 @@ int batch_launch(Batch* b, const BatchPlan& p, uint32_t* launches) {
     KTRY(prk::launch_raster_batch(b->d_fj.p, b->d_fitems.p, (int)V, b->d_queue.p + 1, b->n_sms * b->raster_bps, st));
     KTRY(prk::launch_resolve_batch(b->d_res.p, blk_r, (int)V, p.nb_r, st));
     KTRY(prk::launch_shade_batch(b->d_sh.p, blk_sh, (int)V, p.nb_sh, p.fast, st));
-    KTRY(prk::launch_ao_linemax_batch(b->d_ao.p, blk_sh, (int)V, p.nb_sh, st));
-    KTRY(prk::launch_ao_batch(b->d_ao.p, (int)V, b->chunk.p, b->n_sms * 4, st));
-    n += 11;
+    if (p.lines) KTRY(prk::launch_ao_linemax_batch(b->d_ao.p, blk_sh, (int)V, p.nb_sh, st));
+    KTRY(prk::launch_ao_batch(b->d_ao.p, (int)V, b->chunk.p, b->n_sms * 4, p.lines, st));
+    n += p.lines ? 11 : 10;
     CUDA_TRY(cudaMemcpyAsync(b->h_cnt, b->cnt.p, sizeof(prk::Counters) * (V + S), cudaMemcpyDeviceToHost, st));
     *launches = n;
     return PR_OK;

@@ -2728,12 +2728,13 @@ __device__ __noinline__ float ao_total_taps(const AoParams& P, uint32_t i, const
 // Pixel j of the AO list's n (every lane of a warp calls, those past the end
 // with the last pixel and nothing to write): its total T, then (kApply) the
 // colour scaling, or (!kApply) T stored for ao_apply_kernel.
-template <bool kApply>
+// kLines: the frame has line maxima.
+template <bool kApply, bool kLines>
 PR_DEV void ao_one(const AoParams& P, uint32_t j, uint32_t n, const AoTables& S) {
     const bool mine = j < n;
     const uint32_t i = P.list[min(j, n - 1u)];
     float T;
-    if (P.cnt->nan_flag != 0u || !P.linemax) {  // some NaN-depth fragment reached this frame (the raster flags every one)
+    if (!kLines || P.cnt->nan_flag != 0u) {  // some NaN-depth fragment reached this frame (the raster flags every one)
         T = ao_total_taps(P, i, S);
     } else {
         const int W = P.W, H = P.H, r = (int)(i / (uint32_t)W), x = (int)i - r * W, y = H - 1 - r;
@@ -2814,6 +2815,7 @@ PR_DEV void ao_finish(const AoParams& P, uint32_t i, float T) {
 // instructions. Bound by issue (71% active): 713k pixels at 1920x1080 take
 // 206 us and 160 M warp instructions; every tap compared by itself, eight to
 // a unit, took 286 us and 227 M.
+template <bool kLines>
 __global__ void __launch_bounds__(kAoThreads, 4) ao_kernel(const __grid_constant__ AoParams P) {
     __shared__ AoTables S;
     const uint32_t n = P.cnt->n_ao;
@@ -2823,7 +2825,7 @@ __global__ void __launch_bounds__(kAoThreads, 4) ao_kernel(const __grid_constant
         reinterpret_cast<uint4*>(&S)[e] = reinterpret_cast<const uint4*>(P.tables)[e];
     __syncthreads();
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x)
-        ao_one<false>(P, base + threadIdx.x, n, S);
+        ao_one<false, kLines>(P, base + threadIdx.x, n, S);
 }
 // The tap tables of a frame size, once per context and size.
 __global__ void __launch_bounds__(kAoThreads) ao_tables_kernel(const __grid_constant__ AoParams P, void* out) {
@@ -2989,7 +2991,7 @@ __global__ void __launch_bounds__(256) shade_batch_kernel(const ShadeParams* vie
 __global__ void __launch_bounds__(256) ao_linemax_batch_kernel(const AoParams* views, const uint32_t* blk, int n_views) {
     const int v = job_of(blk, n_views, blockIdx.x);
     const AoParams& P = views[v];
-    if (!P.linemax || P.cnt->nan_flag || P.cnt->n_ao == 0) return;
+    if (P.cnt->nan_flag || P.cnt->n_ao == 0) return;
     const uint32_t b = blockIdx.x - blk[v], tiles_x = (uint32_t)(P.W + 31) / 32u;
     const uint32_t ty = b / tiles_x;
     ao_linemax_tile(P.W, P.H, (int)((b - ty * tiles_x) * 32u), (int)(ty * 8u), P.linemax,
@@ -2998,6 +3000,8 @@ __global__ void __launch_bounds__(256) ao_linemax_batch_kernel(const AoParams* v
 
 // Persistent AO over every view's list, in chunks of one block taken from
 // per-view counters; tap tables rebuilt when the frame size changes.
+// kLines: the batch has line maxima.
+template <bool kLines>
 __global__ void __launch_bounds__(kAoThreads) ao_batch_kernel(const AoParams* views, int n_views,
                                                                 uint32_t* chunk_ctr) {
     __shared__ AoTables S;
@@ -3022,7 +3026,7 @@ __global__ void __launch_bounds__(kAoThreads) ao_batch_kernel(const AoParams* vi
             const uint32_t c = s_chunk;
             __syncthreads();
             if (c * blockDim.x >= n) break;
-            ao_one<true>(P, c * blockDim.x + threadIdx.x, n, S);
+            ao_one<true, kLines>(P, c * blockDim.x + threadIdx.x, n, S);
         }
     }
 }
@@ -3177,9 +3181,9 @@ int launch_shade_batch(const ShadeParams* views, const uint32_t* blk, int n_view
         shade_batch_kernel<false><<<n_blocks, 256, 0, (cudaStream_t)stream>>>(views, blk, n_views);
     return check(cudaGetLastError());
 }
-int launch_ao_batch(const AoParams* views, int n_views, uint32_t* chunk_ctr, int n_blocks, void* stream) {
-    ao_batch_kernel<<<n_blocks, kAoThreads, 0, (cudaStream_t)stream>>>(views, n_views, chunk_ctr);
-    return check(cudaGetLastError());
+int launch_ao_batch(const AoParams* views, int n_views, uint32_t* chunk_ctr, int n_blocks, bool lines, void* stream) {
+    return launch(false, lines ? ao_batch_kernel<true> : ao_batch_kernel<false>, (unsigned)n_blocks, kAoThreads, stream, views,
+                  n_views, chunk_ctr);
 }
 // ---------------------------------------------------------------- MSAA resize
 
@@ -3298,8 +3302,8 @@ int launch_ao_T(const AoParams& p, void* stream) {
     // list's length exit at once.
     const size_t n = (size_t)p.W * p.H;
     if (n == 0) return 0;
-    ao_kernel<<<(unsigned)((n + kAoThreads - 1) / kAoThreads), kAoThreads, 0, (cudaStream_t)stream>>>(p);
-    return check(cudaGetLastError());
+    const unsigned nb = (unsigned)((n + kAoThreads - 1) / kAoThreads);
+    return launch(false, p.linemax ? ao_kernel<true> : ao_kernel<false>, nb, kAoThreads, stream, p);
 }
 int launch_ao_apply(const AoParams& p, int n_blocks, void* stream) {
     return launch(false, ao_apply_kernel, (unsigned)n_blocks, 256, stream, p);

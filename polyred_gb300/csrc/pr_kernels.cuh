@@ -318,8 +318,8 @@ int launch_resolve_batch(const ResolveParams* jobs, const uint32_t* blk, int n_j
 // fast: every view is shade_is_fast
 int launch_shade_batch(const ShadeParams* views, const uint32_t* blk, int n_views, uint32_t n_blocks, bool fast, void* stream);
 int launch_ao_linemax_batch(const AoParams* views, const uint32_t* blk, int n_views, uint32_t n_blocks, void* stream);
-// Persistent; chunk counters [n_views] zeroed by the caller.
-int launch_ao_batch(const AoParams* views, int n_views, uint32_t* chunk_ctr, int n_blocks, void* stream);
+// Persistent; chunk counters [n_views] zeroed by the caller. lines: every view's linemax is set (else none is).
+int launch_ao_batch(const AoParams* views, int n_views, uint32_t* chunk_ctr, int n_blocks, bool lines, void* stream);
 int launch_col_to_float(const uchar4* col, float4* out, size_t n, void* stream);
 int launch_fill_u32(uint32_t* p, uint32_t v, size_t n, void* stream);
 // Triangle.IsValid (kTriValid) and the AO flag of each triangle's material (kTriAO).
