@@ -553,14 +553,17 @@ PR_DEV void emit_run(const SetupParams& P, uint2* list, uint32_t cap, uint32_t o
 // the pixel tests' issue): raster 8.7 -> 4.2 ms, and the clip kernel no longer
 // writes a ground plane's tasks by the ten thousand (1080p: 45 -> 24 us). From
 // 1024 pixels on, a sphere of 2000-pixel boxes rastered in 18 us, from 4096 in 15.
+// A box under five pixels wide or high keeps its small tasks: from five on, w h
+// >= 4096 makes (w + 31)(h + 31) / 1024 blocks at most a quarter of w h / 32
+// tasks, which is the room they have; a frame that cannot grow its lists must
+// not need more than before.
 constexpr uint32_t kBigArea = 4096;
-PR_DEV bool is_big(const SetupParams& P, uint32_t area) { return area >= kBigArea && P.cap_big != 0u; }
-PR_DEV uint32_t small_tasks(const SetupParams& P, uint32_t area) {
-    return is_big(P, area) ? 0u : n_tasks_of(area, P.task_shift);
+PR_DEV bool is_big(const SetupParams& P, const PixBox& pb) {
+    if (pb.area < kBigArea || P.cap_big == 0u) return false;
+    return min((pb.bx >> 16) - (pb.bx & 0xffffu), (pb.by >> 16) - (pb.by & 0xffffu)) >= 4u;
 }
 // The block tasks of this lane's record, if it is a large one; all lanes call.
-PR_DEV void emit_blocks(const SetupParams& P, uint32_t ridx, const PixBox& pb) {
-    const bool big = is_big(P, pb.area);
+PR_DEV void emit_blocks(const SetupParams& P, uint32_t ridx, const PixBox& pb, bool big) {
     if (!__any_sync(0xffffffffu, big)) return;
     const uint32_t n = big ? (((pb.bx >> 16) - (pb.bx & 0xffffu) + 32u) >> 5) * (((pb.by >> 16) - (pb.by & 0xffffu) + 32u) >> 5) : 0u;
     uint32_t tot;
@@ -759,7 +762,8 @@ PR_DEV void setup_main_one(const SetupParams& P, const ObjCache* C, uint32_t t, 
     PixBox pb = {0u, 0u, 0u};
     if (emit) pb = pixel_box(box, v[0].pos, v[1].pos, v[2].pos, sabc, P.W, P.H);
     uint32_t ridx, o;
-    const uint32_t nt = small_tasks(P, pb.area);
+    const bool big = is_big(P, pb);
+    const uint32_t nt = big ? 0u : n_tasks_of(pb.area, P.task_shift);
     block_reserve(P, S, emit ? 1u : 0u, nt, &ridx, &o);
     if (emit) {
         if (ridx >= P.cap_rec) {
@@ -771,7 +775,7 @@ PR_DEV void setup_main_one(const SetupParams& P, const ObjCache* C, uint32_t t, 
         }
     }
     emit_run(P, P.tasks, P.cap_tasks, o, 1u, ridx, nt);
-    emit_blocks(P, ridx, pb);
+    emit_blocks(P, ridx, pb, big);
 }
 // 8 blocks per SM (64 registers, a few spilled on rare paths): more warps to
 // hide the per-triangle loads and stores measured faster than 80 registers at 6.
@@ -885,10 +889,11 @@ PR_DEV void clip_one_group(const SetupParams& P, const uint32_t* clip_list, uint
             write_sub(P, ridx, t * 8u + sub, s3, recipw, matid, sabc, pb, attrs ? mw : nullptr);
         }
     }
-    const uint32_t nt = small_tasks(P, pb.area);
+    const bool big = is_big(P, pb);
+    const uint32_t nt = big ? 0u : n_tasks_of(pb.area, P.task_shift);
     const uint32_t o = warp_reserve(&P.cnt->n_tasks, nt, &tot);
     emit_run(P, P.tasks, P.cap_tasks, o, 1u, ridx, nt);
-    emit_blocks(P, ridx, pb);
+    emit_blocks(P, ridx, pb, big);
 }
 __global__ void __launch_bounds__(128) clip_kernel(const __grid_constant__ SetupParams P, const uint32_t* clip_list) {
     after_previous();
@@ -942,14 +947,15 @@ PR_DEV void setup_shadow_one(const SetupParams& P, const ObjCache* C, uint32_t t
     PixBox pb = {0u, 0u, 0u};
     if (ok) pb = pixel_box(box, v[0].pos, v[1].pos, v[2].pos, sabc, P.W, P.H);
     uint32_t none, o;
-    const uint32_t nt = small_tasks(P, pb.area);
+    const bool big = is_big(P, pb);
+    const uint32_t nt = big ? 0u : n_tasks_of(pb.area, P.task_shift);
     block_reserve(P, S, 0u, nt, &none, &o);
     if (ok) {
         const float rw[3] = {1, 1, 1};
         write_sub(P, t, t, v, rw, -1, sabc, pb);
     }
     emit_run(P, P.tasks, P.cap_tasks, o, 1u, t, nt);
-    emit_blocks(P, t, pb);
+    emit_blocks(P, t, pb, big);
 }
 // 9 blocks per SM (56 registers): more warps than at 62 registers and 8.
 __global__ void __launch_bounds__(128, 9) setup_shadow_kernel(const __grid_constant__ SetupParams P) {
