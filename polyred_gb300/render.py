@@ -14,6 +14,7 @@ Usage::
 """
 import collections
 import ctypes as C
+import math
 import weakref
 
 import numpy as np
@@ -270,38 +271,70 @@ def host_array(shape, dtype):
     return a
 
 
+def _nbytes(shape, dtype):
+    return math.prod(map(int, shape)) * np.dtype(dtype).itemsize
+
+
 class _Spare:
     """Host memory of one renderer's images, used again once the program has
     dropped them. A fresh 1.6 MB array is fresh pages, and the faults of three
-    took longer than a frame of 800x500 (Render(): 1300 -> 230 us). An array is
-    handed out over a buffer of its own; when its last view goes, the buffer
-    comes back, at most `keep` of a size stay, and they go with the renderer.
+    took longer than a frame of 800x500: a program that keeps one renderer and
+    drops its images waits 230 us for Render() instead of 1300; one that keeps
+    every image gains nothing. An array is handed out over a buffer of its own;
+    when its last view goes, the buffer comes back. At most the last frame's
+    images stay, and they go with the renderer; a renderer without a buffer
+    takes another's idle one, which the allocator would have had without this.
     Plain memory: it survives a fork, as the arrays before did. deque's append
     and pop are atomic, and the callback that returns a buffer may run on any
     thread, inside a collection, so there is no lock to hold."""
 
+    _live = {}  # id: weak reference, of every pool
+
     def __init__(self, keep):
-        self.keep = keep
-        self.free = {}
+        self.keep = keep  # buffers of a size, where only() is not told how many
+        self.count, self.free = {}, {}
+        me = id(self)
+        self._live[me] = weakref.ref(self, lambda _, live=self._live: live.pop(me, None))
 
     def _give(self, n, buf):
         q = self.free.get(n)
-        if q is not None and len(q) < self.keep:
-            q.append(buf)
+        if q is not None:
+            q.append(buf)  # the oldest of a full deque goes
 
     def only(self, sizes):
-        """Forget the sizes that the next frame does not ask for."""
-        self.free = {n: self.free.get(n) or collections.deque() for n in sizes}
+        """Forget the sizes that the next frame does not ask for. sizes: how
+        many of each it asks for, or just the sizes."""
+        count = sizes if isinstance(sizes, dict) else dict.fromkeys(sizes, self.keep)
+        if count == self.count:
+            return
+        free = {}
+        for n, k in count.items():
+            q = self.free.get(n)
+            if q is None or q.maxlen != k:
+                old, q = q, collections.deque(maxlen=k)
+                while old:  # emptied by pops: another thread may return a buffer meanwhile
+                    q.append(old.pop())
+            free[n] = q
+        self.count, self.free = count, free
+
+    def _take(self, n):
+        try:
+            return self.free[n].pop()
+        except (KeyError, IndexError):
+            pass
+        for ref in list(self._live.values()):
+            try:
+                return ref().free[n].pop()
+            except (AttributeError, KeyError, IndexError):  # gone, other sizes, none idle
+                pass
+        return np.empty(n, np.uint8)
 
     def array(self, shape, dtype):
         """An array that the caller overwrites whole."""
-        n = int(np.prod(shape)) * np.dtype(dtype).itemsize
+        n = _nbytes(shape, dtype)
         if n == 0:
             return np.zeros(shape, dtype)
-        try:
-            buf = self.free[n].pop()
-        except (KeyError, IndexError):
-            buf = np.empty(n, np.uint8)
+        buf = self._take(n)
         lease = (C.c_uint8 * n).from_buffer(buf)
         weakref.finalize(lease, self._give, n, buf).atexit = False
         return np.frombuffer(lease, dtype).reshape(shape)
@@ -337,7 +370,11 @@ class Outputs:
                 h, w = (height, width) if name == "rgba" else (height * msaa, width * msaa)
                 form[name] = (h, w, k) if k > 1 else (h, w), dt
         if spare is not None:
-            spare.only({int(np.prod(shape)) * np.dtype(dt).itemsize for shape, dt in form.values()})
+            sizes = {}
+            for shape, dt in form.values():
+                n = _nbytes(shape, dt)
+                sizes[n] = sizes.get(n, 0) + 1
+            spare.only(sizes)
         for name, (shape, dt) in form.items():
             written = name != "shadow_maps" or n_shadow > 0
             a = (spare.array if spare is not None and written else alloc)(shape, dt)
