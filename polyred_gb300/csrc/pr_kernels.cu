@@ -3593,8 +3593,9 @@ extern "C" int pr_depth_map_noalloc(const pr_depth_map_desc* d) {
     if (e != cudaSuccess) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: scratch initialisation failed");
     float* obj_trans = (float*)(base + kNaObjTrans);
     uint32_t* blk_obj = (uint32_t*)(base + kNaBlkObj);
-    noalloc_init_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d->depth, keys, lastnan, n, cnt, obj_first, obj_trans,
-                                                                  blk_obj, d->n_tris, O);
+    int rc = launch(false, noalloc_init_kernel, (unsigned)((n + 255) / 256), 256, st, d->depth, keys, lastnan, n, cnt, obj_first,
+                    obj_trans, blk_obj, d->n_tris, O);
+    if (rc) return err(PR_ERR_CUDA, "pr_depth_map_noalloc: scratch initialisation failed");
 
     SetupParams sp{};
     sp.pos = (const float4*)d->pos;
@@ -3636,8 +3637,8 @@ extern "C" int pr_depth_map_noalloc(const pr_depth_map_desc* d) {
         return long_map ? launch(false, long_map_raster_kernel, (unsigned)sm_count() * 8u, 256, st, rp, d->n_tris)
                         : launch_raster(rp, sm_count() * 8, st);
     };
-    int rc = !long_map ? launch_setup_shadow(sp, st)
-                       : d->n_tris ? launch(false, long_map_setup_kernel, (d->n_tris + 127u) / 128u, 128, st, sp) : 0;
+    rc = !long_map ? launch_setup_shadow(sp, st)
+                   : d->n_tris ? launch(false, long_map_setup_kernel, (d->n_tris + 127u) / 128u, 128, st, sp) : 0;
     if (!rc) rc = raster(kShadow, &cnt->take[0]);
     if (!rc) rc = launch_shadow_fixup_reset(d->width, d->height, lastnan, keys, cnt, st);
     if (!rc) rc = raster(kShadowFixup, &cnt->take[1]);

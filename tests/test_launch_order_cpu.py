@@ -1,8 +1,9 @@
-"""What a programmatic launch leaves to the kernel: every kernel launched so
+"""What a launch leaves to the code. Programmatic ones: every kernel launched so
 waits for its predecessor before it reads, a kernel that releases its successor
 has waited itself, and the raster that clip_kernel releases finds setup's writes
 by an acquire of the word that clip_kernel stored with release before releasing
-it, else it waits. Read from the source: the order has no other trace."""
+it, else it waits. Any: its error is read. Read from the source: neither has
+another trace."""
 import os
 import re
 
@@ -48,3 +49,12 @@ def test_the_raster_behind_clipping_acquires_what_clipping_published():
     at = raster.index("if (!published(&P.cnt->set_up)) after_previous();")
     assert at < raster.index("__syncthreads()") < raster.index("c->n_tasks")
     assert "st.release.gpu" in SRC and "ld.acquire.gpu" in SRC
+
+
+def test_every_launch_is_checked():
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith(".cu"):
+            src = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+            for m in re.finditer(r"<<<", src):
+                after = src[m.end():m.end() + 500].split("return ", 1)[1]
+                assert after.startswith("check(cudaGetLastError())"), (name, src[m.start() - 60:m.end()])
