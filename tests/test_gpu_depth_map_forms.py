@@ -1,6 +1,7 @@
 """pr_depth_map_noalloc against the oracle's drawDepth: vertices so far out that
 the reference's int64 pixel bounds overflow; maps up to 2^20 texels long, whose
-corners do not fit 16 bits."""
+corners do not fit 16 bits; as many objects as travel with the launch, one more,
+and the most."""
 import ctypes as C
 
 import numpy as np
@@ -111,3 +112,19 @@ def test_long_map_overflow_leaves_the_map_unchanged(native_lib):
         rc, got = device_map(native_lib, flat, 131072, 8, view, proj, init)
         same = np.array_equal(got.view(np.uint32), init.view(np.uint32))
         assert (rc, same) == ((_abi.PR_OK, False) if ok else (_abi.PR_ERR_OVERFLOW, True))
+
+
+@pytest.mark.parametrize("w,h", [(200, 120), (70000, 9)])
+@pytest.mark.parametrize("n", [31, 32, 33, 256])
+def test_objects(native_lib, n, w, h):
+    """Objects of 0 to 3 hundred triangles (several to a block of 128, and more than a block) with models of their own."""
+    g = np.random.default_rng(n)
+    counts = g.choice([0, 2, 14, 130, 300], n, p=[0.2, 0.4, 0.3, 0.07, 0.03])
+    counts[[0, -1]] = 2
+    parts, tris = [], []
+    for c in counts:
+        parts.append((int(c), tuple(g.uniform(-1.5, 1.5, 3))))
+        at = g.uniform(-0.3, 0.3, (c // 2, 1, 3)) + g.normal(0, 0.15, (c // 2, 3, 3))
+        tris.append(both_windings(at))
+    want = check(native_lib, _soup(np.concatenate(tris)), w, h, [p for p in parts])
+    assert (want != 0).sum() > 0.05 * w * h
