@@ -215,7 +215,7 @@ struct Ctx {
     // submitted frames: scene uploads and host-output copies on their own streams
     cudaStream_t stream_u = nullptr, stream_d = nullptr;
     cudaEvent_t ev_frame = nullptr, ev_d2h = nullptr;
-    bool submitted = false;  // ev_d2h has been recorded
+    bool submitted = false;  // ev_d2h has been recorded, and the host has not waited for it since
     // raster work space
     DevBuf<prk::RasterRec> rrec;
     DevBuf<prk::AttrRec> arec;
@@ -1074,6 +1074,7 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             return PR_OK;
         }
         CUDA_TRY(cudaStreamSynchronize(st));
+        c->submitted = false;  // shading waited for ev_d2h, the host for shading
         // capacity check
         uint32_t ov = 0, need_rec = 0, need_tasks = 0;
         for (int k = 0; k < prk::kNumCounters; k++) {
@@ -1261,6 +1262,7 @@ int pr_scene_upload(void* ctx, const pr_scene_desc* s) {
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream_u));
     CUDA_TRY(cudaStreamSynchronize(c->stream_d));
+    c->submitted = false;
     clear_stale_error();
     c->has_scene = false;  // until the new scene is complete (a failed upload leaves none)
     const MayYield yield(c->linemax);

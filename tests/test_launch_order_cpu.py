@@ -58,3 +58,12 @@ def test_every_launch_is_checked():
             for m in re.finditer(r"<<<", src):
                 after = src[m.end():m.end() + 500].split("return ", 1)[1]
                 assert after.startswith("check(cudaGetLastError())"), (name, src[m.start() - 60:m.end()])
+
+
+def test_the_wait_for_submitted_outputs_ends():
+    """A context that has submitted a frame waits for its outputs' copies until the host has waited itself."""
+    api = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "pr_api.cpp")).read())
+    frame = api[api.index("int render_impl("):]
+    assert frame.index("cudaStreamWaitEvent(st, c->ev_d2h, 0)") < frame.index("cudaStreamSynchronize(st)") < frame.index("c->submitted = false;")
+    upload = api[api.index("int pr_scene_upload("):]
+    assert upload.index("cudaStreamSynchronize(c->stream_d)") < upload.index("c->submitted = false;") < upload.index("scene_fill(")
