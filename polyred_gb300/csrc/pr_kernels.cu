@@ -1746,19 +1746,19 @@ static __device__ __noinline__ uint32_t texture_exact(const prt::TexDesc* td, co
     return prt::tex_query(*td, texels, prt::tex_lod(*td, du, dv), u, v);
 }
 
-// Four channels as floats. Truncation of v in [0, 2^23) is v + 2^23 rounded down.
+// Four channels as floats. trunc_pos: truncation of v in [0, 2^23), as v + 2^23 rounded down.
 struct Rgba {
     float c[4];
 };
 PR_DEV Rgba unpack_rgba(uint32_t t) {
     return {{small_u2f(t & 0xffu), small_u2f((t >> 8) & 0xffu), small_u2f((t >> 16) & 0xffu), small_u2f(t >> 24)}};
 }
-PR_DEV float trunc_small(float v) { return __fsub_rn(__fadd_rz(v, 8388608.0f), 8388608.0f); }
+PR_DEV float trunc_pos(float v) { return __fsub_rn(__fadd_rz(v, 8388608.0f), 8388608.0f); }
 // lerpc in floats: the channels are 0 .. 255 and t is in [0, 1), so uint8() only truncates.
 PR_DEV Rgba lerp_rgba(const Rgba& a, const Rgba& b, float t) {
     Rgba r;
 #pragma unroll
-    for (int k = 0; k < 4; k++) r.c[k] = trunc_small(__fadd_rn(a.c[k], __fmul_rn(t, __fsub_rn(b.c[k], a.c[k]))));
+    for (int k = 0; k < 4; k++) r.c[k] = trunc_pos(__fadd_rn(a.c[k], __fmul_rn(t, __fsub_rn(b.c[k], a.c[k]))));
     return r;
 }
 // queryBilinear for finite u, v in [0, 2): the same products, floors and
@@ -1825,7 +1825,7 @@ PR_DEV uint32_t texture_colour(const prt::TexDesc* td, const uint32_t* texels, f
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float ab = __fsub_rn(b.c[k], a.c[k]), m = __fmaf_rn(p, ab, a.c[k]), e = __fmaf_rn(fabsf(ab), d, 6.5e-5f);
-            const float lo = trunc_small(fmaxf(__fsub_rn(m, e), 0.0f)), hi = trunc_small(__fadd_rn(m, e));
+            const float lo = trunc_pos(fmaxf(__fsub_rn(m, e), 0.0f)), hi = trunc_pos(__fadd_rn(m, e));
             ok = ok && (lo == hi || ab == 0.0f);
             c.c[k] = ab == 0.0f ? a.c[k] : hi;
         }

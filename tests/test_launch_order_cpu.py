@@ -67,3 +67,13 @@ def test_the_wait_for_submitted_outputs_ends():
     assert frame.index("cudaStreamWaitEvent(st, c->ev_d2h, 0)") < frame.index("cudaStreamSynchronize(st)") < frame.index("c->submitted = false;")
     upload = api[api.index("int pr_scene_upload("):]
     assert upload.index("cudaStreamSynchronize(c->stream_d)") < upload.index("c->submitted = false;") < upload.index("scene_fill(")
+
+
+def test_device_functions_hide_none_of_the_header():
+    """A function of pr_kernels.cu with the name of one of pr_devmath.cuh would take its calls from that line on."""
+    def names(src):
+        return set(re.findall(r"PR_DEV [\w:<>*& ]+?(\w+)\(", src))
+    header = names(re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "pr_devmath.cuh")).read()))
+    own = names(SRC)
+    assert len(header) > 20 and len(own) > 60
+    assert not header & own, header & own
