@@ -32,6 +32,12 @@ int64_t pr_testing_alloc_count(void);
  * in (-1/99, 0). Returns the number of directions or a negative status. */
 int pr_debug_ao_dirs(int W, int H, float* cosv, float* sinv, int8_t* fast, int8_t* tiny);
 
+/* The shadow lookup's single transform (host only, no device) of a light's
+ * view and projection and a width x height map: rows x, y, z of the matrix and
+ * of its error bound per |p| (12 floats each). Returns 1 when lookups use it,
+ * 0 when they take the three transforms, or a negative status. */
+int pr_debug_shadow_composite(const float* view, const float* proj, int width, int height, float* smap, float* serr);
+
 /* Device arithmetic probes (one thread per element, n device-resident
  * elements; synchronous): */
 /* the shade kernel's float32 Pow beside the float64 algorithm */

@@ -7,7 +7,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdarg>
-#include <cmath>
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
@@ -631,39 +630,9 @@ void fill_shade_frame(const Ctx* c, const pr_frame_desc* f, const M4& s2w, int S
     std::memcpy(sp.s2w, s2w.m, 64);
     M4 svp = prh::viewport((float)SW, (float)SH);
     std::memcpy(sp.shadow_vp, svp.m, 64);
-    auto unit_bottom = [](const float* m) { return m[12] == 0.0f && m[13] == 0.0f && m[14] == 0.0f && m[15] == 1.0f; };
     for (uint32_t l = 0; l < f->n_lights; l++) {
         prk::LightK& K = sp.lights[l];
-        K.sfast = unit_bottom(K.lview) && unit_bottom(K.lproj) && unit_bottom(svp.m) ? 1 : 0;
-        // The reference's three Applies (four roundings a row and step) stay
-        // within 12.01 u |Vp||P||V||p| of the product's exact value (u = 2^-24,
-        // double rounding included), smap rounded to float32 and applied by
-        // float32 FMAs within 5.01 u of the same.
-        double m[16], a[16], m2[16], a2[16];
-        auto mul = [](const double* p, const double* q, double* r) {
-            for (int i = 0; i < 4; i++)
-                for (int j = 0; j < 4; j++) {
-                    r[i * 4 + j] = 0;
-                    for (int k = 0; k < 4; k++) r[i * 4 + j] += p[i * 4 + k] * q[k * 4 + j];
-                }
-        };
-        double v[16], p[16], s[16], va[16], pa[16], sa[16];
-        for (int e = 0; e < 16; e++) {
-            v[e] = K.lview[e];
-            p[e] = K.lproj[e];
-            s[e] = svp.m[e];
-            va[e] = std::fabs(v[e]);
-            pa[e] = std::fabs(p[e]);
-            sa[e] = std::fabs(s[e]);
-        }
-        mul(p, v, m);
-        mul(s, m, m2);
-        mul(pa, va, a);
-        mul(sa, a, a2);
-        for (int e = 0; e < 12; e++) {
-            K.smap[e] = (float)m2[e];
-            K.serr[e] = (float)(a2[e] * (17.5 * 5.9604644775390625e-08));  // 17.5 u: float32's own rounding included
-        }
+        K.sfast = prh::shadow_composite(K.lview, K.lproj, svp.m, K.smap, K.serr) ? 1 : 0;
     }
     sp.SW = SW;
     sp.SH = SH;
@@ -1431,6 +1400,12 @@ int pr_debug_ao_dirs(int W, int H, float* cosv, float* sinv, int8_t* fast, int8_
     prh::ao_directions(cosv, sinv, &n);
     prh::ao_classify(cosv, sinv, n, W, H, fast, tiny);
     return n;
+}
+
+int pr_debug_shadow_composite(const float* view, const float* proj, int width, int height, float* smap, float* serr) {
+    if (!view || !proj || !smap || !serr) return fail(PR_ERR_INVALID_ARG, "pr_debug_shadow_composite: NULL argument");
+    if (width <= 0 || height <= 0) return fail(PR_ERR_INVALID_ARG, "pr_debug_shadow_composite: bad map size");
+    return prh::shadow_composite(view, proj, prh::viewport((float)width, (float)height).m, smap, serr) ? 1 : 0;
 }
 
 int pr_host_free(void* ptr) {

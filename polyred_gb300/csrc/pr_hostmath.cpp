@@ -313,4 +313,37 @@ float ao_classify(const float cosv[8], const float sinv[8], int n, int W, int H,
     return h;
 }
 
+bool shadow_composite(const float* view, const float* proj, const float* vp, float smap[12], float serr[12]) {
+    // The reference's three Applies (four roundings a row and step) stay
+    // within 12.01 u |Vp||P||V||p| of the product's exact value (u = 2^-24,
+    // double rounding included), smap rounded to float32 and applied by
+    // float32 FMAs within 5.01 u of the same.
+    auto mul = [](const double* p, const double* q, double* r) {
+        for (int i = 0; i < 4; i++)
+            for (int j = 0; j < 4; j++) {
+                r[i * 4 + j] = 0;
+                for (int k = 0; k < 4; k++) r[i * 4 + j] += p[i * 4 + k] * q[k * 4 + j];
+            }
+    };
+    double v[16], p[16], s[16], va[16], pa[16], sa[16], m[16], a[16], m2[16], a2[16];
+    for (int e = 0; e < 16; e++) {
+        v[e] = view[e];
+        p[e] = proj[e];
+        s[e] = vp[e];
+        va[e] = std::fabs(v[e]);
+        pa[e] = std::fabs(p[e]);
+        sa[e] = std::fabs(s[e]);
+    }
+    mul(p, v, m);
+    mul(s, m, m2);
+    mul(pa, va, a);
+    mul(sa, a, a2);
+    for (int e = 0; e < 12; e++) {
+        smap[e] = (float)m2[e];
+        serr[e] = (float)(a2[e] * (17.5 * 5.9604644775390625e-08));  // 17.5 u: float32's own rounding included
+    }
+    auto unit_bottom = [](const float* q) { return q[12] == 0.0f && q[13] == 0.0f && q[14] == 0.0f && q[15] == 1.0f; };
+    return unit_bottom(view) && unit_bottom(proj) && unit_bottom(vp);
+}
+
 }  // namespace prh

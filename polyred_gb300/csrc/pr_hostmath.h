@@ -28,5 +28,10 @@ void ao_directions(float cosv[8], float sinv[8], int* n); // material/ao.go:28
 // Returns half an ulp of float32 at max(W, H) + 100, which bounds the
 // rounding of every tap coordinate.
 float ao_classify(const float cosv[8], const float sinv[8], int n, int W, int H, int8_t fast[8], int8_t tiny[8]);
+// The shadow lookup's single transform: rows x, y, z of smap = vp * proj * view
+// in float32, and of serr, a bound per |p| on smap * p by float32 FMAs against
+// the reference's three Applies (render/shadow.go:244-246). False: a bottom row
+// is not (0, 0, 0, 1), and w changes on the way.
+bool shadow_composite(const float* view, const float* proj, const float* vp, float smap[12], float serr[12]);
 
 }  // namespace prh
