@@ -154,6 +154,10 @@ struct RasterParams {
     uint32_t* take2 = nullptr;
 };
 
+// What shading reads. Of a scene only its materials and images: a submitted
+// frame's triangle arrays (positions, normals, uv, colours, material ids, flags)
+// are overwritten by the next upload once the attributes are written, while
+// shading may still run (SceneBufs::ev_geometry).
 struct ShadeParams {
     int W, H;
     uint32_t flags;             // PR_FRAME_*
