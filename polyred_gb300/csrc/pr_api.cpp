@@ -226,10 +226,11 @@ struct Ctx {
     int W = 0, H = 0;
     DevBuf<float> obj_trans;  // [1 + lights][n_objects][16]: Proj·View·Model per pass and object
     DevBuf<unsigned long long> keys;
-    DevBuf<uint32_t> nanseq, beaten, win;
+    DevBuf<uint32_t> nanseq, beaten;
     bool nan_in_use = false;  // a frame's raster was queued, but not the resolve that puts nanseq and beaten back
-    DevBuf<float> depth_ao;
-    DevBuf<uint32_t> ao_list;
+    DevBuf<uint32_t> pix;  // one allocation (a context's first frame waits for each); in it:
+    uint32_t *win = nullptr, *ao_list = nullptr;
+    float* depth_ao = nullptr;
     int n_ao_dirs = 0;
     float ao_cos[8] = {}, ao_sin[8] = {};
     // shadow maps (persistent across frames)
@@ -264,8 +265,8 @@ struct Ctx {
     bool ao_marched = false;  // the last frame ran the AO march (ev_ao0, ev_ao hold it)
     DevBuf<float> ao_T;
     DevBuf<float> linemax;  // [4][H][W], AO's line maxima; empty without memory for them
-    DevBuf<uint8_t> gamma;   // GammaCorrection's table (prh::gamma_table)
-    DevBuf<uint8_t> ao_tab;  // AO's tap tables for frames of width ao_tab_w and rounding ao_tab_ulp
+    DevBuf<uint8_t> tables;  // GammaCorrection's table (prh::gamma_table, 256 B), then
+    uint8_t* ao_tab = nullptr;  // AO's tap tables for frames of width ao_tab_w and rounding ao_tab_ulp
     int ao_tab_w = 0;
     float ao_tab_ulp = 0.0f;
     int n_sms = 1;
@@ -447,9 +448,11 @@ int ensure_frame(Ctx* c, int W, int H) {
     if ((rc = c->beaten.ensure(n))) return rc;
     if (c->beaten.n != b0 || c->nan_in_use) CUDA_TRY(cudaMemsetAsync(c->beaten.p, 0, c->beaten.n * 4, c->stream));
     c->nan_in_use = false;
-    if ((rc = c->win.ensure(n))) return rc;
-    if ((rc = c->depth_ao.ensure(n))) return rc;
-    if ((rc = c->ao_list.ensure(n))) return rc;
+    const size_t plane = (n + 63) & ~(size_t)63;
+    if ((rc = c->pix.ensure(3 * plane))) return rc;
+    c->win = c->pix.p;
+    c->ao_list = c->pix.p + plane;
+    c->depth_ao = (float*)(c->pix.p + 2 * plane);
     c->W = W;
     c->H = H;
     return PR_OK;
@@ -636,7 +639,7 @@ void fill_shade_frame(const Ctx* c, const pr_frame_desc* f, const M4& s2w, int S
     }
     sp.SW = SW;
     sp.SH = SH;
-    sp.gamma = c->gamma.p;
+    sp.gamma = c->tables.p;
 }
 
 // Matrices of a frame (render/raster.go:232-246, 281-295).
@@ -926,34 +929,33 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
             if ((rc = c->ao_T.ensure(npx))) return rc;
             ensure_optional(c->linemax, 4 * npx);
         }
-        KTRY(prk::launch_resolve(W, H, c->keys.p, c->nanseq.p, c->beaten.p, dcnt, c->win.p, c->depth_ao.p, c->first_rec.p,
-                                 c->attr_state.p, c->sb.tri_flags.p, with_ao ? c->ao_list.p : nullptr, c->linemax.p, st));
+        KTRY(prk::launch_resolve(W, H, c->keys.p, c->nanseq.p, c->beaten.p, dcnt, c->win, c->depth_ao, c->first_rec.p,
+                                 c->attr_state.p, c->sb.tri_flags.p, with_ao ? c->ao_list : nullptr, c->linemax.p, st));
         c->nan_in_use = false;
         prk::AoParams ap{};
         cudaStream_t sc = c->stream_c;
         if (with_ao) {
             CUDA_TRY(cudaEventRecord(c->ev_resolved, st));
-            CUDA_TRY(cudaStreamWaitEvent(sc, c->ev_resolved, 0));
-            CUDA_TRY(cudaEventRecord(c->ev_ao0, sc));
             ap.W = W;
             ap.H = H;
             ap.gamma_on = (f->flags & PR_FRAME_GAMMA) ? 1 : 0;
             ap.n_dirs = c->n_ao_dirs;
             ap.ao_half_ulp = prh::ao_classify(c->ao_cos, c->ao_sin, c->n_ao_dirs, W, H, ap.dir_fast, ap.dir_tiny);
-            ap.depth = c->depth_ao.p;
-            ap.list = c->ao_list.p;
+            ap.depth = c->depth_ao;
+            ap.list = c->ao_list;
             ap.cnt = dcnt;
             ap.T = c->ao_T.p;
             ap.exact_T = dh ? 1 : 0;
             if (c->ao_tab_w != W || c->ao_tab_ulp != ap.ao_half_ulp) {
                 c->ao_tab_w = 0;
-                if ((rc = c->ao_tab.ensure(prk::ao_tables_bytes()))) return rc;
-                KTRY(prk::launch_ao_tables(ap, c->ao_tab.p, sc));
+                KTRY(prk::launch_ao_tables(ap, c->ao_tab, sc));
                 c->ao_tab_w = W;
                 c->ao_tab_ulp = ap.ao_half_ulp;
             }
-            ap.tables = c->ao_tab.p;
-            ap.linemax = c->linemax.p;  // here: an allocation since resolve may have taken their memory
+            CUDA_TRY(cudaStreamWaitEvent(sc, c->ev_resolved, 0));
+            CUDA_TRY(cudaEventRecord(c->ev_ao0, sc));
+            ap.tables = c->ao_tab;
+            ap.linemax = c->linemax.p;
             KTRY(prk::launch_ao_T(ap, sc));
             CUDA_TRY(cudaEventRecord(c->ev_ao, sc));
             launches += 1;
@@ -967,12 +969,12 @@ int render_impl(Ctx* c, const pr_frame_desc* f, pr_outputs* out, bool sync, cons
         if (!sp_owner) return fail(PR_ERR_OOM, "host allocation failed");
         prk::ShadeParams& sp = *sp_owner;
         fill_shade_frame(c, f, s2w, SW, SH, sp);
-        sp.win = c->win.p;
-        sp.depth_ao = c->depth_ao.p;
+        sp.win = c->win;
+        sp.depth_ao = c->depth_ao;
         sp.rrec = c->rrec.p;
         sp.arec = c->arec.p;
         sp.smaps = shadows ? c->smap.p : nullptr;
-        sp.ao_list = c->ao_list.p;
+        sp.ao_list = c->ao_list;
         sp.cnt_w = dcnt;
         if (dh) {
             sp.tri_scr = c->tri_scr.p;
@@ -1156,21 +1158,16 @@ int pr_create(int device, void** out_ctx) {
     }
     c->n_sms = prk::sm_count();
     {
-        prh::ao_directions(c->ao_cos, c->ao_sin, &c->n_ao_dirs);
-        int e = prk::set_ao_tables(c->ao_cos, c->ao_sin, c->n_ao_dirs, c->stream);
-        if (e) {
-            pr_destroy(c);
-            return fail(PR_ERR_CUDA, "AO table upload: %s", cudaGetErrorString((cudaError_t)e));
-        }
-    }
-    {
         uint8_t table[256];
         prh::gamma_table(table);
-        if ((rc = upload(c->gamma, table, 256, false, c->stream))) { pr_destroy(c); return rc; }
-        cudaError_t e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess) {
+        if ((rc = c->tables.ensure(256 + prk::ao_tables_bytes()))) { pr_destroy(c); return rc; }
+        c->ao_tab = c->tables.p + 256;
+        prh::ao_directions(c->ao_cos, c->ao_sin, &c->n_ao_dirs);
+        int e = (int)cudaMemcpyAsync(c->tables.p, table, 256, cudaMemcpyHostToDevice, c->stream);
+        if (!e) e = prk::set_ao_tables(c->ao_cos, c->ao_sin, c->n_ao_dirs, c->stream);  // waits for both copies
+        if (e) {
             pr_destroy(c);
-            return fail(PR_ERR_CUDA, "gamma table upload: %s", cudaGetErrorString(e));
+            return fail(PR_ERR_CUDA, "table upload: %s", cudaGetErrorString((cudaError_t)e));
         }
     }
     *out_ctx = c;
@@ -1192,8 +1189,7 @@ int pr_destroy(void* ctx) {
     if (c->stream_d) cudaStreamDestroy(c->stream_d);
     c->rrec.release(); c->arec.release(); c->tasks.release(); c->first_rec.release(); c->attr_state.release();
     c->clip_list.release();
-    c->keys.release(); c->nanseq.release(); c->beaten.release(); c->win.release(); c->depth_ao.release();
-    c->ao_list.release();
+    c->keys.release(); c->nanseq.release(); c->beaten.release(); c->pix.release();
     c->smap.release(); c->lastnan.release(); c->cnt.release();
     c->o_rgba.release(); c->o_vcol.release(); c->o_msaa.release(); c->o_tri.release(); c->o_depth.release(); c->o_shadow.release();
     c->o_nor.release(); c->o_fnor.release(); c->o_wpos.release(); c->o_uvd.release(); c->o_mat.release();
@@ -1203,7 +1199,7 @@ int pr_destroy(void* ctx) {
     if (c->ev_resolved) cudaEventDestroy(c->ev_resolved);
     if (c->ev_ao0) cudaEventDestroy(c->ev_ao0);
     if (c->ev_ao) cudaEventDestroy(c->ev_ao);
-    c->ao_T.release(); c->linemax.release(); c->ao_tab.release(); c->gamma.release();
+    c->ao_T.release(); c->linemax.release(); c->tables.release();
     if (c->stream_c) {
         cudaStreamSynchronize(c->stream_c);
         cudaStreamDestroy(c->stream_c);
