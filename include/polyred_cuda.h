@@ -217,8 +217,15 @@ typedef struct pr_stats {
     uint32_t n_nan_fragments;  /* fragments with NaN depth (degenerate triangles) */
     uint32_t n_kernel_launches;
     uint32_t reserved;
+    /* Device times. ms_total: the frame's first launch to its last. ms_shadow:
+       the first launch to the shadow maps' completion (they are drawn beside
+       the main pass; 0 where no light casts). The main pass: ms_setup from the
+       clearing of its counters to the raster's first block, ms_raster from
+       there to shading's first block (clipping, raster, resolve, attributes,
+       and the wait for the maps), both by the device's clock; ms_shade what is
+       left of ms_total. */
     float    ms_shadow, ms_setup, ms_raster, ms_shade, ms_total;
-    float    ms_ao;            /* ambient occlusion part of ms_shade */
+    float    ms_ao;            /* the ambient occlusion march, beside attributes and shading */
     uint32_t n_ao_pixels;
 } pr_stats;
 
