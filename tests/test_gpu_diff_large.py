@@ -1,13 +1,16 @@
 """The backward pass's shared gradients over many pixels: float32 partial sums
 stay short. A flat plane that faces its light, whose terms are whole numbers
 below 2^12: sums of 4096 of them are exact in float32 (and the totals in
-float64), longer ones are not."""
+float64), longer ones are not. And spheres of several materials under a gradient
+of either sign, against the FP64 adjoint on the same G-buffer."""
 import ctypes as C
 
 import numpy as np
 import pytest
 
+import oracle
 from polyred_gb300 import _abi, diff, native, scene as sc
+from test_gpu_diff_sums import _renderer
 
 pytestmark = pytest.mark.gpu
 LIT, FLAT = 1, 2  # G-buffer pixel flags
@@ -42,3 +45,22 @@ def test_partial_sums(W, H):
     torch.cuda.synchronize()
     native.check(r.lib.pr_diff_backward(r.device.handle, C.byref(fd.desc), C.byref(d), gbuf.data_ptr(), grad.data_ptr(), C.byref(g)))
     assert host["ambient"][0] == host["light_intensity"][0] == host["kd"][0] == total, ({n: a[0] - total for n, a in host.items()})
+
+
+def test_all_shared_gradients(W=2600, H=1701):
+    import torch
+    r = _renderer(W, H, 3)
+    p = r.initial_params()
+    _, gbuf = r.forward_raw(0, p)
+    grad = torch.randn(H, W, 4, generator=torch.Generator().manual_seed(5)).cuda()
+    got = r.backward_raw(0, p, gbuf, grad)
+    fd = r.frame(0, p["light_pos"].numpy(), p["light_intensity"].numpy(), p["ambient"].numpy())
+    npp = {k: v.detach().cpu().numpy().astype(np.float64) for k, v in p.items()}
+    inp = oracle.DiffInputs(r.flat, gbuf.cpu().numpy(), npp, fd.desc, oracle.normal_matrices(r.flat))
+    g64 = grad.cpu().numpy().astype(np.float64)
+    want, scale = oracle.diff_backward64(inp, g64), oracle.diff_backward64(inp, g64, absolute=True)
+    for k in ("kd", "ks", "shininess", "light_pos", "light_intensity", "ambient"):
+        a, b = got[k].cpu().numpy().astype(np.float64).reshape(-1), want[k].reshape(-1)
+        # each pixel's float32 terms within 2^-17 of their magnitudes (as in the central-difference checks)
+        assert (np.abs(a - b) <= 2.0 ** -17 * scale[k].reshape(-1)).all(), (k, np.abs(a - b) / scale[k].reshape(-1))
+        assert np.abs(b).max() > 0
